@@ -69,7 +69,7 @@ struct GravItem {
     int src0, src1;       // absolute source range of this chunk
     int chunk, nchunk;
     int tile;             // tile id: counter index when nchunk > 1
-    int part_off;         // first partial record of the tile
+    int part_off;         // first partial record (red-exact mode: first pair term) of the tile
     int lanes;            // threads per sink (4, 8, 16 or 32), lanes * nsink <= kTile
     int cls;
     int soff;             // first body of the system; its stars are [soff, soff + nstar)
@@ -78,7 +78,7 @@ struct GravItem {
     int spt;              // sinks per thread group (1, or 2 in the FP32 modes: lanes >= 8)
     int mstar_set;        // 1: mstar holds the mass of the system's first star (0 if inactive)
     float mstar_hi, mstar_lo;   // that mass, double-single
-    int pad[2];
+    int first_src, n_src;   // the tile's whole source list [first_src, first_src + n_src)
 };
 
 // Per-body kernels: one CTA per segment of one system.

@@ -164,6 +164,9 @@ static void gravity_classes(const SysInfo& si, int mode, GravClass out[3])
     out[2] = {CLS_NI, si.n_massive, si.n, src_start, si.n_massive};
 }
 
+constexpr int kExactCtas = 304;           // red-exact mode: chunks of a class, two CTAs per SM
+constexpr size_t kExactTerms = 1u << 22;   // and the most pair terms of a launch in memory (96 MB)
+
 // Threads per sink group and sinks per group of one class: a power of two in
 // [4, 32] lanes.  Many sinks against more than 64 sources in the FP32 modes: 8
 // lanes serving 2 sinks each (each source read feeds two interactions).  A
@@ -227,7 +230,19 @@ void plan_gravity_items(const SysInfo& si, int s, int mode, int chunk_override, 
             const int s0 = q.s0 + t * tile_sinks;
             const int nsink = std::min(tile_sinks, q.s1 - s0);
             int chunk = std::max(nsrc, 1);
-            if (mode != MODE_FP64_EXACT) {
+            if (mode == MODE_FP64_EXACT) {
+                // A class of few tiles and a long source list (the large bodies): the pair
+                // terms are formed by several CTAs, chunks of at least 32 sources and at
+                // most kExactCtas of them, and added in order by one.  A class with more
+                // tiles fills the GPU without chunks, whose terms pass through memory (24
+                // bytes each, kExactTerms at most).  chunk_override (an allocation-free
+                // caller) takes none.
+                if (chunk_override == 0 && nsrc > kTile && 2 * ntile <= kExactCtas &&
+                    part + (size_t)nsrc * nsink <= kExactTerms) {
+                    const long long c = ((long long)nsrc * ntile + kExactCtas - 1) / kExactCtas;
+                    chunk = (int)std::max(32ll, (c + 31) / 32 * 32);
+                }
+            } else {
                 if (chunk_override > 0) {
                     chunk = chunk_override;
                 } else {
@@ -265,7 +280,9 @@ void plan_gravity_items(const SysInfo& si, int s, int mode, int chunk_override, 
             }
             g.tile = nchunk > 1 ? tiles++ : -1;
             g.part_off = (int)part;
-            if (nchunk > 1) part += (size_t)nchunk * nsink;
+            g.first_src = si.off + q.j0;
+            g.n_src = nsrc;
+            if (nchunk > 1) part += (size_t)(mode == MODE_FP64_EXACT ? nsrc : nchunk) * nsink;
             for (int c = 0; c < nchunk; c++) {
                 g.chunk = c;
                 g.src0 = si.off + q.j0 + c * chunk;

@@ -568,8 +568,7 @@ __device__ __forceinline__ void gravity_f32_pair(SmemStage& sm, const StageParam
     mine_ok = lane < 3 * SPT && mine_k < it.nsink;
 }
 
-// Gravity of the chunk's sources, FP64 modes (one sink per thread group).
-template <int MODE>
+// Gravity of the chunk's sources, FP64 mode (one sink per thread group).
 __device__ __forceinline__ void gravity_f64(SmemStage& sm, const StageParams& P, const GravItem& it, D4& td, int& tid,
                                             double& mine, int& mine_k, bool& mine_ok)
 {
@@ -577,7 +576,6 @@ __device__ __forceinline__ void gravity_f64(SmemStage& sm, const StageParams& P,
     const int L = it.lanes;
     const int k = t / L, lane = t % L;
     const bool has = k < it.nsink;
-    const int i = it.sink0 + (has ? k : 0);
     const int ks = has ? k : 0;
     const double xi = sm.snk.d[3 * ks], yi = sm.snk.d[3 * ks + 1], zi = sm.snk.d[3 * ks + 2];
     double ax = 0.0, ay = 0.0, az = 0.0;
@@ -588,37 +586,19 @@ __device__ __forceinline__ void gravity_f64(SmemStage& sm, const StageParams& P,
             const int j = j0 + kTile + t;
             tid = P.id[j];
             const double m = P.mass[j];
-            td = D4{P.r_in[3 * j], P.r_in[3 * j + 1], P.r_in[3 * j + 2], (MODE == MODE_FP64 && tid < 0) ? 0.0 : m};
+            td = D4{P.r_in[3 * j], P.r_in[3 * j + 1], P.r_in[3 * j + 2], tid < 0 ? 0.0 : m};
         }
         if (has) {
-            if (MODE == MODE_FP64_EXACT) {
-                // calc_grav_accel_naive, pp_disk.cu:389-413, bit for bit: lane 0 alone,
-                // sources in index order
-                if (lane == 0) {
-                    for (int jj = 0; jj < nj; jj++) {
-                        const D4 q = sm.src.d.d[jj];
-                        if (j0 + jj == i || 0 > sm.src.d.id[jj]) continue;
-                        const double dx = __dsub_rn(q.x, xi), dy = __dsub_rn(q.y, yi), dz = __dsub_rn(q.z, zi);
-                        double w = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-                        const double d = __dsqrt_rn(w);
-                        w = __ddiv_rn(q.w, __dmul_rn(d, w));
-                        ax = __dadd_rn(ax, __dmul_rn(w, dx));
-                        ay = __dadd_rn(ay, __dmul_rn(w, dy));
-                        az = __dadd_rn(az, __dmul_rn(w, dz));
-                    }
-                }
-            } else {
-                for (int jj = lane; jj < nj; jj += L) {
-                    const D4 q = sm.src.d.d[jj];
-                    const double dx = q.x - xi, dy = q.y - yi, dz = q.z - zi;
-                    const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
-                    double ri = rsqrt(r2);
-                    ri = r2 > 0.0 ? ri : 0.0;
-                    const double sc = q.w * ri * ri * ri;
-                    ax = fma(sc, dx, ax);
-                    ay = fma(sc, dy, ay);
-                    az = fma(sc, dz, az);
-                }
+            for (int jj = lane; jj < nj; jj += L) {
+                const D4 q = sm.src.d.d[jj];
+                const double dx = q.x - xi, dy = q.y - yi, dz = q.z - zi;
+                const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+                double ri = rsqrt(r2);
+                ri = r2 > 0.0 ? ri : 0.0;
+                const double sc = q.w * ri * ri * ri;
+                ax = fma(sc, dx, ax);
+                ay = fma(sc, dy, ay);
+                az = fma(sc, dz, az);
             }
         }
         if (more) {
@@ -628,19 +608,118 @@ __device__ __forceinline__ void gravity_f64(SmemStage& sm, const StageParams& P,
             __syncthreads();
         }
     }
-    if (MODE == MODE_FP64_EXACT) {
-        const int gbase = (t & 31) & ~(L - 1);
-        ax = __shfl_sync(0xffffffffu, ax, gbase);
-        ay = __shfl_sync(0xffffffffu, ay, gbase);
-        az = __shfl_sync(0xffffffffu, az, gbase);
-    } else {
-        ax = group_sum(ax, L);
-        ay = group_sum(ay, L);
-        az = group_sum(az, L);
-    }
+    ax = group_sum(ax, L);
+    ay = group_sum(ay, L);
+    az = group_sum(az, L);
     mine = lane == 0 ? ax : (lane == 1 ? ay : az);
     mine_k = k;
     mine_ok = has && lane < 3;
+}
+
+// Gravity in red's arithmetic, bit for bit (calc_grav_accel_naive,
+// pp_disk.cu:389-413).  red adds the pair terms of a sink one after the other
+// in index order; the terms themselves do not depend on the order.  So the
+// CTA's threads form the terms side by side (a square root and a division each,
+// ~60 FP64 instructions of which the SM issues a full warp in 16 cycles), and
+// one thread per (sink, component) adds them in order.  A pair that red skips
+// (the sink itself, an inactive source) adds +0.0: the sum starts at +0.0 and
+// round-to-nearest never makes it -0.0, so that changes no bit.
+//
+// An unchunked tile keeps the terms in shared memory, kPairBatch at a time.  A
+// chunked tile (few sinks against many sources: the large-body class) writes
+// them to `partial`, 3 nsink doubles per source, and the CTA that counts last
+// adds all of them (sum_terms): its chain of dependent additions, ~110 cycles
+// each, is then all that is serial.  4100-body disk (9 large bodies), adaptive
+// RKF7(8): 57.6 ms per try when one lane formed and added the terms of its
+// sink in turn, 2.95 ms now.
+constexpr int kPairBatch = 512;
+constexpr int kPairStride = kPairBatch + 6;   // the components' rows start in different banks
+
+__device__ __forceinline__ void exact_term(const D4& q, int jd, bool self, double xi, double yi, double zi, double& tx,
+                                           double& ty, double& tz)
+{
+    tx = ty = tz = 0.0;
+    if (self || 0 > jd) return;
+    const double dx = __dsub_rn(q.x, xi), dy = __dsub_rn(q.y, yi), dz = __dsub_rn(q.z, zi);
+    double w = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+    const double d = __dsqrt_rn(w);
+    w = __ddiv_rn(q.w, __dmul_rn(d, w));
+    tx = __dmul_rn(w, dx);
+    ty = __dmul_rn(w, dy);
+    tz = __dmul_rn(w, dz);
+}
+
+// `terms`: 3 kPairStride doubles of shared memory.  Returns the sum of element
+// threadIdx.x of an unchunked tile.
+__device__ __forceinline__ double gravity_exact(SmemStage& sm, double* terms, const StageParams& P, const GravItem& it,
+                                                D4& td, int& tid)
+{
+    const int t = threadIdx.x;
+    const int ns = it.nsink;
+    const bool chunked = it.nchunk > 1;   // uniform
+    const int batch = max(1, kPairBatch / ns);   // sources per batch of an unchunked tile
+    double a = 0.0;
+    for (int j0 = it.src0; j0 < it.src1; j0 += kTile) {
+        const int nj = min(kTile, it.src1 - j0);
+        const bool more = j0 + kTile < it.src1;
+        if (more && t < min(kTile, it.src1 - j0 - kTile)) {
+            const int j = j0 + kTile + t;
+            tid = P.id[j];
+            td = D4{P.r_in[3 * j], P.r_in[3 * j + 1], P.r_in[3 * j + 2], P.mass[j]};
+        }
+        for (int b0 = 0; b0 < nj; b0 += batch) {
+            const int nb = chunked ? nj : min(batch, nj - b0);
+            for (int p = t; p < nb * ns; p += kTile) {
+                const int jj = b0 + p / ns, k = p % ns;
+                double tx, ty, tz;
+                exact_term(sm.src.d.d[jj], sm.src.d.id[jj], j0 + jj == it.sink0 + k, sm.snk.d[3 * k],
+                           sm.snk.d[3 * k + 1], sm.snk.d[3 * k + 2], tx, ty, tz);
+                if (chunked) {
+                    double* o = P.partial + 3 * (it.part_off + (long long)(j0 + jj - it.first_src) * ns + k);
+                    o[0] = tx;
+                    o[1] = ty;
+                    o[2] = tz;
+                } else {
+                    terms[p] = tx;
+                    terms[kPairStride + p] = ty;
+                    terms[2 * kPairStride + p] = tz;
+                }
+            }
+            if (chunked) break;
+            __syncthreads();
+            if (t < 3 * ns) {
+                const double* q = terms + (t % 3) * kPairStride + t / 3;
+                for (int u = 0; u < nb; u++) a = __dadd_rn(a, q[u * ns]);
+            }
+            __syncthreads();
+        }
+        if (more) {
+            __syncthreads();
+            sm.src.d.d[t] = td;
+            sm.src.d.id[t] = tid;
+            __syncthreads();
+        }
+    }
+    return a;
+}
+
+// The n terms of one element of a chunked tile (`stride` doubles apart), added
+// in order: the next batch is loaded while one is added.
+__device__ __forceinline__ double sum_terms(const double* base, long long stride, int n)
+{
+    constexpr int kB = 24;
+    double cur[kB], nxt[kB], a = 0.0;
+#pragma unroll
+    for (int u = 0; u < kB; u++) cur[u] = u < n ? __ldcg(base + u * stride) : 0.0;
+    for (int b = 0; b < n; b += kB) {
+#pragma unroll
+        for (int u = 0; u < kB; u++) nxt[u] = b + kB + u < n ? __ldcg(base + (b + kB + u) * stride) : 0.0;
+#pragma unroll
+        for (int u = 0; u < kB; u++) a = __dadd_rn(a, cur[u]);
+#pragma unroll
+        for (int u = 0; u < kB; u++) cur[u] = nxt[u];
+    }
+    return a;
 }
 
 // ---------------------------------------------------------------------------
@@ -672,10 +751,14 @@ __device__ __forceinline__ void gravity_f64(SmemStage& sm, const StageParams& P,
 // CTA hides more of it (512-disk ensemble stage -17 %, 65536-body gas-drag
 // disk -13 %, all-pairs 16384-body disk -1.3 %; 8 CTAs at 64 registers spill
 // and are slower).  The one-wave instance keeps 80 registers.
+// The red-exact instances keep 24 terms of a sum in flight (sum_terms) and hold
+// 12 KB of terms: 4 CTAs per SM.
 template <int MODE, bool EXACT, bool CL, int VT, bool PK = false>
-__global__ void __launch_bounds__(kTile, PK ? 6 : (VT >= 0 ? 7 : 6)) k_stage(const StageParams P, const int Vrt)
+__global__ void __launch_bounds__(kTile, MODE == MODE_FP64_EXACT ? 4 : PK ? 6 : (VT >= 0 ? 7 : 6))
+k_stage(const StageParams P, const int Vrt)
 {
     constexpr bool kF32 = (MODE == MODE_MIXED || MODE == MODE_FP32);
+    constexpr bool kRedSum = MODE == MODE_FP64_EXACT;   // gravity as terms added in red's order
     const int V = VT >= 0 ? VT : Vrt;
     const bool kRkf = (V >= 1 && V <= 12);
     const int nk = var_nk(V);
@@ -683,6 +766,7 @@ __global__ void __launch_bounds__(kTile, PK ? 6 : (VT >= 0 ? 7 : 6)) k_stage(con
     constexpr int kUnroll = VT >= 0 ? kNkMax : 1;   // operand loops: unrolled when nk is a constant
     __shared__ SmemStage sm;
     __shared__ double ops[kOpsMax][kMaxElem];
+    __shared__ double terms[kRedSum ? 3 * kPairStride : 1];
     const GravItem it = P.items[blockIdx.x];
     const int s = P.stage;
     // Stage 0 follows the kernels that update the system records, y and the
@@ -846,14 +930,16 @@ __global__ void __launch_bounds__(kTile, PK ? 6 : (VT >= 0 ? 7 : 6)) k_stage(con
     // ---- gravity of the chunk's sources ----
     float2 mine_ds = make_float2(0.f, 0.f);   // FP32 modes: double-single sums
     double mine = 0.0;                        // FP64 modes
-    int mine_k;
-    bool mine_ok;
+    int mine_k = 0;
+    bool mine_ok = false;
     if constexpr (kF32) {
         if (PK && it.spt == 2) gravity_f32_pair<MODE>(sm, P, it, staged, th, tl, mine_ds, mine_k, mine_ok);
         else if (!PK && it.spt == 2) gravity_f32<MODE, 2>(sm, P, it, staged, th, tl, mine_ds, mine_k, mine_ok);
         else gravity_f32<MODE, 1>(sm, P, it, staged, th, tl, mine_ds, mine_k, mine_ok);
+    } else if constexpr (kRedSum) {
+        mine = gravity_exact(sm, terms, P, it, td, tid);
     } else {
-        gravity_f64<MODE>(sm, P, it, td, tid, mine, mine_k, mine_ok);
+        gravity_f64(sm, P, it, td, tid, mine, mine_k, mine_ok);
     }
     const int mine_c = (t % it.lanes) % 3;
 
@@ -870,7 +956,7 @@ __global__ void __launch_bounds__(kTile, PK ? 6 : (VT >= 0 ? 7 : 6)) k_stage(con
     // the fences, whose latency other CTAs hide, so that their reducing CTA
     // never waits on a store in flight.  The element threads form the star
     // term meanwhile ----
-    constexpr bool kFencedRecords = VT >= 0;
+    constexpr bool kFencedRecords = VT >= 0 || kRedSum;
     float2 g_ds = make_float2(0.f, 0.f);   // gravity of the element, FP32 modes
     double a = 0.0;                         // gravity of the element, FP64 modes
     float2* acc2 = reinterpret_cast<float2*>(sm.acc);
@@ -946,40 +1032,47 @@ __global__ void __launch_bounds__(kTile, PK ? 6 : (VT >= 0 ? 7 : 6)) k_stage(con
             cp_async_wait_all();   // no copy may land in shared memory after the CTA has gone
             return;
         }
-        const int nsplit = kTile / nel;
-        const int sp_i = t / nel;
-        const int e = t - sp_i * nel;
-        const int c0 = sp_i < nsplit ? sp_i * it.nchunk / nsplit : 0;
-        const int c1 = sp_i < nsplit ? (sp_i + 1) * it.nchunk / nsplit : 0;
-        if constexpr (kFencedRecords) {
-            const long long base = 3 * (long long)it.part_off + e;
-            if (kF32) acc2[t] = sum_records_ds(reinterpret_cast<const float2*>(P.partial) + base, 3LL * it.nsink, c0, c1);
-            else sm.acc[t] = sum_records(P.partial + base, 3LL * it.nsink, c0, c1);
+        if constexpr (kRedSum) {
+            if (elem) a = sum_terms(P.partial + 3 * (long long)it.part_off + t, 3LL * it.nsink, it.n_src);
+            if (t == 0) P.tile_cnt[it.tile] = 0u;
         } else {
-            unsigned long long* recs = reinterpret_cast<unsigned long long*>(P.partial) + 3 * (long long)it.part_off + e;
-            bool landed;
-            if (kF32) {
-                float2 sum = make_float2(0.f, 0.f);
-                landed = sum_polled_records(recs, 3LL * it.nsink, c0, c1, sum);
-                acc2[t] = sum;
+            const int nsplit = kTile / nel;
+            const int sp_i = t / nel;
+            const int e = t - sp_i * nel;
+            const int c0 = sp_i < nsplit ? sp_i * it.nchunk / nsplit : 0;
+            const int c1 = sp_i < nsplit ? (sp_i + 1) * it.nchunk / nsplit : 0;
+            if constexpr (kFencedRecords) {
+                const long long base = 3 * (long long)it.part_off + e;
+                if (kF32) acc2[t] = sum_records_ds(reinterpret_cast<const float2*>(P.partial) + base, 3LL * it.nsink, c0, c1);
+                else sm.acc[t] = sum_records(P.partial + base, 3LL * it.nsink, c0, c1);
             } else {
-                double sum = 0.0;
-                landed = sum_polled_records(recs, 3LL * it.nsink, c0, c1, sum);
-                sm.acc[t] = sum;
+                unsigned long long* recs = reinterpret_cast<unsigned long long*>(P.partial) + 3 * (long long)it.part_off + e;
+                bool landed;
+                if (kF32) {
+                    float2 sum = make_float2(0.f, 0.f);
+                    landed = sum_polled_records(recs, 3LL * it.nsink, c0, c1, sum);
+                    acc2[t] = sum;
+                } else {
+                    double sum = 0.0;
+                    landed = sum_polled_records(recs, 3LL * it.nsink, c0, c1, sum);
+                    sm.acc[t] = sum;
+                }
+                if (!landed) {   // RED_ERR_TIMEOUT; the system stops (k_control then leaves it alone)
+                    S->status = 4;
+                    S->halted = 1;
+                }
             }
-            if (!landed) {   // RED_ERR_TIMEOUT; the system stops (k_control then leaves it alone)
-                S->status = 4;
-                S->halted = 1;
+            __syncthreads();
+            if (elem) {
+                for (int q = 0; q < nsplit; q++) {
+                    if (kF32) g_ds = dsn_add(g_ds, acc2[q * nel + t]);
+                    else a += sm.acc[q * nel + t];
+                }
             }
+            if (t == 0) P.tile_cnt[it.tile] = 0u;
         }
-        __syncthreads();
-        if (elem) {
-            for (int q = 0; q < nsplit; q++) {
-                if (kF32) g_ds = dsn_add(g_ds, acc2[q * nel + t]);
-                else a += sm.acc[q * nel + t];
-            }
-        }
-        if (t == 0) P.tile_cnt[it.tile] = 0u;
+    } else if constexpr (kRedSum) {
+        if (elem) a = mine;
     } else {
         if (mine_ok) {
             if (kF32) acc2[3 * mine_k + mine_c] = mine_ds;
