@@ -9,7 +9,7 @@
 //               bodies (FP32 prefilter + red's FP64 test) and hash queries
 //   k_collision, k_grid_insert, k_grid_query   the same, for the explicit check
 //   k_ejhc      ejection / hit-centrum test
-//   k_potential per-body potential sums for the integrals
+//   k_potential potential sums for the integrals
 #include <algorithm>
 #include <cfloat>
 #include <cstdio>
@@ -431,35 +431,76 @@ __global__ void __launch_bounds__(kSegment) k_ejhc(const EjhcParams P)
     }
 }
 
-// Per-body potential sums in FP64: u_i = m_i * sum_j m_j / r_ij over the
-// partners of i (all other active bodies, or the interacting partners j > i).
-__global__ void __launch_bounds__(kSegment) k_potential(const Segment* segs, const SysInfo* sinfo,
-                                                        const double* y_r, const double* mass, const int* id,
-                                                        int sys_filter, int interacting, double* u)
+// 1 / sqrt(x) in FP64 with few FP64 instructions (GB300 issues one warp of them
+// in 16 cycles): the FP32 hardware estimate y of the truncated x, then one
+// Householder step of third order, y + y e (1/2 + 3/8 e) with e = 1 - x y^2;
+// y^2 is exact (48 bits) and e^3 ~ 2^-63, so the result is within an ulp or
+// so.  x outside FP32's normal range takes the library's function.
+__device__ __forceinline__ double rsqrt_f64(double x)
 {
-    const Segment sg = segs[blockIdx.x];
-    if (sg.sys != sys_filter) return;
-    const SysInfo si = sinfo[sg.sys];
-    const int i = sg.b0 + threadIdx.x;
-    if (i >= sg.b1) return;
-    double acc = 0.0;
-    if (id[i] >= 0) {
-        const double xi = y_r[3 * i], yi = y_r[3 * i + 1], zi = y_r[3 * i + 2];
-        int j0 = si.off, j1 = si.off + si.n;
-        if (interacting) {
-            // each interacting pair once: from its SI member i towards j > i among the massive bodies
-            const int rel = i - si.off;
-            j0 = i + 1;
-            j1 = rel < si.n_SI ? si.off + si.n_massive : j0;
-        }
-        for (int j = j0; j < j1; j++) {
-            if (j == i || id[j] < 0) continue;
-            const double dx = y_r[3 * j] - xi, dy = y_r[3 * j + 1] - yi, dz = y_r[3 * j + 2] - zi;
-            acc += mass[j] / sqrt(dx * dx + dy * dy + dz * dz);
-        }
-        acc *= mass[i];
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const int e = (int)(b >> 52);   // negative x and NaN are above the range
+    if (!(e > 1023 - 126 && e < 1023 + 127)) return rsqrt(x);
+    const float xf = __uint_as_float(((unsigned)(e - 1023 + 127) << 23) | (unsigned)((b >> 29) & 0x7FFFFFu));
+    const double y = f2d_bits(rsqrtf(xf));
+    const double r = fma(-x, y * y, 1.0);
+    return fma(y * r, fma(r, 0.375, 0.5), y);
+}
+
+// Potential sums in FP64, each pair once: a CTA holds kTile bodies j (one per
+// thread) against a range of bodies i, and writes sum m_i m_j / r_ij over its
+// pairs with i < j, i < ni, j < nj (indices relative to the system; ids < 0 are
+// skipped).  All pairs: ni = nj = n; the interacting ones: ni = n_SI, nj =
+// n_massive.  CTA (x, y) of the grid: j from x kTile, i from y isub; one
+// partial each, added by the host in order.  Bound by the FP64 pipe: 12
+// instructions per pair.  With one thread per body i, over every j with a root
+// and a division (one thread per large body for the interacting pairs), the
+// two sums, the collision check and the state of the 16384-body disk took 44.1
+// ms; with this kernel 4.6 ms.
+__global__ void __launch_bounds__(kTile) k_potential(int off, int ni, int nj, int isub, const double* y_r,
+                                                     const double* mass, const int* id, double* u)
+{
+    __shared__ D4 sh[kTile];
+    __shared__ int on[kTile];
+    __shared__ double part[kTile / 32];
+    const int t = threadIdx.x;
+    const int jt = blockIdx.x * kTile;
+    const int i0 = blockIdx.y * isub, i1 = min(min(ni, i0 + isub), jt + kTile);
+    const int j = jt + t;
+    const bool live = j < nj && id[off + j] >= 0;
+    double x = 0.0, y = 0.0, z = 0.0, acc = 0.0;
+    if (live) {
+        x = y_r[3 * (off + j)];
+        y = y_r[3 * (off + j) + 1];
+        z = y_r[3 * (off + j) + 2];
     }
-    u[i] = acc;
+    for (int b = i0; b < i1; b += kTile) {   // uniform over the CTA
+        const int nb = min(kTile, i1 - b);
+        __syncthreads();
+        if (t < nb) {
+            const int i = off + b + t;
+            sh[t] = D4{y_r[3 * i], y_r[3 * i + 1], y_r[3 * i + 2], mass[i]};
+            on[t] = id[i] >= 0;
+        }
+        __syncthreads();
+        const int ne = live ? min(nb, j - b) : 0;   // i < j
+#pragma unroll 4
+        for (int k = 0; k < ne; k++) {
+            const D4 q = sh[k];
+            const double dx = q.x - x, dy = q.y - y, dz = q.z - z;
+            const double ri = rsqrt_f64(fma(dz, dz, fma(dy, dy, dx * dx)));
+            if (on[k]) acc = fma(q.w, ri, acc);
+        }
+    }
+    acc = live ? acc * mass[off + j] : 0.0;
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if ((t & 31) == 0) part[t >> 5] = acc;
+    __syncthreads();
+    if (t == 0) {
+        double a = part[0];
+        for (int w = 1; w < kTile / 32; w++) a += part[w];
+        u[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = a;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -646,11 +687,23 @@ void launch_ejhc(const EjhcParams& P, int n_segs, cudaStream_t s)
     if (n_segs > 0) launch_k(k_ejhc, (unsigned)n_segs, (unsigned)kSegment, s, P);
 }
 
-void launch_potential(const Segment* segs, int n_segs, const SysInfo* sinfo, const double* y_r,
-                      const double* mass, const int* id, int sys_filter, int interacting, double* u,
+int potential_partials(int ni, int nj, int* isub)
+{
+    const int tx = std::max(1, (nj + kTile - 1) / kTile);
+    int ty = std::max(1, kPotentialCtas / tx);
+    const int sub = std::max(32, ((ni + ty - 1) / ty + 31) / 32 * 32);
+    ty = std::max(1, (ni + sub - 1) / sub);
+    if (isub) *isub = sub;
+    return tx * ty;
+}
+
+void launch_potential(int off, int ni, int nj, const double* y_r, const double* mass, const int* id, double* u,
                       cudaStream_t s)
 {
-    if (n_segs > 0) k_potential<<<n_segs, kSegment, 0, s>>>(segs, sinfo, y_r, mass, id, sys_filter, interacting, u);
+    int isub = 0;
+    const int parts = potential_partials(ni, nj, &isub);
+    const int tx = std::max(1, (nj + kTile - 1) / kTile);
+    k_potential<<<dim3((unsigned)tx, (unsigned)(parts / tx)), kTile, 0, s>>>(off, ni, nj, isub, y_r, mass, id, u);
 }
 
 }  // namespace redgb

@@ -309,8 +309,12 @@ void launch_pack_state(int o, int n, const double* y_r, const double* y_v, const
 void launch_unpack_state(int o, int n, int what, StateSegs src, const int* ib, double* y_r, double* y_v,
                          double* mass, double* radius, double* density, double* cd, int* id, float4* hi0,
                          float4* lo0, cudaStream_t s);
-void launch_potential(const Segment* segs, int n_segs, const SysInfo* sinfo, const double* y_r,
-                      const double* mass, const int* id, int sys_filter, int interacting, double* u,
+// The potential of ni x nj pairs as partial sums (k_potential): how many (their
+// count fits kPotentialCtas or, for long systems, one per kTile bodies), and
+// the bodies i of one partial.
+constexpr int kPotentialCtas = 4096;   // ~27 CTAs per SM, half of them above the diagonal
+int potential_partials(int ni, int nj, int* isub);
+void launch_potential(int off, int ni, int nj, const double* y_r, const double* mass, const int* id, double* u,
                       cudaStream_t s);
 
 }  // namespace redgb

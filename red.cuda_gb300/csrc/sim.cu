@@ -657,7 +657,7 @@ void red_sim::create(const red_config_t* c, uint32_t n_systems, const uint32_t* 
     }
     mass = dalloc<double>(N); radius = dalloc<double>(N); density = dalloc<double>(N); cd = dalloc<double>(N);
     id = dalloc<int>(N); btype = dalloc<int>(N);
-    d_u = dalloc<double>(N);
+    d_u = dalloc<double>(kPotentialCtas + (N + kTile - 1) / kTile);   // potential_partials() of any system
     d_next = dalloc<int>(N);
     d_cell = dalloc<int4>(N);
     d_grid = dalloc<GridInfo>(n_sys);
@@ -1676,17 +1676,21 @@ int red_calc_dydx(red_sim* sim, uint32_t sys, int32_t i, double t, red_var4_t* d
     GUARD_END
 }
 
-static int potential(red_sim* sim, uint32_t sys, int interacting, std::vector<double>& u)
+// The potential of system sys: sum of m_i m_j / r_ij over all pairs, or over the
+// interacting ones (an SI body and any later massive body).
+static double potential(red_sim* sim, uint32_t sys, int interacting)
 {
     const SysHost& h = sim->sh[sys];
-    launch_potential(sim->d_segs, (int)sim->segs.size(), sim->d_sinfo, sim->y_r, sim->mass, sim->id, (int)sys,
-                     interacting, sim->d_u, sim->stream);
+    const int ni = (int)(interacting ? h.n_SI() : h.n), nj = (int)(interacting ? h.n_massive() : h.n);
+    launch_potential((int)h.off, ni, nj, sim->y_r, sim->mass, sim->id, sim->d_u, sim->stream);
     CK(cudaGetLastError());
     sim->launches++;
-    u.resize(h.n);
-    CK(cudaMemcpyAsync(u.data(), sim->d_u + h.off, h.n * sizeof(double), cudaMemcpyDeviceToHost, sim->stream));
+    std::vector<double> u((size_t)potential_partials(ni, nj, nullptr));
+    CK(cudaMemcpyAsync(u.data(), sim->d_u, u.size() * sizeof(double), cudaMemcpyDeviceToHost, sim->stream));
     CK(cudaStreamSynchronize(sim->stream));
-    return RED_OK;
+    double U = 0.0;
+    for (double x : u) U += x;
+    return U;
 }
 
 int red_calc_integral(red_sim* sim, uint32_t sys, red_integral_t* out)
@@ -1720,14 +1724,11 @@ int red_calc_integral(red_sim* sim, uint32_t sys, red_integral_t* out)
         C[2] += m * (r.x * v.y - r.y * v.x);
         T += m * (v.x * v.x + v.y * v.y + v.z * v.z);
     }
-    std::vector<double> u;
-    potential(sim, sys, 0, u);
-    double U = 0.0;
-    for (double x : u) U += x;
+    const double U = potential(sim, sys, 0);
     out->R = red_var4_t{R[0] / M0, R[1] / M0, R[2] / M0, 0.0};
     out->V = red_var4_t{V[0] / M0, V[1] / M0, V[2] / M0, 0.0};
     out->C = red_var4_t{C[0], C[1], C[2], 0.0};
-    out->E = T / 2.0 - U / 2.0;
+    out->E = T / 2.0 - U;
     return RED_OK;
     GUARD_END
 }
@@ -1752,10 +1753,7 @@ int red_calc_energy_interacting(red_sim* sim, uint32_t sys, double out[4])
         C[1] += m * (r.z * v.x - r.x * v.z);
         C[2] += m * (r.x * v.y - r.y * v.x);
     }
-    std::vector<double> u;
-    potential(sim, sys, 1, u);
-    double U = 0.0;
-    for (double x : u) U += x;
+    const double U = potential(sim, sys, 1);
     out[0] = T / 2.0 - U;
     out[1] = C[0];
     out[2] = C[1];
