@@ -18,7 +18,8 @@ constexpr int oW3 = oB2 + kHid;
 constexpr int oB3 = oW3 + kHid;
 constexpr int kNParam = oB3 + 1;   // 5057
 constexpr int kNPart = 10;     // partial sums per feature segment
-constexpr int kTrainRows = 16; // rows per CTA of the training kernel
+constexpr int kTrainRows = 16; // rows per tile of the training kernel
+constexpr int kTrainCtas = 4 * 152;   // its largest grid: resident at once (38 KB of shared memory per CTA)
 
 struct MlpNorm {
     float x_mean[kFeat], x_std[kFeat];
