@@ -342,6 +342,15 @@ static __device__ void drag_factor_fast(const GasDev& g, double decr, double m_s
     f = decr * (double)((3.0f * (float)cd * dens * un) / (8.0f * (float)radius * (float)density));
 }
 
+// The time offset c_s of stage s (RKF7(8), RK4, RK2; Euler evaluates at t).
+__device__ __forceinline__ double stage_c(int scheme, int s)
+{
+    if (scheme == SCHEME_RKF78) return c_tb.c[s];
+    if (scheme == SCHEME_RK4) return c_tb.c4[s];
+    if (scheme == SCHEME_RK2) return c_tb.c2[s];
+    return 0.0;
+}
+
 struct alignas(32) D4 {
     double x, y, z, w;
 };

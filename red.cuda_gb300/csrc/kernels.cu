@@ -15,6 +15,8 @@
 #include <cstdio>
 
 #include "common.cuh"
+#include "control.cuh"
+#include "try.cuh"
 
 namespace redgb {
 
@@ -45,10 +47,7 @@ __global__ void __launch_bounds__(kSegment) k_prep(const Segment* segs, const Sy
     reinterpret_cast<float*>(lo1 + i)[3] = __double2float_rn(radius[i]);
 }
 
-// One thread per system: integrator::step's accept / reject logic
-// (int_rungekutta8.cu:690-716, int_rungekutta4.cu:226-248), the counters
-// (integrator.cu:270-275) and run_simulation's dt_next clamp and loop bound
-// (main.cu:471, 535-538).
+// One thread per system: the step control after a try (control.cuh).
 __global__ void k_control(const ControlParams P)
 {
     pdl_wait();
@@ -58,65 +57,15 @@ __global__ void k_control(const ControlParams P)
     DevSys& S = P.sys[s];
     S.accepted = 0;
     if (!runnable(S)) return;
-    const double dt = S.dt_try;
-    double dt_new = dt;
-    S.iter++;
-    if (P.adaptive) {
-        const double err = __longlong_as_double((long long)S.err_bits);
-        S.err_bits = 0ull;
-        const double max_err = fabs(P.lambda * dt * err);
-        S.err_last = max_err;
-        if (max_err != max_err) {
-            S.status = 5;   // RED_ERR_NONFINITE
-            S.halted = 1;
-            S.active = 0;
-            return;
-        }
-        // the red-exact mode takes the nearest double of the power, as the C
-        // library's pow of red's host controller does (crmath.cuh)
-        if (0.0 < max_err)
-            dt_new = dt * (0.9 * (P.exact ? crmath::cr_pow(P.tolerance / max_err, 1.0 / (double)P.order)
-                                          : pow(P.tolerance / max_err, 1.0 / (double)P.order)));
-        else dt_new = dt * 2.0;
-        if (max_err > P.tolerance) {
-            S.dt_try = dt_new;
-            S.dt_next = dt_new;
-            return;
-        }
-    }
-    S.dt_did = dt;
-    S.dt_next = dt_new;
-    S.t += dt;
-    S.n_tried += (unsigned long long)S.iter;
-    S.n_failed += (unsigned long long)(S.iter - 1);
-    S.n_passed += 1ull;
-    S.iter = 0;
-    S.accepted = 1;
-    if (S.quota > 0) S.quota--;
-    if (P.output_interval != 0.0 && fabs(P.output_interval) < fabs(S.dt_next))
-        S.dt_next = 0.0 < dt ? P.output_interval : -P.output_interval;
-    // euler::step / rungekutta2::step take dt_try, never dt_next (int_euler.cu:73-105)
-    if (!P.keep_dt) S.dt_try = S.dt_next;
-    if (P.length != 0.0 && fabs(S.t - S.t_start) > fabs(P.length)) S.active = 0;
+    const unsigned long long err = S.err_bits;
+    if (P.adaptive) S.err_bits = 0ull;
+    control_system(P, S, err);
 }
 
-// Spatial-hash broad phase for the small bodies.  Cell coordinates are
-// clamped so that far-away bodies share border cells (tested exactly, never
-// missed).
-__device__ __forceinline__ int cell_coord(double x, double inv_h)
-{
-    const double lim = 1.0e9;
-    return (int)floor(fmin(fmax(x * inv_h, -lim), lim));
-}
+// Spatial-hash broad phase for the small bodies.
 __device__ __forceinline__ int4 cell_of(double x, double y, double z, double inv_h)
 {
     return make_int4(cell_coord(x, inv_h), cell_coord(y, inv_h), cell_coord(z, inv_h), 0);
-}
-
-__device__ __forceinline__ int bucket_of(int cx, int cy, int cz, int mask)
-{
-    const unsigned h = ((unsigned)cx * 73856093u) ^ ((unsigned)cy * 19349663u) ^ ((unsigned)cz * 83492791u);
-    return (int)(h & (unsigned)mask);
 }
 
 // Inserts small body i at position (x, y, z) into its system's hash table.
@@ -592,6 +541,7 @@ void set_tableau(const Tableau& tb, cudaStream_t s)
     set_tableau_fp32(tb, s);
     set_tableau_fp64(tb, s);
     set_tableau_exact(tb, s);
+    set_tableau_try(tb, s);
 }
 
 // Variant of k_stage: the shape of the combination its epilogue forms.

@@ -21,6 +21,7 @@
 
 #include "redgb_dev.cuh"
 #include "proposer.cuh"
+#include "try.cuh"
 #include "redgb.h"
 
 using namespace redgb;
@@ -109,6 +110,76 @@ Tableau make_tableau()
     memcpy(t.b2, b2, sizeof(b2));
     memcpy(t.c2, c2, sizeof(c2));
     return t;
+}
+
+// A scheme's Nystroem form (try.cuh) from its tableau a (rows of n_stage), b.
+void ny_row(NyTableau& n, int row, const std::vector<double>& a)
+{
+    int u = n.beg[row];
+    for (size_t q = 0; q < a.size(); q++)
+        if (a[q] != 0.0) {
+            NyTerm& t = n.term[u++];
+            t.a.x = (float)a[q];
+            t.a.y = (float)(a[q] - (double)t.a.x);
+            t.q = (int)q;
+        }
+    n.beg[row + 1] = u;
+}
+
+// a row times the matrix a: sum_q x_q a_qj
+std::vector<double> times_a(const std::vector<double>& x, const std::vector<std::vector<double>>& a)
+{
+    std::vector<double> y(x.size(), 0.0);
+    for (size_t j = 0; j < x.size(); j++) {
+        long double s = 0.0L;
+        for (size_t q = 0; q < x.size(); q++) s += (long double)x[q] * a[q][j];
+        y[j] = (double)s;
+    }
+    return y;
+}
+
+NyTableau make_nystroem(const Tableau& t, int scheme)
+{
+    const int ns = scheme == SCHEME_RKF78 ? 13 : scheme == SCHEME_RK4 ? 5 : scheme == SCHEME_RK2 ? 2 : 1;
+    std::vector<std::vector<double>> a(ns, std::vector<double>(ns, 0.0));
+    std::vector<double> b(ns, 0.0), er(ns, 0.0);
+    if (scheme == SCHEME_RKF78) {
+        for (int s = 1; s < ns; s++)
+            for (int q = 0; q < s; q++) a[s][q] = t.a[1 + s * (s - 1) / 2 + q];
+        for (int q = 0; q < 11; q++) b[q] = t.b[q];
+        er[0] = er[10] = 1.0;   // of the stage velocities (int_rungekutta8.cu:248-260)
+        er[11] = er[12] = -1.0;
+    } else if (scheme == SCHEME_RK4) {
+        for (int s = 1; s < 4; s++) a[s][s - 1] = t.a4[s];
+        b[0] = b[3] = t.b4[0];
+        b[1] = b[2] = t.b4[1];
+        a[4] = b;               // the adaptive stage 4 is evaluated at y_{n+1}
+        er[3] = 1.0;            // int_rungekutta4.cu:62-73
+        er[4] = -1.0;
+    } else if (scheme == SCHEME_RK2) {
+        a[1][0] = t.a2[1];
+        b[1] = t.b2[1];
+    } else {
+        b[0] = 1.0;
+    }
+    NyTableau n;
+    memset(&n, 0, sizeof(n));
+    const std::vector<double> none(ns, 0.0);
+    for (int s = 0; s < kMaxStages; s++) {
+        long double c = 0.0L;
+        if (s < ns)
+            for (double x : a[s]) c += x;
+        n.c[s] = (double)c;
+        ny_row(n, s, s < ns ? times_a(a[s], a) : none);
+    }
+    for (int s = 0; s < kMaxStages; s++) ny_row(n, kTryRowV + s, s < ns ? a[s] : none);
+    long double cb = 0.0L;
+    for (double x : b) cb += x;
+    n.cb = (double)cb;
+    ny_row(n, kTryRowRB, times_a(b, a));
+    ny_row(n, kTryRowVB, b);
+    ny_row(n, kTryRowER, times_a(er, a));
+    return n;
 }
 
 template <class T> T* dalloc(size_t n)
@@ -459,6 +530,17 @@ struct red_sim {
     int lanes_cap = 32;         // upper bound on threads per sink (autotuner)
     bool allow_cluster = true;  // the planner may lay chunk groups out as clusters (autotuner)
     bool allow_packed = true;   // plans of 2-sink tiles may take the packed-pair instance (autotuner)
+    // whole tries in one cooperative launch (try.cuh), for one sparse system
+    bool allow_try = true;      // (autotuner)
+    bool use_try = false;
+    int try_cta = 0, try_nb = 0, try_pull = 0, try_bodies = 0, try_owners = 0, try_lanes = 0;
+    uint4* d_try = nullptr;     // exchange records
+    size_t try_cap = 0;
+    unsigned* d_epoch = nullptr;
+    NyTableau* d_ny = nullptr;
+    bool tries_whole() const { return use_try && !prop_on && !log_on; }   // the proposer reads Kv[0]
+    void plan_try();
+    TryParams try_params();
     bool use_packed = false;    // the plan's stage launches take the packed-pair instance
     red_plan_info_t plan_info{};   // what the last red_autotune measured
 
@@ -473,6 +555,7 @@ struct red_sim {
                 const double* dt0);
     void build_plan();
     StageParams stage_params(int s, bool standalone);
+    ControlParams control_params();
     void enqueue_try(std::vector<int>* kinds = nullptr, std::vector<cudaEvent_t>* evs = nullptr);
     void capture();
     void launch_tries(uint32_t n);
@@ -533,6 +616,7 @@ red_sim::~red_sim()
     cudaFree(partial); cudaFree(tile_cnt); cudaFree(d_sys); cudaFree(d_sinfo); cudaFree(d_items); cudaFree(d_sparse_items);
     cudaFree(d_segs); cudaFree(d_pairs); cudaFree(d_events); cudaFree(d_nev); cudaFree(d_u);
     cudaFree(d_grid); cudaFree(d_head); cudaFree(d_next); cudaFree(d_cell); cudaFree(d_fsegs);
+    cudaFree(d_try); cudaFree(d_epoch); cudaFree(d_ny);
     cudaFree(d_xfer);
     if (h_xfer) cudaFreeHost(h_xfer);
     if (h_sys) cudaFreeHost(h_sys);
@@ -646,20 +730,21 @@ void red_sim::create(const red_config_t* c, uint32_t n_systems, const uint32_t* 
     }
     y_r = dalloc<double>(3 * N);
     y_v = dalloc<double>(3 * N);
+    // what a whole try reads lies together (fewer pages touched)
+    mass = dalloc<double>(N); radius = dalloc<double>(N); density = dalloc<double>(N); cd = dalloc<double>(N);
+    id = dalloc<int>(N); btype = dalloc<int>(N);
+    d_next = dalloc<int>(N);
+    d_cell = dalloc<int4>(N);
+    for (int k = 0; k < 2; k++) {
+        pos_hi[k] = dalloc<float4>(N);
+        pos_lo[k] = dalloc<float4>(N);
+    }
     tr[0] = dalloc<double>(3 * N);
     tr[1] = dalloc<double>(3 * N);
     Kr[0] = y_v;
     for (int s = 1; s < n_stage; s++) Kr[s] = dalloc<double>(3 * N);
     for (int s = 0; s < n_stage; s++) Kv[s] = dalloc<double>(3 * N);
-    for (int k = 0; k < 2; k++) {
-        pos_hi[k] = dalloc<float4>(N);
-        pos_lo[k] = dalloc<float4>(N);
-    }
-    mass = dalloc<double>(N); radius = dalloc<double>(N); density = dalloc<double>(N); cd = dalloc<double>(N);
-    id = dalloc<int>(N); btype = dalloc<int>(N);
     d_u = dalloc<double>(kPotentialCtas + (N + kTile - 1) / kTile);   // potential_partials() of any system
-    d_next = dalloc<int>(N);
-    d_cell = dalloc<int4>(N);
     d_grid = dalloc<GridInfo>(n_sys);
     CK(cudaMemcpy(y_r, hr.data(), 3 * N * sizeof(double), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(y_v, hv.data(), 3 * N * sizeof(double), cudaMemcpyHostToDevice));
@@ -687,6 +772,9 @@ void red_sim::create(const red_config_t* c, uint32_t n_systems, const uint32_t* 
     d_nev = dalloc<unsigned int>(1);
     Tableau tb = make_tableau();
     set_tableau(tb, stream);
+    const NyTableau ny = make_nystroem(tb, scheme);
+    d_ny = dalloc<NyTableau>(1);
+    CK(cudaMemcpy(d_ny, &ny, sizeof(ny), cudaMemcpyHostToDevice));
     build_plan();
     prep_positions();
     CK(cudaStreamSynchronize(stream));
@@ -797,6 +885,7 @@ void red_sim::build_plan()
             }
         }
     }
+    plan_try();
     // A plan of many waves whose tiles mostly hold 2 sinks per thread (FP32
     // modes) takes the packed-pair stage instance.
     // REDGB_PACKED=0 keeps the scalar instance.
@@ -863,6 +952,111 @@ void red_sim::build_plan()
         tile_cap = tiles;
         tile_cnt = dalloc<unsigned int>(tile_cap);
     }
+}
+
+// Whether the tries of this sim run as one cooperative launch each, and its
+// shape: one system, FP32 pair terms, up to kTryMaxLarge large bodies and small
+// ones that only these act on, whose accelerations of all stages fit in the
+// shared memory of the SMs.  At least 32 small bodies per CTA: with fewer, a
+// CTA's stage is no shorter and the exchange has more partials.  REDGB_TRY=0
+// keeps one launch per stage.
+void red_sim::plan_try()
+{
+    use_try = false;
+    const char* env = getenv("REDGB_TRY");
+    if (!allow_try || n_sys != 1 || (mode != MODE_MIXED && mode != MODE_FP32) || (env && env[0] == '0')) return;
+    const SysInfo& si = sinfo[0];
+    const int nl = si.n_SI, small = si.n - nl;
+    if (nl < 1 || nl > kTryMaxLarge || si.n_star > kTryMaxStars || small < 1 || si.n != si.n_massive) return;
+    int sms = 0, coop = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !coop)
+        return;
+    int g = std::max(nl, std::min(sms, (small + 31) / 32));
+    if (g > sms) return;
+    const int nb = (small + g - 1) / g;
+    g = std::max(nl, (small + nb - 1) / nb);
+    // the pull group: 384 threads, 256 for few bodies; with gas drag, whose body
+    // group has a thread per body, what is left of 1024.  Per large body,
+    // as many threads as the groups that form its sum have, with four small bodies
+    // or more each.
+    const bool drag = cfg.gas_disk == 1;
+    const int pull = drag ? 448 : (nb > 64 ? 384 : 256);
+    const int bodies = drag ? std::min(try_pad(nb), 448) : std::min((3 * nb + 31) / 32 * 32, 352);
+    const int owners = drag ? 128 : 32 + std::min(160, (g + 31) / 32 * 32);
+    const int pullers = drag ? pull + bodies : pull;
+    int lg = 2;
+    while (lg < 5 && (2 << lg) * nl <= pullers && try_pad(nb) >= 4 * (2 << lg)) lg++;
+    if (try_ctas_per_sm(mode, drag, pull + bodies + owners, try_smem(nb, n_stage, pull)) < 1) return;
+    const size_t recs = (size_t)nl * g * 4 + (size_t)nl * 8 * kTryCopies + g + nl + 1;
+    if (recs > try_cap) {
+        cudaFree(d_try);
+        d_try = nullptr;
+        try_cap = 0;
+        d_try = dalloc<uint4>(recs);
+        try_cap = recs;
+    }
+    if (!d_epoch) d_epoch = dalloc<unsigned>(1);
+    try_cta = g;
+    try_nb = nb;
+    try_pull = pull;
+    try_bodies = bodies;
+    try_owners = owners;
+    try_lanes = lg;
+    use_try = true;
+}
+
+TryParams red_sim::try_params()
+{
+    TryParams T;
+    memset(&T, 0, sizeof(T));
+    const SysInfo& si = sinfo[0];
+    T.scheme = scheme;
+    T.n_stage = n_stage;
+    T.adaptive = cfg.adaptive;
+    T.n_cta = try_cta;
+    T.nb = try_nb;
+    T.pull = try_pull;
+    T.bodies = try_bodies;
+    T.owners = try_owners;
+    T.lanes_log2 = try_lanes;
+    T.off = si.off;
+    T.n = si.n;
+    T.n_large = si.n_SI;
+    T.n_star = si.n_star;
+    T.sys = d_sys;
+    T.y_r = y_r;
+    T.y_v = y_v;
+    T.mass = mass; T.radius = radius; T.density = density; T.cd = cd; T.id = id;
+    T.pos_hi = pos_hi[0];
+    T.pos_lo = pos_lo[0];
+    T.tab = d_ny;
+    T.part = d_try;
+    T.pos = T.part + (size_t)si.n_SI * try_cta * 4;
+    T.err = T.pos + (size_t)si.n_SI * 8 * kTryCopies;
+    T.decision = T.err + try_cta + si.n_SI;
+    T.epoch = d_epoch;
+    T.gas = stage_params(0, false).gas;
+    T.ctl = control_params();
+    return T;
+}
+
+ControlParams red_sim::control_params()
+{
+    ControlParams C;
+    memset(&C, 0, sizeof(C));
+    C.n_sys = (int)n_sys;
+    C.scheme = scheme;
+    C.adaptive = cfg.adaptive;
+    C.order = order;
+    C.keep_dt = (scheme == SCHEME_EULER || scheme == SCHEME_RK2) ? 1 : 0;
+    C.exact = mode == MODE_FP64_EXACT ? 1 : 0;
+    C.tolerance = cfg.tolerance;
+    C.lambda = lambda;
+    C.output_interval = cfg.output_interval;
+    C.length = cfg.length;
+    C.sys = d_sys;
+    return C;
 }
 
 StageParams red_sim::stage_params(int s, bool standalone)
@@ -942,66 +1136,71 @@ void red_sim::enqueue_try(std::vector<int>* kinds, std::vector<cudaEvent_t>* evs
     mark(-1);
     const bool coll = cfg.threshold[RED_THRESHOLD_RADII_ENHANCE_FACTOR] > 0.0;
     const bool hash = coll && use_grid && !segs.empty();   // the small bodies' spatial hash
-    for (int s = 0; s < n_stage; s++) {
-        StageParams P = stage_params(s, false);
-        if (s == 0 && hash) {
-            P.head = d_head;
-            P.head_n = (long long)table_size;
+    if (tries_whole()) {
+        TryParams T = try_params();
+        if (hash) {
+            T.head = d_head;
+            T.next = d_next;
+            T.cell = d_cell;
+            T.grid = d_grid;
+            // schemes of up to two stages have no exchange that orders the clearing
+            // of the hash before the insertions of other CTAs
+            if (n_stage > 2) T.head_n = (long long)table_size;
+            else CK(cudaMemsetAsync(d_head, 0xff, table_size * sizeof(int), stream));
         }
-        if (items_override) P.items = items_override;
-        launch_stage(P, items_override ? n_items_override : (int)items.size(), mode, stream);
+        launch_try(T, mode, stream);
         mark(0);
         n++;
-    }
-    ControlParams C;
-    memset(&C, 0, sizeof(C));
-    C.n_sys = (int)n_sys;
-    C.scheme = scheme;
-    C.adaptive = cfg.adaptive;
-    C.order = order;
-    C.keep_dt = (scheme == SCHEME_EULER || scheme == SCHEME_RK2) ? 1 : 0;
-    C.exact = mode == MODE_FP64_EXACT ? 1 : 0;
-    C.tolerance = cfg.tolerance;
-    C.lambda = lambda;
-    C.output_interval = cfg.output_interval;
-    C.length = cfg.length;
-    C.sys = d_sys;
-    launch_control(C, stream);
-    mark(1);
-    n++;
-    FinishParams F;
-    memset(&F, 0, sizeof(F));
-    F.scheme = scheme;
-    F.adaptive = cfg.adaptive;
-    F.commit_from_stage4 = (scheme == SCHEME_RK4 && cfg.adaptive) ? 1 : 0;
-    F.stage_exact = cfg.stage_exact;
-    F.segs = d_fsegs;
-    F.sinfo = d_sinfo;
-    F.sys = d_sys;
-    F.y_r = y_r;
-    F.y_v = y_v;
-    for (int k = 0; k < kMaxStages; k++) {
-        F.Kr[k] = Kr[k];
-        F.Kv[k] = Kv[k];
-    }
-    F.t_r0 = tr[0];
-    F.mass = mass;
-    F.radius = radius;
-    F.id = id;
-    F.pos_hi0 = pos_hi[0];
-    F.pos_lo0 = pos_lo[0];
-    if (hash) {
-        F.head = d_head;
-        F.next = d_next;
-        F.cell = d_cell;
-        F.grid = d_grid;
-    }
-    launch_finish(F, (int)fsegs.size(), stream);
-    mark(2);
-    n++;
-    if (prop_on || log_on) {
-        enqueue_proposer(n);
-        mark(5);
+    } else {
+        for (int s = 0; s < n_stage; s++) {
+            StageParams P = stage_params(s, false);
+            if (s == 0 && hash) {
+                P.head = d_head;
+                P.head_n = (long long)table_size;
+            }
+            if (items_override) P.items = items_override;
+            launch_stage(P, items_override ? n_items_override : (int)items.size(), mode, stream);
+            mark(0);
+            n++;
+        }
+        const ControlParams C = control_params();
+        launch_control(C, stream);
+        mark(1);
+        n++;
+        FinishParams F;
+        memset(&F, 0, sizeof(F));
+        F.scheme = scheme;
+        F.adaptive = cfg.adaptive;
+        F.commit_from_stage4 = (scheme == SCHEME_RK4 && cfg.adaptive) ? 1 : 0;
+        F.stage_exact = cfg.stage_exact;
+        F.segs = d_fsegs;
+        F.sinfo = d_sinfo;
+        F.sys = d_sys;
+        F.y_r = y_r;
+        F.y_v = y_v;
+        for (int k = 0; k < kMaxStages; k++) {
+            F.Kr[k] = Kr[k];
+            F.Kv[k] = Kv[k];
+        }
+        F.t_r0 = tr[0];
+        F.mass = mass;
+        F.radius = radius;
+        F.id = id;
+        F.pos_hi0 = pos_hi[0];
+        F.pos_lo0 = pos_lo[0];
+        if (hash) {
+            F.head = d_head;
+            F.next = d_next;
+            F.cell = d_cell;
+            F.grid = d_grid;
+        }
+        launch_finish(F, (int)fsegs.size(), stream);
+        mark(2);
+        n++;
+        if (prop_on || log_on) {
+            enqueue_proposer(n);
+            mark(5);
+        }
     }
     if (coll) {
         CollParams Q;
@@ -2170,13 +2369,16 @@ int red_autotune(red_sim* sim)
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
-    struct Cand { int chunk, lanes; bool cluster, packed; };
+    struct Cand { int chunk, lanes; bool cluster, packed, whole; };
     std::vector<Cand> cands;
+    sim->allow_try = true;
+    sim->plan_try();
+    if (sim->tries_whole()) cands.push_back({0, 32, true, false, true});   // a try as one launch
     for (int lanes : {32, 16, 8}) {
-        cands.push_back({0, lanes, true, false});   // a cluster plan never takes the packed instance
+        cands.push_back({0, lanes, true, false, false});   // a cluster plan never takes the packed instance
         for (bool pk : {true, false}) {
-            cands.push_back({0, lanes, false, pk});
-            for (int c : {256, 512, 1024, 2048, 4096}) cands.push_back({c, lanes, false, pk});
+            cands.push_back({0, lanes, false, pk, false});
+            for (int c : {256, 512, 1024, 2048, 4096}) cands.push_back({c, lanes, false, pk, false});
         }
     }
     float best = 1e30f;
@@ -2187,8 +2389,9 @@ int red_autotune(red_sim* sim)
         sim->lanes_cap = c.lanes;
         sim->allow_cluster = c.cluster;
         sim->allow_packed = c.packed;
+        sim->allow_try = c.whole;
         sim->build_plan();
-        if (c.cluster && !sim->use_cluster && c.chunk == 0) continue;   // same plan as a later candidate
+        if (c.cluster && !sim->use_cluster && c.chunk == 0 && !c.whole) continue;   // same plan as a later candidate
         if (c.packed && !sim->use_packed) continue;                       // the same as its unpacked twin
         sim->prep_positions();
         sim->launch_tries(2);                  // graph capture, warm caches
@@ -2222,6 +2425,7 @@ int red_autotune(red_sim* sim)
     sim->lanes_cap = best_c.lanes;
     sim->allow_cluster = best_c.cluster;
     sim->allow_packed = best_c.packed;
+    sim->allow_try = best_c.whole || !cands[0].whole;   // not timed: as before
     sim->build_plan();
     swap_state(false);
     sim->ejhc_initial_done = ejhc_done;

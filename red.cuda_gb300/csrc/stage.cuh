@@ -224,14 +224,6 @@ __host__ __device__ constexpr int var_nk(int v)
 }
 constexpr int kNkMax = 9;                  // the most K operands of a variant (RKF7(8) stage 12)
 constexpr int kOpsMax = 3 + 2 * kNkMax;    // shared-memory operand slots
-// The time offset c_s of stage s (RKF7(8), RK4, RK2; Euler evaluates at t).
-__device__ __forceinline__ double stage_c(int scheme, int s)
-{
-    if (scheme == SCHEME_RKF78) return c_tb.c[s];
-    if (scheme == SCHEME_RK4) return c_tb.c4[s];
-    if (scheme == SCHEME_RK2) return c_tb.c2[s];
-    return 0.0;
-}
 
 // Thread-block cluster helpers (a tile's source chunks as one cluster): the
 // barrier in two halves (every thread of every CTA of the cluster arrives;

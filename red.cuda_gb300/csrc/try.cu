@@ -1,0 +1,812 @@
+// try.cu -- k_try: a whole try of one sparse system (try.cuh).
+#include "try.cuh"
+
+namespace redgb {
+
+namespace {
+
+// 16-byte records: three words and a tag, one 128-bit access each way.
+__device__ __forceinline__ void st_rec16(uint4* p, unsigned x, unsigned y, unsigned z, unsigned tag)
+{
+    asm volatile("{\n\t.reg .b128 q;\n\t.reg .b64 a, b;\n\tmov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\t"
+                 "mov.b128 q, {a, b};\n\tst.relaxed.gpu.global.b128 [%0], q;\n\t}\n" ::"l"(p), "r"(x), "r"(y), "r"(z),
+                 "r"(tag)
+                 : "memory");
+}
+__device__ __forceinline__ uint4 ld_rec16(const uint4* p)
+{
+    uint4 v;
+    asm volatile("{\n\t.reg .b128 q;\n\t.reg .b64 a, b;\n\tld.relaxed.gpu.global.b128 q, [%4];\n\t"
+                 "mov.b128 {a, b}, q;\n\tmov.b64 {%0, %1}, a;\n\tmov.b64 {%2, %3}, b;\n\t}\n"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(p)
+                 : "memory");
+    return v;
+}
+
+// Waits for the record with this tag.  A missing one stops the system; *dead
+// (shared memory) then ends the CTA's other waits.
+__device__ __noinline__ uint4 missing_record(DevSys* S, volatile int* dead)
+{
+    *dead = 1;
+    S->status = 4;   // RED_ERR_TIMEOUT
+    S->halted = 1;
+    return make_uint4(0x7fc00000u, 0x7fc00000u, 0x7fc00000u, 0u);
+}
+__device__ __forceinline__ uint4 poll16(const uint4* p, unsigned tag, DevSys* S, volatile int* dead)
+{
+    for (int k = 0; k < kTryPollLimit; k++) {
+        const uint4 v = ld_rec16(p);
+        if (v.w == tag) return v;
+        if ((k & 63) == 63 && *dead) break;
+    }
+    return missing_record(S, dead);
+}
+
+__device__ __forceinline__ void group_sync(int id, int threads)
+{
+    asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
+}
+
+// The acceleration m d / |d|^3 of a star of double-single mass m at (S, SL) on a
+// body at (H, L), added to (ax, ay, az).
+__device__ __forceinline__ void star_term(float4 S, float4 SL, float2 m, float4 H, float4 L, float2& ax, float2& ay,
+                                          float2& az)
+{
+    const float2 dx = dsn_sub(dsn(S.x, SL.x), dsn(H.x, L.x));
+    const float2 dy = dsn_sub(dsn(S.y, SL.y), dsn(H.y, L.y));
+    const float2 dz = dsn_sub(dsn(S.z, SL.z), dsn(H.z, L.z));
+    const float2 r2 = dsn_add(dsn_add(dsn_sqr(dx), dsn_sqr(dy)), dsn_sqr(dz));
+    const float2 ri = dsn_rsqrt(r2);
+    const float2 f = dsn_mul(m, dsn_mul(dsn_sqr(ri), ri));
+    ax = dsn_add(ax, dsn_mul(f, dx));
+    ay = dsn_add(ay, dsn_mul(f, dy));
+    az = dsn_add(az, dsn_mul(f, dz));
+}
+
+// One FP32 pair term of the body at (H, L) from a source (h, l) of mass h.w,
+// added to (x, y, z): the stage kernel's term (gravity_f32).
+template <int MODE>
+__device__ __forceinline__ void pair_term(float4 h, float4 l, float4 H, float4 L, float& x, float& y, float& z)
+{
+    float dx = h.x - H.x, dy = h.y - H.y, dz = h.z - H.z;
+    if (MODE == MODE_MIXED) {
+        dx += l.x - L.x;
+        dy += l.y - L.y;
+        dz += l.z - L.z;
+    }
+    const float ri = rsqrtf(fmaf(dz, dz, fmaf(dy, dy, fmaf(dx, dx, kEps2))));
+    const float sc = h.w * ri * (ri * ri);
+    x = fmaf(sc, dx, x);
+    y = fmaf(sc, dy, y);
+    z = fmaf(sc, dz, z);
+}
+
+// This CTA's copy of the large bodies' position records of stage s.
+__device__ __forceinline__ const uint4* pos_records(const TryParams& P, int s)
+{
+    return P.pos + (size_t)((s & 3) * kTryCopies + blockIdx.x % kTryCopies) * P.n_large * 2;
+}
+
+struct Ds3 {   // a double-single vector
+    float xh, xl, yh, yl, zh, zl;
+};
+__device__ __forceinline__ void fold(Ds3& a, float x, float y, float z)
+{
+    ds_add(a.xh, a.xl, x);
+    ds_add(a.yh, a.yl, y);
+    ds_add(a.zh, a.zl, z);
+}
+// The sum of a over `lanes` (4 .. 32) consecutive threads, a component to each:
+// lane 0 returns x, lane 1 y, lane 2 z (of every group of 4).  The first two
+// rounds halve the components a thread still carries.
+__device__ __forceinline__ float2 reduce_scatter(const Ds3& a, int lane, int lanes)
+{
+    const bool odd = lane & 1;
+    // round 1: even lanes keep (x, z), odd ones (y, -)
+    const float sh = odd ? a.xh : a.yh, sl = odd ? a.xl : a.yl;
+    float kh = odd ? a.yh : a.xh, kl = odd ? a.yl : a.xl, zh = a.zh, zl = a.zl;
+    float rh = __shfl_xor_sync(0xffffffffu, sh, 1), rl = __shfl_xor_sync(0xffffffffu, sl, 1);
+    ds_merge(kh, kl, rh, rl);
+    rh = __shfl_xor_sync(0xffffffffu, zh, 1);
+    rl = __shfl_xor_sync(0xffffffffu, zl, 1);
+    ds_merge(zh, zl, rh, rl);
+    // round 2: lanes 0, 1 keep x, y; lanes 2, 3 the z of their pair (the same in both)
+    const bool up = lane & 2;
+    rh = __shfl_xor_sync(0xffffffffu, up ? kh : zh, 2);
+    rl = __shfl_xor_sync(0xffffffffu, up ? kl : zl, 2);
+    kh = up ? zh : kh;
+    kl = up ? zl : kl;
+    ds_merge(kh, kl, rh, rl);
+    for (int m = 4; m < lanes; m <<= 1) {
+        rh = __shfl_xor_sync(0xffffffffu, kh, m);
+        rl = __shfl_xor_sync(0xffffffffu, kl, m);
+        ds_merge(kh, kl, rh, rl);
+    }
+    return dsn_norm(kh, kl);
+}
+
+// Adds a x to the double-single sum (h, l), rounding errors carried.
+__device__ __forceinline__ void ds_term(float& h, float& l, float2 a, float2 x)
+{
+    const float p = a.x * x.x;
+    const float e = fmaf(a.y, x.x, fmaf(a.x, x.y, fmaf(a.x, x.x, -p)));
+    float sum, t;
+    two_sum(h, p, sum, t);
+    h = sum;
+    l += t + e;
+}
+// sum a_q K_q over the terms [u0, u1) of the tableau for N components; K_q of
+// component c at k[q st + c].
+template <int N>
+__device__ __forceinline__ void row_sum(const NyTableau& T, int u0, int u1, const float2* k, int st, float2 (&out)[N])
+{
+    float h[N], l[N];
+#pragma unroll
+    for (int c = 0; c < N; c++) h[c] = l[c] = 0.f;
+#pragma unroll 2
+    for (int u = u0; u < u1; u++) {
+        const float4 m = *reinterpret_cast<const float4*>(&T.term[u]);
+        const float2* x = k + __float_as_int(m.z) * st;
+#pragma unroll
+        for (int c = 0; c < N; c++) ds_term(h[c], l[c], make_float2(m.x, m.y), x[c]);
+    }
+#pragma unroll
+    for (int c = 0; c < N; c++) out[c] = dsn_norm(h[c], l[c]);
+}
+template <int N>
+__device__ __forceinline__ void row_sum(const NyTableau& T, int row, const float2* k, int st, float2 (&out)[N])
+{
+    row_sum<N>(T, T.beg[row], T.beg[row + 1], k, st, out);
+}
+__device__ __forceinline__ float2 to_ds(double x)
+{
+    float2 a;
+    split_ds(x, a.x, a.y);
+    return a;
+}
+
+// The larger of a component's position and velocity errors, as bits (NaN above all).
+template <int N>
+__device__ __forceinline__ unsigned long long component_error(const NyTableau& T, int scheme, float2 dt,
+                                                              const float2* k, int st)
+{
+    float2 r[N];
+    row_sum(T, kTryRowER, k, st, r);
+    unsigned long long m = 0ull;
+#pragma unroll
+    for (int c = 0; c < N; c++) {
+        const float2 d = scheme == SCHEME_RKF78
+                             ? dsn_sub(dsn_sub(dsn_add(k[c], k[10 * st + c]), k[11 * st + c]), k[12 * st + c])
+                             : dsn_sub(k[3 * st + c], k[4 * st + c]);
+        const double er = fabs(dsn_to_double(dsn_mul(r[c], dt))), ev = fabs(dsn_to_double(d));
+        double e = fmax(er, ev);
+        if (er != er || ev != ev) e = __longlong_as_double(0x7ff8000000000000ll);
+        m = max(m, (unsigned long long)__double_as_longlong(e));
+    }
+    return m;
+}
+// The solution of N components from (y, v): y + dt (cb v) + dt^2 sum, v + dt sum.
+template <int N>
+__device__ __forceinline__ void solution(const NyTableau& T, double dt, float2 dt1, float2 dt2, const float2* k, int st,
+                                         double (&y)[N], double (&v)[N])
+{
+    float2 r[N], w[N];
+    row_sum(T, kTryRowRB, k, st, r);
+    row_sum(T, kTryRowVB, k, st, w);
+    const double cdt = T.cb * dt;
+#pragma unroll
+    for (int c = 0; c < N; c++) {
+        y[c] = fma(cdt, v[c], y[c]) + dsn_to_double(dsn_mul(r[c], dt2));
+        v[c] = v[c] + dsn_to_double(dsn_mul(w[c], dt1));
+    }
+}
+// The double-single position y + cdt v + inc.
+__device__ __forceinline__ float2 position(double y, double cdt, double v, float2 inc)
+{
+    return dsn_add(to_ds(fma(cdt, v, y)), inc);
+}
+__device__ __forceinline__ void put_comp(float4* hi, float4* lo, int b, int c, float2 x)
+{
+    reinterpret_cast<float*>(hi + b)[c] = x.x;
+    reinterpret_cast<float*>(lo + b)[c] = x.y;
+}
+
+__device__ __forceinline__ bool not_finite(double x)
+{
+    return ((__double_as_longlong(x) >> 52) & 0x7ff) == 0x7ff;
+}
+
+// The step control on a copy of the system record; the fields it sets go back.
+__device__ __noinline__ void control_of(const ControlParams& P, DevSys& C, unsigned long long err)
+{
+    control_system(P, C, err);
+}
+__device__ __forceinline__ void store_control(DevSys* S, const DevSys& C)
+{
+    S->t = C.t;
+    S->dt_try = C.dt_try;
+    S->dt_did = C.dt_did;
+    S->dt_next = C.dt_next;
+    S->n_tried = C.n_tried;
+    S->n_passed = C.n_passed;
+    S->n_failed = C.n_failed;
+    S->iter = C.iter;
+    S->accepted = C.accepted;
+    S->active = C.active;
+    S->quota = C.quota;
+    S->err_last = C.err_last;
+    if (C.status) S->status = C.status;   // else as it is: other CTAs may set these
+    if (C.halted) S->halted = C.halted;
+}
+
+// Gas drag of a body at (H, L) with velocity v, added to its acceleration g
+// (drag_factor_fast, common.cuh, with its FP64 part in double-single: GB300's
+// FP64 rate held a stage of the 65536-body gas-drag disk for ~7 us).  The gas
+// velocity and its difference from v are good to ~1e-13 of the difference, the
+// factor f is FP32 as there.
+__device__ __forceinline__ void gas_drag(const GasDev& G, double decr, float2 mstar, float4 H, float4 L,
+                                         const float2 (&v)[3], double cd, double radius, double density, float2* g)
+{
+    const float2 x = dsn(H.x, L.x), y = dsn(H.y, L.y);
+    const float2 r2 = dsn_add(dsn_sqr(x), dsn_sqr(y));   // 0 on the disk's axis: NaN drag, as red's pow(0, p < 0)
+    const float2 ir = dsn_rsqrt(r2);
+    const float r = r2.x * ir.x;
+    const float q = 2.0f * (float)G.eta[0] * powf(r, (float)G.eta[1]);
+    const float d = -q / (1.0f + sqrtf(1.0f - q));       // the gas speed is 1 + d of the circular one
+    const float2 mi = dsn_mul(mstar, ir);
+    float2 s = dsn_mul(dsn_mul(mi, dsn_rsqrt(mi)), ir);  // sqrt(m / r) / r
+    s = dsn_mul(s, dsn_norm(1.0f, d));
+    const float2 ux = dsn_sub(dsn_mul(dsn(-y.x, -y.y), s), v[0]), uy = dsn_sub(dsn_mul(x, s), v[1]);
+    const float h = (float)G.sch[0] * powf(r, (float)G.sch[1]);
+    const float zh = H.z / h;
+    const float arg = zh * zh;
+    float dens;
+    if (0.1f < r) {
+        dens = (float)G.rho[0] * powf(r, (float)G.rho[1]) * expf(-arg);
+    } else {
+        const float a = (float)G.rho[0] * powf(0.1f, (float)G.rho[1] - 4.0f);
+        dens = a * (r * r) * (r * r) * expf(-arg);
+    }
+    const float un = sqrtf(ux.x * ux.x + uy.x * uy.x + v[2].x * v[2].x);
+    const float f = (float)decr * ((3.0f * (float)cd * dens * un) / (8.0f * (float)radius * (float)density));
+    const float2 f2 = make_float2(f, 0.f);
+    g[0] = dsn_add(g[0], dsn_mul(f2, ux));
+    g[1] = dsn_add(g[1], dsn_mul(f2, uy));
+    g[2] = dsn_sub(g[2], dsn_mul(f2, v[2]));
+}
+
+struct OwnerSmem {   // of the CTA that owns a large body
+    float4 hi[kTryMaxLarge], lo[kTryMaxLarge];
+    float2 red[2][kTryMaxOwners / 32 - 1][3];
+    float2 k[kMaxStages][3];
+    unsigned long long err;
+    DevSys sys;   // CTA 0's copy of the system record
+};
+
+// The group of threads that owns large body k: per stage the sum of the
+// CTAs' partials, the pairs of the large bodies and the stars' terms, then the
+// body's position two stages on for everyone; at the end its solution.  CTA 0's
+// group decides over the try.  All warps but the last gather the partials; the
+// last one meanwhile forms what does not need them, and then the position.
+template <int MODE>
+__device__ __forceinline__ void run_owner(const TryParams& P, OwnerSmem& sm, const NyTableau& T, volatile int* dead,
+                                          unsigned tag0, double dt, const double* ly, const double* lv, int o)
+{
+    const int k = blockIdx.x, nl = P.n_large;
+    const int lane = o & 31, w = o >> 5, W = P.owners, GW = W / 32 - 1;   // warps that gather
+    DevSys* S = P.sys;
+    if (w < GW) {
+        for (int s = 0; s < P.n_stage; s++) {
+            Ds3 a{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            for (int j = o; j < P.n_cta; j += 32 * GW) {
+                const uint4* rec = P.part + ((size_t)((s & 1) * nl + k) * P.n_cta + j) * 2;
+                const uint4 p = poll16(rec, tag0 + 1 + s, S, dead), q = poll16(rec + 1, tag0 + 1 + s, S, dead);
+                ds_merge(a.xh, a.xl, __uint_as_float(p.x), __uint_as_float(p.y));
+                ds_merge(a.yh, a.yl, __uint_as_float(p.z), __uint_as_float(q.x));
+                ds_merge(a.zh, a.zl, __uint_as_float(q.y), __uint_as_float(q.z));
+            }
+            const float2 part = reduce_scatter(a, lane, 32);
+            if (lane < 3) sm.red[s & 1][w][lane] = part;
+            group_sync(2, W);   // two sets of `red`: the last warp reads one while the next is formed
+        }
+    }
+    const int body = P.off + k;
+    const float2 dt1 = to_ds(dt), dt2 = to_ds(dt * dt);
+    const int comp = min(lane, 2);
+    const double y = ly[3 * k + comp], v = lv[3 * k + comp];
+    if (w == GW) {
+        const bool live = P.id[body] > 0;
+        float mj[2];   // the masses of large bodies lane and lane + 32
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int j = lane + 32 * u;
+            mj[u] = j < nl && P.id[P.off + j] >= 0 ? __double2float_rn(P.mass[P.off + j]) : 0.f;
+        }
+        float2 ms = make_float2(0.f, 0.f);
+        if (lane < P.n_star) {
+            const double m = P.id[P.off + lane] < 0 ? 0.0 : P.mass[P.off + lane];
+            ms.x = __double2float_rn(m);
+            ms.y = __double2float_rn(m - (double)ms.x);
+        }
+        if (lane == 0) sm.err = 0ull;
+        for (int s = 0; s < P.n_stage; s++) {
+            if (s < 2) {
+                for (int e = lane; e < 3 * nl; e += 32)
+                    put_comp(sm.hi, sm.lo, e / 3, e % 3, to_ds(s == 0 ? ly[e] : fma(T.c[1] * dt, lv[e], ly[e])));
+            } else {
+                for (int e = lane; e < 2 * nl; e += 32) {
+                    const uint4 q = poll16(pos_records(P, s) + e, tag0 + 1 + s, S, dead);
+                    float* f = reinterpret_cast<float*>((e & 1 ? sm.lo : sm.hi) + (e >> 1));
+                    f[0] = __uint_as_float(q.x);
+                    f[1] = __uint_as_float(q.y);
+                    f[2] = __uint_as_float(q.z);
+                }
+            }
+            __syncwarp();
+            const float4 H = sm.hi[k], L = sm.lo[k];
+            Ds3 a{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const int j = lane + 32 * u;
+                if (j >= P.n_star && j < nl && j != k) {
+                    float4 h = sm.hi[j];
+                    h.w = mj[u];
+                    float px = 0.f, py = 0.f, pz = 0.f;
+                    pair_term<MODE>(h, sm.lo[j], H, L, px, py, pz);
+                    fold(a, px, py, pz);
+                }
+            }
+            if (lane < P.n_star && lane != k) {
+                float2 ax = make_float2(0.f, 0.f), ay = ax, az = ax;
+                star_term(sm.hi[lane], sm.lo[lane], ms, H, L, ax, ay, az);
+                ds_merge(a.xh, a.xl, ax.x, ax.y);
+                ds_merge(a.yh, a.yl, ay.x, ay.y);
+                ds_merge(a.zh, a.zl, az.x, az.y);
+            }
+            float2 g0 = reduce_scatter(a, lane, 32);
+            g0 = make_float2(__shfl_sync(0xffffffffu, g0.x, comp), __shfl_sync(0xffffffffu, g0.y, comp));
+            // the position of stage s + 2 but for the term of K_s, its row's last one if present
+            const bool more = s + 2 < P.n_stage;
+            float2 base = make_float2(0.f, 0.f), coef = base;
+            if (more) {
+                const int u0 = T.beg[s + 2];
+                int u1 = T.beg[s + 3];
+                if (u1 > u0 && T.term[u1 - 1].q == s) coef = dsn_mul(T.term[--u1].a, dt2);
+                float2 r[1];
+                row_sum<1>(T, u0, u1, &sm.k[0][comp], 3, r);
+                base = position(y, T.c[s + 2] * dt, v, dsn_mul(r[0], dt2));
+            }
+            group_sync(2, W);
+            const float2(*red)[3] = sm.red[s & 1];
+            float2 g = dsn_add(red[0][comp], g0);
+            if (GW > 2) g = dsn_add(g, dsn_add(red[1][comp], red[2][comp]));
+            else if (GW > 1) g = dsn_add(g, red[1][comp]);
+            if (GW > 4) g = dsn_add(g, dsn_add(red[3][comp], red[4][comp]));
+            else if (GW > 3) g = dsn_add(g, red[3][comp]);
+            if (!live) g = make_float2(0.f, 0.f);
+            if (more) {
+                const float2 x = dsn_add(base, dsn_mul(coef, g));
+                const float h1 = __shfl_sync(0xffffffffu, x.x, 1), h2 = __shfl_sync(0xffffffffu, x.x, 2);
+                const float l0 = __shfl_sync(0xffffffffu, x.y, 0), l2 = __shfl_sync(0xffffffffu, x.y, 2);
+                const float h0 = __shfl_sync(0xffffffffu, x.x, 0), l1 = __shfl_sync(0xffffffffu, x.y, 1);
+                if (lane < 2 * kTryCopies) {   // lanes 2 c, 2 c + 1: the two words of copy c
+                    uint4* rec = P.pos + ((size_t)(((s + 2) & 3) * kTryCopies + (lane >> 1)) * nl + k) * 2 + (lane & 1);
+                    st_rec16(rec, __float_as_uint(lane & 1 ? l0 : h0), __float_as_uint(lane & 1 ? l1 : h1),
+                             __float_as_uint(lane & 1 ? l2 : h2), tag0 + 3 + s);
+                }
+            }
+            if (lane < 3) sm.k[s][lane] = g;
+            __syncwarp();
+        }
+    }
+    // the solution, the error, the decision: the last warp; CTA 0's others gather the errors
+    double rn[1] = {y}, vn[1] = {v};
+    if (P.adaptive && w == GW) {
+        unsigned long long eb = component_error<1>(T, P.scheme, dt1, &sm.k[0][comp], 3);
+        const unsigned long long e1 = __shfl_sync(0xffffffffu, eb, 1), e2 = __shfl_sync(0xffffffffu, eb, 2);
+        eb = max(eb, max(e1, e2));
+        if (lane == 0) st_rec16(P.err + P.n_cta + k, (unsigned)eb, (unsigned)(eb >> 32), 0u, tag0 + 14);
+    }
+    if (P.adaptive && k == 0) {
+        if (w < GW) {
+            unsigned long long m = 0ull;
+            for (int j = o; j < P.n_cta + nl; j += 32 * GW) {
+                const uint4 q = poll16(P.err + j, tag0 + 14, S, dead);
+                m = max(m, ((unsigned long long)q.y << 32) | q.x);
+            }
+            atomicMax(&sm.err, m);
+        }
+        group_sync(2, W);
+        if (w == 0 && lane == 0) {
+            // accepted or not: control_system's test, before the rest of the step control
+            const double max_err = fabs(P.ctl.lambda * dt * __longlong_as_double((long long)sm.err));
+            st_rec16(P.decision, max_err <= P.ctl.tolerance ? 1u : 0u, 0u, 0u, tag0 + 15);
+        }
+    }
+    if (k == 0 && o == 0) {
+        control_of(P.ctl, sm.sys, P.adaptive ? sm.err : 0ull);
+        store_control(S, sm.sys);
+        *P.epoch = tag0 / 16 + 1;
+    }
+    if (w != GW) return;
+    solution<1>(T, dt, dt1, dt2, &sm.k[0][comp], 3, rn, vn);
+    bool accepted = true;
+    if (P.adaptive) {
+        unsigned acc = 0u;
+        if (lane == 0) acc = poll16(P.decision, tag0 + 15, S, dead).x;
+        accepted = __shfl_sync(0xffffffffu, acc, 0) == 1u;
+    }
+    if (lane < 3 && accepted) {
+        P.y_r[3 * body + lane] = rn[0];
+        P.y_v[3 * body + lane] = vn[0];
+        if (not_finite(rn[0]) || not_finite(vn[0])) S->status = 5;   // RED_ERR_NONFINITE
+        write_pos_c(P.pos_hi, P.pos_lo, body, lane, rn[0]);
+    }
+}
+
+}  // namespace
+
+// The pull of the small bodies bhi / blo [0, pad) on the large ones at stage s: a
+// record of this CTA's sums for each, 1 << P.lanes_log2 of the threads t per
+// large body.  The exchange waits for these records.
+template <int MODE>
+__device__ __forceinline__ void pull_large(const TryParams& P, int s, int t, int pad, const float4* bhi,
+                                           const float4* blo, const float4* si_hi, const float4* si_lo, unsigned tag)
+{
+    const int nl = P.n_large, lg = P.lanes_log2, LS = 1 << lg;
+    if ((t & ~31) >> lg >= nl) return;   // uniform over the warp
+    const int lane = t & (LS - 1), g = t >> lg, k = min(g, nl - 1);
+    const float4 H = si_hi[k], L = si_lo[k];
+    Ds3 a{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    for (int j0 = lane; j0 < pad; j0 += 16 << lg) {
+        float x = 0.f, y = 0.f, z = 0.f;
+        const int j1 = min(pad, j0 + (16 << lg));
+#pragma unroll 4
+        for (int j = j0; j < j1; j += LS) pair_term<MODE>(bhi[j], blo[j], H, L, x, y, z);
+        fold(a, x, y, z);
+    }
+    const float2 part = reduce_scatter(a, lane, LS);   // x, y, z in lanes 0, 1, 2
+    const int l0 = (t & 31) - lane;
+    const float yh = __shfl_sync(0xffffffffu, part.x, l0 + 1), yl = __shfl_sync(0xffffffffu, part.y, l0 + 1);
+    const float zh = __shfl_sync(0xffffffffu, part.x, l0 + 2), zl = __shfl_sync(0xffffffffu, part.y, l0 + 2);
+    if (lane < 2 && g < nl) {
+        uint4* rec = P.part + (((size_t)(s & 1) * nl + k) * P.n_cta + blockIdx.x) * 2;
+        if (lane == 0) st_rec16(rec, __float_as_uint(part.x), __float_as_uint(part.y), __float_as_uint(yh), tag);
+        else st_rec16(rec + 1, __float_as_uint(yl), __float_as_uint(zh), __float_as_uint(zl), tag);
+    }
+}
+
+// The accelerations of small bodies b, ... by the large ones, share p of them:
+// part 0 the stars, the others (or part 0 too, if it is alone) a share of the
+// protoplanets each.
+template <int MODE>
+__device__ __forceinline__ void pull_small(const TryParams& P, int p, int b, int cnt, int pad, int np, const float4* bhi,
+                                           const float4* blo, const float4* si_hi, const float4* si_lo,
+                                           const float2* star_m, float2* parts)
+{
+    const int nl = P.n_large;
+    if (p >= np) return;
+    for (; b < cnt; b += np > 1 ? pad : P.pull) {
+        const float4 H = bhi[b], L = blo[b];
+        float2 ax = make_float2(0.f, 0.f), ay = ax, az = ax;
+        if (p > 0 || np == 1) {
+            const int step = np > 1 ? np - 1 : 1;
+            Ds3 a{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            for (int k0 = P.n_star + (np > 1 ? p - 1 : 0); k0 < nl; k0 += 8 * step) {
+                float x = 0.f, y = 0.f, z = 0.f;
+                const int k1 = min(nl, k0 + 8 * step);
+#pragma unroll 4
+                for (int k = k0; k < k1; k += step) pair_term<MODE>(si_hi[k], si_lo[k], H, L, x, y, z);
+                fold(a, x, y, z);
+            }
+            ax = dsn_norm(a.xh, a.xl);
+            ay = dsn_norm(a.yh, a.yl);
+            az = dsn_norm(a.zh, a.zl);
+        }
+        if (p == 0)
+            for (int k = 0; k < P.n_star; k++) star_term(si_hi[k], si_lo[k], star_m[k], H, L, ax, ay, az);
+        float2* o = parts + 3 * (p * pad + b);
+        o[0] = ax;
+        o[1] = ay;
+        o[2] = az;
+    }
+}
+
+template <int MODE, bool DRAG>
+__global__ void __launch_bounds__(try_max_threads(DRAG)) k_try(const __grid_constant__ TryParams P)
+{
+    __shared__ float4 si_hi[2][kTryMaxLarge], si_lo[2][kTryMaxLarge];
+    __shared__ float2 star_m[kTryMaxStars];
+    __shared__ double ly[3 * kTryMaxLarge], lv[3 * kTryMaxLarge];   // the large bodies' state at the start of the try
+    __shared__ NyTableau T;
+    __shared__ OwnerSmem own;
+    __shared__ unsigned long long err_sm;
+    __shared__ int dead, take;
+    __shared__ struct { double dt, t; unsigned tag; int runs; } start;
+    extern __shared__ __align__(16) unsigned char dyn[];
+
+    const int t = threadIdx.x;
+    const int nl = P.n_large, ns = P.n_stage, nb = P.nb;
+    const int main = P.pull + P.bodies;
+    DevSys* S = P.sys;
+    const int b0 = nl + blockIdx.x * nb;
+    const int cnt = max(0, min(P.n - b0, nb));
+    const int first = P.off + b0;
+    const int pad = try_pad(nb), np = try_parts(nb, P.pull);
+    // 16-byte records first: the doubles' count may be odd
+    float4* bhi = reinterpret_cast<float4*>(dyn);            // [2][pad], by stage parity
+    float4* blo = bhi + 2 * pad;
+    float2* parts = reinterpret_cast<float2*>(blo + 2 * pad);   // [2][np][pad][3]
+    const int n3 = 3 * nb;
+    float2* ks = parts + (size_t)2 * np * 3 * pad;              // accelerations, [stage][nb][3]
+    double* yr = reinterpret_cast<double*>(ks + (size_t)ns * n3);   // [nb][3]
+    double* yv = yr + n3;
+
+    // ---- everything the try starts from, read before this CTA's first record, so
+    // before any CTA writes the solution ----
+    if (t >= P.pull && t < main) {
+        for (int b = t - P.pull; b < pad; b += P.bodies) {   // a thread per body here
+            float4 H = make_float4(1.0e9f, 0.f, 0.f, 0.f), L = make_float4(0.f, 0.f, 0.f, 0.f);   // no body: no mass
+            if (b < cnt) {
+                const int i = first + b;
+                const int id = P.id[i];
+                const double m = P.mass[i];
+                double y[3], v[3];
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    y[c] = P.y_r[3 * i + c];
+                    v[c] = P.y_v[3 * i + c];
+                }
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    yr[3 * b + c] = y[c];
+                    yv[3 * b + c] = v[c];
+                }
+                split_ds(y[0], H.x, L.x);
+                split_ds(y[1], H.y, L.y);
+                split_ds(y[2], H.z, L.z);
+                H.w = id >= 0 ? __double2float_rn(m) : 0.f;
+                L.w = id > 0 ? 1.f : 0.f;   // an inactive sink's gravity is zero
+            }
+            bhi[b] = H;
+            blo[b] = L;
+            bhi[pad + b] = H;
+            blo[pad + b] = L;
+        }
+    } else if (t < 3 * nl) {   // 3 n_large <= pull
+        const double y = P.y_r[3 * P.off + t], v = P.y_v[3 * P.off + t];
+        const int id = P.id[P.off + t / 3];
+        const double m = P.mass[P.off + t / 3];
+        ly[t] = y;
+        lv[t] = v;
+        float h, l;
+        split_ds(y, h, l);
+        reinterpret_cast<float*>(&si_hi[0][t / 3])[t % 3] = h;
+        reinterpret_cast<float*>(&si_lo[0][t / 3])[t % 3] = l;
+        if (t % 3 == 0) {
+            const double me = id >= 0 ? m : 0.0;
+            const float mh = __double2float_rn(me);
+            si_hi[0][t / 3].w = si_hi[1][t / 3].w = mh;
+            if (t / 3 < P.n_star) star_m[t / 3] = make_float2(mh, __double2float_rn(me - (double)mh));
+        }
+    } else if (t >= main) {
+        const int o = t - main;
+        const uint4* src = reinterpret_cast<const uint4*>(P.tab);
+        for (int k = o; k < (int)(sizeof(NyTableau) / 16); k += P.owners) reinterpret_cast<uint4*>(&T)[k] = src[k];
+        if (blockIdx.x == 0)
+            for (int k = o; k < (int)(sizeof(DevSys) / 4); k += P.owners)
+                reinterpret_cast<unsigned*>(&own.sys)[k] = reinterpret_cast<const volatile unsigned*>(S)[k];
+        if (o == 0) {   // one thread of a CTA: every thread's reads would queue up on these sectors for ~4 us
+            const volatile DevSys* V = S;
+            const double dt = V->dt_try, ts = V->t;
+            const unsigned ep = *(volatile unsigned*)P.epoch;
+            start.runs = V->active && !V->halted && V->quota != 0;
+            start.dt = dt;
+            start.t = ts;
+            start.tag = ep * 16u;
+            dead = 0;
+            err_sm = 0ull;
+        }
+    }
+    __syncthreads();
+    if (!start.runs) {   // uniform over the grid
+        if (blockIdx.x == 0 && t == 0) S->accepted = 0;
+        return;
+    }
+    const double dt = start.dt, tsys = start.t;
+    const unsigned tag0 = start.tag;
+    if (t < P.pull)   // the pull group fences this before its second record
+        for (long long k = (long long)blockIdx.x * P.pull + t; k < P.head_n; k += (long long)gridDim.x * P.pull)
+            P.head[k] = -1;
+    if (t >= main) {
+        if ((int)blockIdx.x < nl) run_owner<MODE>(P, own, T, &dead, tag0, dt, ly, lv, t - main);
+        return;
+    }
+    if (t < P.pull) {
+        const int share = np > 1 ? t / pad : 0, body = np > 1 ? t % pad : t;
+        for (int s = 0; s < ns; s++) {
+            const int q = s & 1;
+            pull_large<MODE>(P, s, t, pad, bhi + q * pad, blo + q * pad, si_hi[q], si_lo[q], tag0 + 1 + s);
+            pull_small<MODE>(P, share, body, cnt, pad, np, bhi + q * pad, blo + q * pad, si_hi[q], si_lo[q], star_m,
+                             parts + (size_t)q * np * 3 * pad);
+            if (s == 0 && P.head_n > 0) __threadfence();   // the cleared hash before the later records
+            group_sync(1, main);
+        }
+        return;
+    }
+
+    // ---- the body group: K of the previous stage, positions of the next ----
+    constexpr int N = DRAG ? 3 : 1;   // components of a thread; its item x: component x % 3 of body x / 3, or body x
+    const int tb = t - P.pull, items = DRAG ? cnt : 3 * cnt;
+    const float2 dt1 = to_ds(dt), dt2 = to_ds(dt * dt);
+    GridInfo grid{};
+    if (P.head) grid = *P.grid;
+    const float2 mstar = DRAG ? to_ds(P.mass[P.off]) : make_float2(0.f, 0.f);
+    for (int s = 0; s <= ns; s++) {
+        if (DRAG && s < ns)
+            pull_large<MODE>(P, s, t, pad, bhi + (s & 1) * pad, blo + (s & 1) * pad, si_hi[s & 1], si_lo[s & 1],
+                             tag0 + 1 + s);
+        double decr = 0.0;
+        if (DRAG && s > 0) decr = gas_reduction_factor<false>(P.gas, tsys + stage_c(P.scheme, s - 1) * dt);
+        for (int x = tb; x < items; x += P.bodies) {
+            const int b = DRAG ? x : x / 3, e = N * x;
+            float2* k = ks + e;
+            if (s > 0) {
+                const int q = (s - 1) & 1;
+                const float2* pt = parts + (size_t)q * np * 3 * pad + e;
+                const bool live = blo[b].w != 0.f;
+                float2 g[N];
+#pragma unroll
+                for (int c = 0; c < N; c++) {
+                    g[c] = pt[c];
+                    for (int u = 1; u < np; u++) g[c] = dsn_add(g[c], pt[3 * u * pad + c]);
+                    if (!live) g[c] = make_float2(0.f, 0.f);
+                }
+                if constexpr (DRAG) {
+                    if (!(1.0e-6 > decr)) {
+                        const float4 H = bhi[q * pad + b], L = blo[q * pad + b];
+                        float2 dv[N];
+                        row_sum(T, kTryRowV + s - 1, k, n3, dv);
+                        float2 v[3];
+#pragma unroll
+                        for (int c = 0; c < 3; c++) v[c] = dsn_add(to_ds(yv[e + c]), dsn_mul(dv[c], dt1));
+                        const int i = first + b;
+                        gas_drag(P.gas, decr, mstar, H, L, v, P.cd[i], P.radius[i], P.density[i], g);
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < N; c++) k[(size_t)(s - 1) * n3 + c] = g[c];
+            }
+            if (s + 1 < ns) {
+                const int q = (s + 1) & 1;
+                float2 r[N];
+                row_sum(T, s + 1, k, n3, r);
+                const double cdt = T.c[s + 1] * dt;
+#pragma unroll
+                for (int c = 0; c < N; c++)
+                    put_comp(bhi + q * pad, blo + q * pad, b, DRAG ? c : x % 3,
+                             position(yr[e + c], cdt, yv[e + c], dsn_mul(r[c], dt2)));
+            }
+        }
+        if (s == ns) break;
+        if (s == 0) {   // the large bodies' positions of stage 1
+            if (ns > 1)
+                for (int e = tb; e < 3 * nl; e += P.bodies)
+                    put_comp(si_hi[1], si_lo[1], e / 3, e % 3, to_ds(fma(T.c[1] * dt, lv[e], ly[e])));
+        } else if (s + 1 < ns) {
+            const int q = (s + 1) & 1;
+            for (int e = tb; e < 2 * nl; e += P.bodies) {
+                const uint4 v = poll16(pos_records(P, s + 1) + e, tag0 + 2 + s, S, &dead);
+                float* f = reinterpret_cast<float*>((e & 1 ? si_lo[q] : si_hi[q]) + (e >> 1));
+                f[0] = __uint_as_float(v.x);
+                f[1] = __uint_as_float(v.y);
+                f[2] = __uint_as_float(v.z);
+            }
+            // the last positions follow every CTA's clearing of the hash (n_stage > 3)
+            if (s + 2 == ns && P.head) __threadfence();
+        }
+        group_sync(1, main);
+    }
+
+    // ---- the error, the solution (formed while the decision is on its way) ----
+    if (P.adaptive) {
+        unsigned long long eb = 0ull;
+        for (int x = tb; x < items; x += P.bodies) eb = max(eb, component_error<N>(T, P.scheme, dt1, ks + N * x, n3));
+        for (int m = 16; m > 0; m >>= 1) eb = max(eb, __shfl_xor_sync(0xffffffffu, eb, m));
+        if ((tb & 31) == 0) atomicMax(&err_sm, eb);
+        group_sync(3, P.bodies);
+        if (tb == 0) st_rec16(P.err + blockIdx.x, (unsigned)err_sm, (unsigned)(err_sm >> 32), 0u, tag0 + 14);
+    }
+    for (int x = tb; x < items; x += P.bodies) {
+        const int e = N * x;
+        double y[N], v[N];
+#pragma unroll
+        for (int c = 0; c < N; c++) {
+            y[c] = yr[e + c];
+            v[c] = yv[e + c];
+        }
+        solution(T, dt, dt1, dt2, ks + e, n3, y, v);
+#pragma unroll
+        for (int c = 0; c < N; c++) {
+            yr[e + c] = y[c];
+            yv[e + c] = v[c];
+        }
+    }
+    if (P.adaptive) {
+        if (tb == 0) take = poll16(P.decision, tag0 + 15, S, &dead).x == 1u;
+        group_sync(3, P.bodies);
+        if (!take) return;
+    } else {
+        group_sync(3, P.bodies);
+    }
+    int* cell = reinterpret_cast<int*>(parts);   // the pull group has left it
+    bool bad = false;
+    for (int e = tb; e < 3 * cnt; e += P.bodies) {
+        const double r = yr[e], v = yv[e];
+        P.y_r[3 * first + e] = r;
+        P.y_v[3 * first + e] = v;
+        bad = bad || not_finite(r) || not_finite(v);
+        write_pos_c(P.pos_hi, P.pos_lo, first + e / 3, e % 3, r);
+        if (grid.enabled) cell[e] = cell_coord(r, grid.inv_h);
+    }
+    if (bad) S->status = 5;   // RED_ERR_NONFINITE
+    if (!grid.enabled) return;   // uniform
+    group_sync(3, P.bodies);
+    for (int b = tb; b < cnt; b += P.bodies) {
+        const int4 cl = make_int4(cell[3 * b], cell[3 * b + 1], cell[3 * b + 2], 0);
+        P.cell[first + b] = cl;
+        P.next[first + b] = atomicExch(&P.head[grid.toff + bucket_of(cl.x, cl.y, cl.z, grid.mask)], first + b);
+    }
+}
+
+namespace {
+typedef void (*TryKernel)(const TryParams);
+TryKernel try_kernel(int mode, bool drag)
+{
+    if (mode == MODE_MIXED) return drag ? k_try<MODE_MIXED, true> : k_try<MODE_MIXED, false>;
+    if (mode == MODE_FP32) return drag ? k_try<MODE_FP32, true> : k_try<MODE_FP32, false>;
+    return nullptr;
+}
+}  // namespace
+
+int try_ctas_per_sm(int mode, bool drag, int threads, size_t smem)
+{
+    TryKernel k = try_kernel(mode, drag);
+    int dev = 0, most = 0, n = 0;
+    if (!k || cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+        return 0;
+    cudaFuncAttributes a;
+    if (cudaFuncGetAttributes(&a, k) != cudaSuccess || smem + a.sharedSizeBytes > (size_t)most ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, threads, smem) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+
+void launch_try(const TryParams& P, int mode, cudaStream_t s)
+{
+    const bool drag = P.gas.enabled != 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)P.n_cta);
+    cfg.blockDim = dim3((unsigned)(P.pull + P.bodies + P.owners));
+    cfg.dynamicSmemBytes = try_smem(P.nb, P.n_stage, P.pull);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, try_kernel(mode, drag), P);
+}
+
+void set_tableau_try(const Tableau& tb, cudaStream_t s)
+{
+    cudaMemcpyToSymbolAsync(c_tb, &tb, sizeof(Tableau), 0, cudaMemcpyHostToDevice, s);
+}
+
+}  // namespace redgb

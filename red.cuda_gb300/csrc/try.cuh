@@ -1,0 +1,130 @@
+// try.cuh -- a whole try of one sparse system in one cooperative launch.
+//
+// A planetesimal disk has a handful of large bodies (stars and protoplanets, the
+// SI class) that everything feels, and many small bodies (the NSI class) that
+// only the large ones feel.  A small body's equations then need nothing but the
+// large bodies' positions, and the large bodies need one sum over the small
+// ones per stage.  k_try gives every CTA a range of small bodies for the whole
+// try: their state, their accelerations of all stages and the large bodies'
+// positions stay in shared memory; per stage the CTAs exchange only the partial
+// sums on the large bodies and the new positions of these.
+//
+// The stages run on accelerations alone.  With the stage velocity v_s = y_v + dt
+// sum_q a_sq K_q put into the stage position (Nystroem's form of the same
+// method),
+//   r_s = y_r + dt (c_s y_v + dt sum_q A_sq K_q),   A = a a,
+// and A_sq = 0 for q >= s - 1: the positions of stage s do not wait for the
+// accelerations of stage s - 1.  An exchange (partial sums to the CTA that owns a
+// large body, its new position back to all) therefore has the time of a whole
+// stage to complete, and stage velocities are formed only for gas drag.
+//
+// The accelerations are double-single, as the pair and star sums leave them (the
+// star term is good to ~2e-14), and so are the sums over them, good to 2^-47: the
+// positions y_r + dt c v_y are formed in FP64, the increments are added as
+// double-single, and the solution adds its increments to the FP64 state.  GB300
+// issues an FP64 warp instruction every 19 cycles and SM and a dependent one
+// takes 64; the ~12 FP32 instructions of a double-single term take 3.
+//
+// Bound: latency -- of the exchange, two trips through L2 per two stages, and of
+// the instruction chains of a phase (~2.7 us per phase on the 16384-body disk, 1.3
+// of them the pull on the large bodies, whose records the exchange waits for).
+// Measured against one launch per stage, per try: 16384-body disk, adaptive
+// RKF7(8), 115 -> 57 us; 65536-body gas-drag disk 418 -> 175 us; 2053-body disk,
+// RK4, 33.2 -> 21.2 us.  What that took besides the layout: the system record is
+// read by one thread of a CTA and the position records are written in kTryCopies
+// copies, because thousands of readers of one sector queue up for microseconds.
+//
+// Records: 16 bytes with a 32-bit tag of the try and stage, written and read as
+// one 128-bit access, so a record is complete when its tag is right and needs no
+// fence or reset.  Two sets of partial sums alternate by stage: a CTA writes a slot
+// again two stages later, when it has positions that the slot's reader formed
+// from it.  The positions take four sets: the group that sums body j's partials
+// can be three stages ahead of the group of body k, but not four, since the
+// partials of a stage wait for k's positions.  Every wait is bounded: after kTryPollLimit reads a
+// record counts as missing, the system's status becomes RED_ERR_TIMEOUT, the
+// system halts and no further wait is entered.  The launch is cooperative: all
+// its CTAs are resident together.
+#pragma once
+#include "common.cuh"
+#include "control.cuh"
+
+namespace redgb {
+
+constexpr int kTryMaxOwners = 192;     // threads of the owner group, at most
+constexpr int kTryMaxLarge = 64;       // large bodies of a system on this path
+constexpr int kTryMaxStars = 4;
+constexpr int kTryCopies = 8;          // of the position records: 1/8 of the CTAs wait on each
+constexpr int kTryPollLimit = 1 << 20;
+
+// Nystroem form of a scheme: its rows over the accelerations, nonzero terms only,
+// ascending stages.  Row s: the positions of stage s (dt^2 sum a K); kTryRowV + s:
+// the velocities (dt sum a K); kTryRowRB and kTryRowVB: the solution's positions
+// (dt^2) and velocities (dt); kTryRowER: the position error (dt).
+constexpr int kTryRowV = kMaxStages, kTryRowRB = 2 * kMaxStages, kTryRowVB = kTryRowRB + 1, kTryRowER = kTryRowVB + 1;
+constexpr int kTryRows = kTryRowER + 1;
+struct NyTerm {
+    float2 a;                // the coefficient, double-single
+    int q, pad;              // the stage
+};
+struct alignas(16) NyTableau {
+    NyTerm term[176];
+    double c[kMaxStages];    // sum of row s of a: the factor of dt y_v in stage s
+    double cb;               // sum of b
+    int beg[kTryRows + 1];   // row k: terms [beg[k], beg[k + 1])
+    int pad[2];
+};
+static_assert(sizeof(NyTableau) % 16 == 0, "copied by 16 bytes");
+
+struct TryParams {
+    int scheme, n_stage, adaptive;
+    int n_cta, nb;           // CTAs, small bodies of each (the last may have fewer)
+    int pull, bodies, owners;   // threads of the three groups
+    int lanes_log2;          // threads per large body in the partial sums (4 .. 32)
+    int off, n, n_large, n_star;
+    DevSys* sys;
+    double* y_r;
+    double* y_v;
+    const double* mass;
+    const double* radius;
+    const double* density;
+    const double* cd;
+    const int* id;
+    float4* pos_hi;          // stage-0 copies
+    float4* pos_lo;
+    const NyTableau* tab;
+    uint4* part;             // [2][n_large][n_cta][2]
+    uint4* pos;              // [4][kTryCopies][n_large][2]
+    uint4* err;              // [n_cta + n_large]
+    uint4* decision;         // [1]
+    unsigned* epoch;         // tries made by this kernel
+    GasDev gas;
+    ControlParams ctl;
+    int* head;               // the collision check's hash (null: none)
+    long long head_n;
+    int* next;
+    int4* cell;
+    const GridInfo* grid;
+};
+
+// Bytes of dynamic shared memory of a CTA with nb small bodies.
+__host__ __device__ constexpr int try_pad(int nb) { return (nb + 31) / 32 * 32; }
+// shares of the pair terms on a small body, one thread each
+__host__ __device__ constexpr int try_parts(int nb, int pull)
+{
+    return pull / try_pad(nb) < 1 ? 1 : (pull / try_pad(nb) > 4 ? 4 : pull / try_pad(nb));
+}
+__host__ __device__ constexpr size_t try_smem(int nb, int n_stage, int pull)
+{
+    return (size_t)try_pad(nb) * 2 * (2 * sizeof(float4) + (size_t)try_parts(nb, pull) * 3 * sizeof(float2)) +
+           (size_t)nb * 3 * (sizeof(float2) * n_stage + sizeof(double) * 2);
+}
+// Threads of a CTA at most.
+__host__ __device__ constexpr int try_max_threads(bool drag) { return drag ? 1024 : 928; }
+
+// CTAs of the cooperative launch that are resident at once per SM with this much
+// shared memory (0: none, or the query failed), and the launch.
+int try_ctas_per_sm(int mode, bool drag, int threads, size_t smem);
+void launch_try(const TryParams& P, int mode, cudaStream_t s);
+void set_tableau_try(const Tableau& tb, cudaStream_t s);
+
+}  // namespace redgb
