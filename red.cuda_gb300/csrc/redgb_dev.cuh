@@ -79,6 +79,8 @@ struct GravItem {
     int mstar_set;        // 1: mstar holds the mass of the system's first star (0 if inactive)
     float mstar_hi, mstar_lo;   // that mass, double-single
     int first_src, n_src;   // the tile's whole source list [first_src, first_src + n_src)
+    int n_rec;              // > 0: the tile's gravity is in this many records (pairs.cuh), it has no sources
+    int pad[3];
 };
 
 // Per-body kernels: one CTA per segment of one system.
@@ -160,6 +162,8 @@ struct StageParams {
     const int* id;
     double* partial;      // 3 doubles per record
     unsigned int* tile_cnt;
+    const float2* rec;    // pair records of the bodies [rec_b0, rec_b0 + rec_n) (pairs.cuh)
+    int rec_b0, rec_n;
     GasDev gas;
     int* head;            // stage 0 sets the collision check's bucket heads to -1 (not null)
     long long head_n;
@@ -253,11 +257,13 @@ constexpr unsigned long long kRecEmpty = 0x7ff0000000000001ull;
 // short_ctas (optional) accumulates the CTAs the system would need with chunks of
 // two source tiles; short_chunks selects those chunks for the plan.
 int count_sink_tiles(const SysInfo& si, int mode, int lanes_cap, long long* short_ctas);
+// pair_slots: the SI bodies after the stars have their gravity in pair records,
+// this many for the bodies of each block (pairs.cuh).
 // star_mass: the effective mass of the system's first star (0 if its id < 0), or
 // nullptr when the host does not hold it (the kernel then reads it).
 void plan_gravity_items(const SysInfo& si, int sys, int mode, int chunk_override, int lanes_cap, int tiles_all,
                         bool short_chunks, const double* star_mass, std::vector<GravItem>& items, size_t& part,
-                        int& tiles);
+                        int& tiles, const std::vector<int>* pair_slots = nullptr);
 
 // Host-side launchers (kernels.cu, stage_*.cu).  The stage kernel's mode
 // fixes the arithmetic of the stage combinations: FP64_EXACT combines in red's

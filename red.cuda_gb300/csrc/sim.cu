@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "redgb_dev.cuh"
+#include "pairs.cuh"
 #include "proposer.cuh"
 #include "try.cuh"
 #include "redgb.h"
@@ -279,7 +280,7 @@ int count_sink_tiles(const SysInfo& si, int mode, int lanes_cap, long long* shor
 
 void plan_gravity_items(const SysInfo& si, int s, int mode, int chunk_override, int lanes_cap, int tiles_all,
                         bool short_chunks, const double* star_mass, std::vector<GravItem>& items, size_t& part,
-                        int& tiles)
+                        int& tiles, const std::vector<int>* pair_slots)
 {
     // Two regimes.  When chunks of two source tiles keep the whole launch within
     // one wave (short_chunks), every chunk is two tiles, staged in shared memory
@@ -289,6 +290,32 @@ void plan_gravity_items(const SysInfo& si, int s, int mode, int chunk_override, 
     const int kTargetCtas = 8 * 6 * 152;
     GravClass cls[3];
     gravity_classes(si, mode, cls);
+    if (pair_slots) {   // the stars as sinks as usual; tiles of 32 records for the others
+        cls[0].s1 = si.n_star;
+        for (int b = si.n_star; b < si.n_SI; b += 32) {
+            GravItem g;
+            memset(&g, 0, sizeof(g));
+            g.sys = s;
+            g.sink0 = si.off + b;
+            g.nsink = std::min(32, si.n_SI - b);
+            g.nchunk = 1;
+            g.lanes = 4;
+            g.spt = 1;
+            g.cls = CLS_SI;
+            g.soff = si.off;
+            g.nstar = si.n_star;
+            g.nerr = si.n_err;
+            g.src0 = g.src1 = si.off;
+            g.tile = -1;
+            g.n_rec = (*pair_slots)[(b - si.n_star) / kPairBlock];
+            if (star_mass && si.n_star > 0) {
+                g.mstar_set = 1;
+                g.mstar_hi = (float)*star_mass;
+                g.mstar_lo = (float)(*star_mass - (double)g.mstar_hi);
+            }
+            items.push_back(g);
+        }
+    }
     for (const GravClass& q : cls) {
         const int nsink_all = q.s1 - q.s0;
         if (nsink_all <= 0) continue;
@@ -530,6 +557,20 @@ struct red_sim {
     int lanes_cap = 32;         // upper bound on threads per sink (autotuner)
     bool allow_cluster = true;  // the planner may lay chunk groups out as clusters (autotuner)
     bool allow_packed = true;   // plans of 2-sink tiles may take the packed-pair instance (autotuner)
+    // each pair of an all-pairs class once (pairs.cuh)
+    bool allow_pairs = true;    // (autotuner)
+    bool use_pairs = false;
+    std::vector<int> pair_slots;
+    std::vector<GravItem> pair_items;   // the tries' items then
+    GravItem* d_pair_items = nullptr;
+    size_t pair_items_cap = 0;
+    PairJob* d_jobs = nullptr;
+    size_t jobs_cap = 0;
+    int n_jobs = 0;
+    float2* d_rec = nullptr;
+    size_t rec_cap = 0;
+    void plan_pairs();
+    void launch_pair_records(int s);
     // whole tries in one cooperative launch (try.cuh), for one sparse system
     bool allow_try = true;      // (autotuner)
     bool use_try = false;
@@ -616,7 +657,7 @@ red_sim::~red_sim()
     cudaFree(partial); cudaFree(tile_cnt); cudaFree(d_sys); cudaFree(d_sinfo); cudaFree(d_items); cudaFree(d_sparse_items);
     cudaFree(d_segs); cudaFree(d_pairs); cudaFree(d_events); cudaFree(d_nev); cudaFree(d_u);
     cudaFree(d_grid); cudaFree(d_head); cudaFree(d_next); cudaFree(d_cell); cudaFree(d_fsegs);
-    cudaFree(d_try); cudaFree(d_epoch); cudaFree(d_ny);
+    cudaFree(d_jobs); cudaFree(d_rec); cudaFree(d_pair_items); cudaFree(d_try); cudaFree(d_epoch); cudaFree(d_ny);
     cudaFree(d_xfer);
     if (h_xfer) cudaFreeHost(h_xfer);
     if (h_sys) cudaFreeHost(h_sys);
@@ -815,6 +856,7 @@ void red_sim::build_plan()
     for (uint32_t s = 0; s < n_sys; s++) tiles_all += count_sink_tiles(sinfo[s], mode, lanes_cap, &short_ctas);
     const bool short_chunks = short_ctas <= 6 * 152;   // one wave at 6 CTAs per SM
     item_begin.assign(n_sys + 1, 0);
+    plan_pairs();
     for (uint32_t s = 0; s < n_sys; s++) {
         const SysHost& h = sh[s];
         SysInfo& si = sinfo[s];
@@ -854,6 +896,12 @@ void red_sim::build_plan()
             table += m;
         }
     }
+    // The tries' items with pair records; their partial records and counters are
+    // their own, since the two plans may run different stage instances.
+    pair_items.clear();
+    if (use_pairs)
+        plan_gravity_items(sinfo[0], 0, mode, 0, 32, tiles_all, false, &star_mass[0], pair_items, part, tiles,
+                           &pair_slots);
     // Cluster plan (FP32 modes): when every tile's chunks fit the two-tile
     // shared-memory buffer as kClusterChunks chunks and the whole launch, laid
     // out in clusters, is resident at once, a tile's chunks run as the CTAs of
@@ -907,6 +955,7 @@ void red_sim::build_plan()
         if (!vec.empty()) CK(cudaMemcpy(dptr, vec.data(), vec.size() * sizeof(T), cudaMemcpyHostToDevice));
     };
     upload(items, d_items, items_cap);
+    upload(pair_items, d_pair_items, pair_items_cap);
     upload(segs, d_segs, segs_cap);
     upload(fsegs, d_fsegs, fsegs_cap);
     upload(pairs, d_pairs, pairs_cap);
@@ -952,6 +1001,75 @@ void red_sim::build_plan()
         tile_cap = tiles;
         tile_cnt = dalloc<unsigned int>(tile_cap);
     }
+}
+
+// Whether the tries form each pair of the SI class once (pairs.cuh): one system
+// in the FP32 modes whose massive bodies all pull each other, kPairMin of them or
+// more.  REDGB_PAIRS=0 keeps one-sided tiles.
+void red_sim::plan_pairs()
+{
+    // One RKF7(8) try, one-sided / each pair once: 346 / 366 us at 4096 bodies, 629 /
+    // 501 at 6144, 903 / 647 at 8192 (MIXED; FP32 mode alike).
+    constexpr int kPairMin = 5120;
+    // Sub-blocks per job: jobs of a few waves (4 CTAs on each of 152 SMs) balance the
+    // SMs, longer ones leave fewer records.  16384 bodies: 1.84 ms per RKF7(8) try at
+    // two (1056 jobs), 1.86 at one; 65536, RK4 in FP32: 5.71 ms per try at eight (4160
+    // jobs), 5.80 at sixteen, 6.11 at 32 (before the pair terms lost an operation).
+    constexpr long long kPairJobs = 4096, kPairWaves = 2048;
+    use_pairs = false;
+    pair_slots.clear();
+    const char* env = getenv("REDGB_PAIRS");
+    if (!allow_pairs || n_sys != 1 || (mode != MODE_MIXED && mode != MODE_FP32) || (env && env[0] == '0')) return;
+    const SysInfo& si = sinfo[0];
+    const int n = si.n_SI - si.n_star;
+    if (si.n_massive != si.n_SI || n < kPairMin) return;
+    const int blocks = (n + kPairBlock - 1) / kPairBlock, subs = (n + kTile - 1) / kTile;
+    long long units = 0;
+    for (int b = 0; b < blocks; b++) units += subs - b * kPairSinks;
+    const int len = units < kPairWaves ? 1 : (int)std::max(2ll, units / kPairJobs);
+    std::vector<PairJob> jobs;
+    int slots = 0;
+    for (int b = 0; b < blocks; b++) {
+        int slot = b;
+        for (int j = b * kPairSinks; j < subs; j += len) jobs.push_back(PairJob{b, j, std::min(subs, j + len), slot++});
+        pair_slots.push_back(slot);
+        slots = std::max(slots, slot);
+    }
+    const size_t recs = (size_t)slots * n * 3;
+    if (recs * sizeof(float2) > (size_t)4 << 30) return;
+    if (recs > rec_cap) {
+        cudaFree(d_rec);
+        d_rec = nullptr;
+        rec_cap = 0;
+        d_rec = dalloc<float2>(recs);
+        rec_cap = recs;
+    }
+    if (jobs.size() > jobs_cap) {
+        cudaFree(d_jobs);
+        d_jobs = nullptr;
+        jobs_cap = 0;
+        d_jobs = dalloc<PairJob>(jobs.size());
+        jobs_cap = jobs.size();
+    }
+    CK(cudaMemcpy(d_jobs, jobs.data(), jobs.size() * sizeof(PairJob), cudaMemcpyHostToDevice));
+    n_jobs = (int)jobs.size();
+    use_pairs = true;
+}
+
+// The pair records of stage s.
+void red_sim::launch_pair_records(int s)
+{
+    const SysInfo& si = sinfo[0];
+    PairParams P;
+    memset(&P, 0, sizeof(P));
+    P.jobs = d_jobs;
+    P.sys = d_sys;
+    P.b0 = si.off + si.n_star;
+    P.n = si.n_SI - si.n_star;
+    P.pos_hi = pos_hi[s & 1];
+    P.pos_lo = pos_lo[s & 1];
+    P.rec = d_rec;
+    launch_pairs(P, n_jobs, mode, stream);
 }
 
 // Whether the tries of this sim run as one cooperative launch each, and its
@@ -1158,8 +1276,23 @@ void red_sim::enqueue_try(std::vector<int>* kinds, std::vector<cudaEvent_t>* evs
                 P.head = d_head;
                 P.head_n = (long long)table_size;
             }
-            if (items_override) P.items = items_override;
-            launch_stage(P, items_override ? n_items_override : (int)items.size(), mode, stream);
+            int n_launch = (int)items.size();
+            if (items_override) {
+                P.items = items_override;
+                n_launch = n_items_override;
+            } else if (use_pairs) {
+                launch_pair_records(s);
+                mark(0);
+                n++;
+                P.items = d_pair_items;
+                n_launch = (int)pair_items.size();
+                P.cluster = P.packed = 0;
+                P.one_wave = pair_items.size() <= (size_t)6 * 152 ? 1 : 0;
+                P.rec = d_rec;
+                P.rec_b0 = sinfo[0].off + sinfo[0].n_star;
+                P.rec_n = sinfo[0].n_SI - sinfo[0].n_star;
+            }
+            launch_stage(P, n_launch, mode, stream);
             mark(0);
             n++;
         }
@@ -2369,11 +2502,14 @@ int red_autotune(red_sim* sim)
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
-    struct Cand { int chunk, lanes; bool cluster, packed, whole; };
+    struct Cand { int chunk, lanes; bool cluster, packed, whole, pairs = false; };
     std::vector<Cand> cands;
     sim->allow_try = true;
     sim->plan_try();
     if (sim->tries_whole()) cands.push_back({0, 32, true, false, true});   // a try as one launch
+    sim->allow_pairs = true;
+    sim->plan_pairs();
+    if (sim->use_pairs) cands.push_back({0, 32, false, false, false, true});   // each pair once
     for (int lanes : {32, 16, 8}) {
         cands.push_back({0, lanes, true, false, false});   // a cluster plan never takes the packed instance
         for (bool pk : {true, false}) {
@@ -2390,6 +2526,7 @@ int red_autotune(red_sim* sim)
         sim->allow_cluster = c.cluster;
         sim->allow_packed = c.packed;
         sim->allow_try = c.whole;
+        sim->allow_pairs = c.pairs;
         sim->build_plan();
         if (c.cluster && !sim->use_cluster && c.chunk == 0 && !c.whole) continue;   // same plan as a later candidate
         if (c.packed && !sim->use_packed) continue;                       // the same as its unpacked twin
@@ -2425,7 +2562,8 @@ int red_autotune(red_sim* sim)
     sim->lanes_cap = best_c.lanes;
     sim->allow_cluster = best_c.cluster;
     sim->allow_packed = best_c.packed;
-    sim->allow_try = best_c.whole || !cands[0].whole;   // not timed: as before
+    sim->allow_try = best_c.whole || !cands[0].whole;    // not timed: as before
+    sim->allow_pairs = best_c.pairs || !cands[0].pairs;
     sim->build_plan();
     swap_state(false);
     sim->ejhc_initial_done = ejhc_done;

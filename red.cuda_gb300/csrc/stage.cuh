@@ -925,7 +925,8 @@ k_stage(const StageParams P, const int Vrt)
     int mine_k = 0;
     bool mine_ok = false;
     if constexpr (kF32) {
-        if (PK && it.spt == 2) gravity_f32_pair<MODE>(sm, P, it, staged, th, tl, mine_ds, mine_k, mine_ok);
+        if (it.n_rec > 0) {   // the pair records hold it (uniform)
+        } else if (PK && it.spt == 2) gravity_f32_pair<MODE>(sm, P, it, staged, th, tl, mine_ds, mine_k, mine_ok);
         else if (!PK && it.spt == 2) gravity_f32<MODE, 2>(sm, P, it, staged, th, tl, mine_ds, mine_k, mine_ok);
         else gravity_f32<MODE, 1>(sm, P, it, staged, th, tl, mine_ds, mine_k, mine_ok);
     } else if constexpr (kRedSum) {
@@ -1065,6 +1066,9 @@ k_stage(const StageParams P, const int Vrt)
         }
     } else if constexpr (kRedSum) {
         if (elem) a = mine;
+    } else if (kF32 && it.n_rec > 0) {
+        if (elem)
+            g_ds = sum_records_ds(P.rec + 3 * (long long)(it.sink0 - P.rec_b0) + t, 3LL * P.rec_n, 0, it.n_rec);
     } else {
         if (mine_ok) {
             if (kF32) acc2[3 * mine_k + mine_c] = mine_ds;
