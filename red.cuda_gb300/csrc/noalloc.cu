@@ -48,16 +48,19 @@ void* g_scratch_dev[kMaxDevices] = {nullptr};
 
 // Layout of the scratch array (offsets in bytes, 256-aligned).
 constexpr size_t kOffSys = 0;
-constexpr size_t kOffSinfo = 128;
-constexpr size_t kOffItems = 256;
+constexpr size_t kOffItems = 256;   // the system record before it
 constexpr size_t kOffTiles = kOffItems + kMaxItems * sizeof(GravItem);
 constexpr size_t kOffPos = ((kOffTiles + kMaxTiles * sizeof(unsigned) + 255) / 256) * 256;
 // then pos_hi (N float4), pos_lo (N float4), partial records (3 doubles each)
 
+// The FP32 positions of the bodies, and the counters and the system record cleared
+// (two memsets less per call).
 __global__ void k_noalloc_prep(int n, const double* r, const double* mass, const double* radius, const int* id,
-                               float4* hi, float4* lo)
+                               float4* hi, float4* lo, unsigned* tiles, int n_tiles, unsigned* sys)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < (int)(sizeof(DevSys) / sizeof(unsigned))) sys[i] = 0u;
+    for (int k = i; k < n_tiles; k += gridDim.x * blockDim.x) tiles[k] = 0u;
     if (i >= n) return;
     // the same double-single split as the allocating path (k_prep)
     redgb::write_pos(hi, lo, i, r[3 * i], r[3 * i + 1], r[3 * i + 2], id[i] >= 0 ? mass[i] : 0.0,
@@ -71,7 +74,9 @@ int redgb_set_error(int code, const char* msg);
 
 namespace {
 int fail(int code, const char* msg) { return redgb_set_error(code, msg); }
-static_assert(sizeof(DevSys) <= 128 && sizeof(SysInfo) <= 128, "scratch header layout");
+static_assert(sizeof(DevSys) <= kOffItems && sizeof(DevSys) % sizeof(unsigned) == 0 &&
+                  sizeof(DevSys) / sizeof(unsigned) <= 256,
+              "scratch header layout; cleared by the first block of k_noalloc_prep");
 }  // namespace
 
 extern "C" int red_calc_accel_noalloc(const red_accel_args_t* a)
@@ -143,7 +148,6 @@ extern "C" int red_calc_accel_noalloc(const red_accel_args_t* a)
     cudaStream_t st = (cudaStream_t)a->stream;
     unsigned char* b = (unsigned char*)base;
     DevSys* d_sys = (DevSys*)(b + kOffSys);
-    SysInfo* d_sinfo = (SysInfo*)(b + kOffSinfo);
     GravItem* d_items = (GravItem*)(b + kOffItems);
     unsigned* d_tiles = (unsigned*)(b + kOffTiles);
     float4* d_hi = (float4*)(b + kOffPos);
@@ -151,12 +155,10 @@ extern "C" int red_calc_accel_noalloc(const red_accel_args_t* a)
     double* d_part = (double*)(b + off_part);
 
     if (cudaMemcpyAsync(d_items, items.data(), items.size() * sizeof(GravItem), cudaMemcpyHostToDevice, st) !=
-            cudaSuccess ||
-        cudaMemsetAsync(d_tiles, 0, kMaxTiles * sizeof(unsigned), st) != cudaSuccess ||
-        cudaMemsetAsync(d_sys, 0, sizeof(DevSys), st) != cudaSuccess ||
-        cudaMemcpyAsync(d_sinfo, &si, sizeof(SysInfo), cudaMemcpyHostToDevice, st) != cudaSuccess)
+        cudaSuccess)
         return fail(RED_ERR_CUDA, "red_calc_accel_noalloc: staging the plan failed");
-    k_noalloc_prep<<<(n + 255) / 256, 256, 0, st>>>((int)n, a->r, a->mass, a->radius, a->id, d_hi, d_lo);
+    k_noalloc_prep<<<(n + 255) / 256, 256, 0, st>>>((int)n, a->r, a->mass, a->radius, a->id, d_hi, d_lo, d_tiles, tiles,
+                                                    (unsigned*)d_sys);
 
     StageParams P;
     memset(&P, 0, sizeof(P));
@@ -166,7 +168,6 @@ extern "C" int red_calc_accel_noalloc(const red_accel_args_t* a)
     P.standalone = 1;
     P.t_standalone = a->t;
     P.items = d_items;
-    P.sinfo = d_sinfo;
     P.sys = d_sys;
     P.pos_hi_in = d_hi;
     P.pos_lo_in = d_lo;

@@ -623,7 +623,7 @@ __device__ __forceinline__ void gravity_f64(SmemStage& sm, const StageParams& P,
 // adds all of them (sum_terms): its chain of dependent additions, ~110 cycles
 // each, is then all that is serial.  4100-body disk (9 large bodies), adaptive
 // RKF7(8): 57.6 ms per try when one lane formed and added the terms of its
-// sink in turn, 2.95 ms now.
+// sink in turn, 2.46 ms now.
 constexpr int kPairBatch = 512;
 constexpr int kPairStride = kPairBatch + 6;   // the components' rows start in different banks
 
@@ -695,21 +695,36 @@ __device__ __forceinline__ double gravity_exact(SmemStage& sm, double* terms, co
     return a;
 }
 
-// The n terms of one element of a chunked tile (`stride` doubles apart), added
-// in order: the next batch is loaded while one is added.
-__device__ __forceinline__ double sum_terms(const double* base, long long stride, int n)
+// The sums over the n sources of a chunked tile's terms (nel doubles per source,
+// contiguous), element threadIdx.x < nel, added in order.  All threads bring the
+// terms to shared memory, a batch ahead of the additions, so that these follow
+// each other at the latency of an FP64 addition (64 cycles).  (With each
+// element loading its own terms to registers, a batch ahead, an addition took
+// ~115 cycles: 2.95 ms per try of the 4100-body disk, 2.46 ms now.)
+__device__ __forceinline__ double sum_terms(const double* base, int nel, int n, double* buf)
 {
-    constexpr int kB = 24;
-    double cur[kB], nxt[kB], a = 0.0;
+    const int t = threadIdx.x;
+    constexpr int kV = (3 * kPairStride + kTile - 1) / kTile;   // terms per thread and batch
+    const int rows = 3 * kPairStride / nel;                     // sources per batch
+    double v[kV], a = 0.0;
+    auto fetch = [&](int r0) {   // past L1: another tile's reader may have left a line there before these were written
+        const int cnt = max(0, min(rows, n - r0)) * nel;
 #pragma unroll
-    for (int u = 0; u < kB; u++) cur[u] = u < n ? __ldcg(base + u * stride) : 0.0;
-    for (int b = 0; b < n; b += kB) {
+        for (int k = 0; k < kV; k++) v[k] = t + k * kTile < cnt ? __ldcg(base + (size_t)r0 * nel + t + k * kTile) : 0.0;
+    };
+    fetch(0);
+    for (int r0 = 0; r0 < n; r0 += rows) {
+        __syncthreads();
 #pragma unroll
-        for (int u = 0; u < kB; u++) nxt[u] = b + kB + u < n ? __ldcg(base + (b + kB + u) * stride) : 0.0;
-#pragma unroll
-        for (int u = 0; u < kB; u++) a = __dadd_rn(a, cur[u]);
-#pragma unroll
-        for (int u = 0; u < kB; u++) cur[u] = nxt[u];
+        for (int k = 0; k < kV; k++)
+            if (t + k * kTile < 3 * kPairStride) buf[t + k * kTile] = v[k];
+        __syncthreads();
+        fetch(r0 + rows);
+        if (t < nel) {
+            const int m = min(rows, n - r0);
+#pragma unroll 8
+            for (int u = 0; u < m; u++) a = __dadd_rn(a, buf[u * nel + t]);
+        }
     }
     return a;
 }
@@ -743,8 +758,7 @@ __device__ __forceinline__ double sum_terms(const double* base, long long stride
 // CTA hides more of it (512-disk ensemble stage -17 %, 65536-body gas-drag
 // disk -13 %, all-pairs 16384-body disk -1.3 %; 8 CTAs at 64 registers spill
 // and are slower).  The one-wave instance keeps 80 registers.
-// The red-exact instances keep 24 terms of a sum in flight (sum_terms) and hold
-// 12 KB of terms: 4 CTAs per SM.
+// The red-exact instances hold 12 KB of terms: 4 CTAs per SM.
 template <int MODE, bool EXACT, bool CL, int VT, bool PK = false>
 __global__ void __launch_bounds__(kTile, MODE == MODE_FP64_EXACT ? 4 : PK ? 6 : (VT >= 0 ? 7 : 6))
 k_stage(const StageParams P, const int Vrt)
@@ -1026,7 +1040,7 @@ k_stage(const StageParams P, const int Vrt)
             return;
         }
         if constexpr (kRedSum) {
-            if (elem) a = sum_terms(P.partial + 3 * (long long)it.part_off + t, 3LL * it.nsink, it.n_src);
+            a = sum_terms(P.partial + 3 * (long long)it.part_off, nel, it.n_src, terms);
             if (t == 0) P.tile_cnt[it.tile] = 0u;
         } else {
             const int nsplit = kTile / nel;
