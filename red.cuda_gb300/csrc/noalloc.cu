@@ -25,9 +25,9 @@
 // need scratch records) does not fit the array, the plan falls back to one
 // CTA per sink tile over the whole source list, which needs no partial
 // records and at most n / 16 + 3 work items.
+#include <algorithm>
 #include <cstring>
 #include <mutex>
-#include <vector>
 
 #include "common.cuh"
 #include "redgb.h"
@@ -53,14 +53,31 @@ constexpr size_t kOffTiles = kOffItems + kMaxItems * sizeof(GravItem);
 constexpr size_t kOffPos = ((kOffTiles + kMaxTiles * sizeof(unsigned) + 255) / 256) * 256;
 // then pos_hi (N float4), pos_lo (N float4), partial records (3 doubles each)
 
-// The FP32 positions of the bodies, and the counters and the system record cleared
-// (two memsets less per call).
+// The launch plan: the class plans, from which the items are made.
+struct PrepPlan {
+    SysInfo si;
+    int n_cls, n_items;
+    ClassPlan cls[3];
+};
+
+// The FP32 positions of the bodies, the stage kernel's work items, and the counters
+// and the system record cleared.  (Items made on the host and copied, and a memset
+// for each cleared array, cost as much as both kernels: 28 us per call for 20011
+// bodies, 18.4 us now.)
 __global__ void k_noalloc_prep(int n, const double* r, const double* mass, const double* radius, const int* id,
-                               float4* hi, float4* lo, unsigned* tiles, int n_tiles, unsigned* sys)
+                               float4* hi, float4* lo, unsigned* tiles, int n_tiles, unsigned* sys,
+                               const PrepPlan plan, GravItem* items)
 {
+    pdl_trigger();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < (int)(sizeof(DevSys) / sizeof(unsigned))) sys[i] = 0u;
     for (int k = i; k < n_tiles; k += gridDim.x * blockDim.x) tiles[k] = 0u;
+    if (i < plan.n_items) {
+        int q = i;
+        if (q < plan.cls[0].n_items) items[i] = class_item(plan.cls[0], plan.si, 0, q);
+        else if ((q -= plan.cls[0].n_items) < plan.cls[1].n_items) items[i] = class_item(plan.cls[1], plan.si, 0, q);
+        else items[i] = class_item(plan.cls[2], plan.si, 0, q - plan.cls[1].n_items);
+    }
     if (i >= n) return;
     // the same double-single split as the allocating path (k_prep)
     redgb::write_pos(hi, lo, i, r[3 * i], r[3 * i + 1], r[3 * i + 2], id[i] >= 0 ? mass[i] : 0.0,
@@ -106,23 +123,30 @@ extern "C" int red_calc_accel_noalloc(const red_accel_args_t* a)
     si.n_SI = (int)(a->playing[0] + a->playing[1] + a->playing[2] + a->playing[3]);
     si.n_massive = si.n_SI + (int)(a->playing[4] + a->playing[5]);
     si.n_err = si.n_massive;
-    std::vector<GravItem> items;
+    PrepPlan plan;
+    memset(&plan, 0, sizeof(plan));
+    plan.si = si;
     size_t part = 0;
     int tiles = 0;
+    auto count = [&]() {
+        plan.n_items = 0;
+        for (int k = 0; k < plan.n_cls; k++) plan.n_items += plan.cls[k].n_items;
+    };
     auto fits = [&]() {
-        return items.size() <= kMaxItems && (size_t)tiles <= kMaxTiles &&
+        return (size_t)plan.n_items <= kMaxItems && (size_t)tiles <= kMaxTiles &&
                off_part + part * 3 * sizeof(double) <= kScratchBytes;
     };
     long long short_ctas = 0;
     const int tiles_all = count_sink_tiles(si, a->precision, 32, &short_ctas);
-    plan_gravity_items(si, 0, a->precision, 0, 32, tiles_all, short_ctas <= 6 * 152, nullptr, items, part, tiles);
+    plan.n_cls = plan_classes(si, a->precision, 0, 32, tiles_all, short_ctas <= 6 * 152, part, tiles, plan.cls);
+    count();
     if (!fits()) {
         // unchunked: one chunk spans all n bodies, and 8 lanes per sink group
         // give tiles of >= 16 sinks, so no partial records and few items
-        items.clear();
         part = 0;
         tiles = 0;
-        plan_gravity_items(si, 0, a->precision, (int)n, 8, tiles_all, false, nullptr, items, part, tiles);
+        plan.n_cls = plan_classes(si, a->precision, (int)n, 8, tiles_all, false, part, tiles, plan.cls);
+        count();
     }
     if (!fits()) return fail(RED_ERR_ARG, "red_calc_accel_noalloc: the launch plan does not fit the scratch array");
 
@@ -154,11 +178,11 @@ extern "C" int red_calc_accel_noalloc(const red_accel_args_t* a)
     float4* d_lo = (float4*)(b + kOffPos + pos_bytes);
     double* d_part = (double*)(b + off_part);
 
-    if (cudaMemcpyAsync(d_items, items.data(), items.size() * sizeof(GravItem), cudaMemcpyHostToDevice, st) !=
-        cudaSuccess)
-        return fail(RED_ERR_CUDA, "red_calc_accel_noalloc: staging the plan failed");
-    k_noalloc_prep<<<(n + 255) / 256, 256, 0, st>>>((int)n, a->r, a->mass, a->radius, a->id, d_hi, d_lo, d_tiles, tiles,
-                                                    (unsigned*)d_sys);
+    // the position kernel also writes the launch plan's items; the stage kernel is
+    // scheduled beside it and waits for it (programmatic dependent launch)
+    const int prep = std::max((int)n, plan.n_items);
+    k_noalloc_prep<<<(prep + 255) / 256, 256, 0, st>>>((int)n, a->r, a->mass, a->radius, a->id, d_hi, d_lo, d_tiles, tiles,
+                                                       (unsigned*)d_sys, plan, d_items);
 
     StageParams P;
     memset(&P, 0, sizeof(P));
@@ -193,7 +217,10 @@ extern "C" int red_calc_accel_noalloc(const red_accel_args_t* a)
     P.gas.t1 = a->gas.t1;
     P.gas.e_folding_time = a->gas.e_folding_time;
     P.gas.gas_decrease = a->gas.gas_decrease;
-    launch_stage(P, (int)items.size(), a->precision, st);
+    const bool pdl = pdl_on();
+    set_pdl(true);
+    launch_stage(P, plan.n_items, a->precision, st);
+    set_pdl(pdl);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(RED_ERR_CUDA, cudaGetErrorString(e));
     return RED_OK;

@@ -70,18 +70,19 @@ struct GravItem {
     int chunk, nchunk;
     int tile;             // tile id: counter index when nchunk > 1
     int part_off;         // first partial record (red-exact mode: first pair term) of the tile
-    int lanes;            // threads per sink (4, 8, 16 or 32), lanes * nsink <= kTile
-    int cls;
     int soff;             // first body of the system; its stars are [soff, soff + nstar)
     int nstar;
     int nerr;             // bodies [soff, soff + nerr) enter the error norm
-    int spt;              // sinks per thread group (1, or 2 in the FP32 modes: lanes >= 8)
-    int mstar_set;        // 1: mstar holds the mass of the system's first star (0 if inactive)
-    float mstar_hi, mstar_lo;   // that mass, double-single
+    float mstar_hi, mstar_lo;   // the mass of the system's first star (0 if inactive), double-single
     int first_src, n_src;   // the tile's whole source list [first_src, first_src + n_src)
     int n_rec;              // > 0: the tile's gravity is in this many records (pairs.cuh), it has no sources
-    int pad[3];
+    signed char lanes;    // threads per sink (4, 8, 16 or 32), lanes * nsink <= kTile
+    signed char cls;
+    signed char spt;      // sinks per thread group (1, or 2 in the FP32 modes: lanes >= 8)
+    signed char mstar_set;   // 1: mstar_hi / lo are set
+    int pad[2];
 };
+static_assert(sizeof(GravItem) == 80, "read as five 16-byte words at the start of every stage CTA");
 
 // Per-body kernels: one CTA per segment of one system.
 struct Segment {
@@ -252,6 +253,50 @@ constexpr int kBatchRecords = 16;   // partial records loaded per batch by the r
 // sums them.
 constexpr unsigned long long kRecEmpty = 0x7ff0000000000001ull;
 
+// The work items of one gravity class of a system (plan_classes, sim.cu): its sinks
+// in tiles, each tile against its source list in chunks; the last tile may be
+// smaller and be cut differently.
+struct ClassPlan {
+    int cls;
+    int s0, nsink;        // sinks [s0, s0 + nsink), relative to the system
+    int j0, nsrc;         // sources
+    int lanes, spt, tile_sinks, ntile;
+    int chunk[2], nchunk[2];   // sources per chunk and chunks of a full tile, of the last one
+    int recs[2];          // partial records of such a tile
+    int part0, tile0;     // the class's first partial record and chunked tile
+    int n_items;
+};
+
+// Item q of the class, without the star's mass.
+__host__ __device__ inline GravItem class_item(const ClassPlan& c, const SysInfo& si, int sys, int q)
+{
+    const int full = (c.ntile - 1) * c.nchunk[0];
+    const int t = q < full ? q / c.nchunk[0] : c.ntile - 1;
+    const int l = t == c.ntile - 1 ? 1 : 0;
+    const int k = l ? q - full : q % c.nchunk[0];
+    GravItem g = {};
+    g.sys = sys;
+    g.sink0 = si.off + c.s0 + t * c.tile_sinks;
+    g.nsink = l ? c.nsink - t * c.tile_sinks : c.tile_sinks;
+    g.nchunk = c.nchunk[l];
+    g.chunk = k;
+    g.lanes = (signed char)c.lanes;
+    g.spt = (signed char)c.spt;
+    g.cls = (signed char)c.cls;
+    g.soff = si.off;
+    g.nstar = si.n_star;
+    g.nerr = si.n_err;
+    g.tile = c.nchunk[l] > 1 ? c.tile0 + (c.nchunk[0] > 1 ? t : 0) : -1;
+    g.part_off = c.part0 + t * c.recs[0];
+    g.first_src = si.off + c.j0;
+    g.n_src = c.nsrc;
+    const int a = k * c.chunk[l], b = a + c.chunk[l];
+    g.src0 = si.off + c.j0 + a;
+    g.src1 = si.off + c.j0 + (b < c.nsrc ? b : c.nsrc);
+    if (c.nsrc == 0) g.src0 = g.src1 = si.off;
+    return g;
+}
+
 // Host-side plan of the stage kernel for one system (sim.cu).
 // tiles_all: sink tiles of every system planned into the same launch (count_sink_tiles).
 // short_ctas (optional) accumulates the CTAs the system would need with chunks of
@@ -261,6 +306,10 @@ int count_sink_tiles(const SysInfo& si, int mode, int lanes_cap, long long* shor
 // this many for the bodies of each block (pairs.cuh).
 // star_mass: the effective mass of the system's first star (0 if its id < 0), or
 // nullptr when the host does not hold it (the kernel then reads it).
+// plan_classes: the class plans of one system, at most three; advances the
+// counts of partial records and chunked tiles.
+int plan_classes(const SysInfo& si, int mode, int chunk_override, int lanes_cap, int tiles_all, bool short_chunks,
+                 size_t& part, int& tiles, ClassPlan out[3], int si_sinks = -1);
 void plan_gravity_items(const SysInfo& si, int sys, int mode, int chunk_override, int lanes_cap, int tiles_all,
                         bool short_chunks, const double* star_mass, std::vector<GravItem>& items, size_t& part,
                         int& tiles, const std::vector<int>* pair_slots = nullptr);

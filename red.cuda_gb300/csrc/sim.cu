@@ -278,20 +278,85 @@ int count_sink_tiles(const SysInfo& si, int mode, int lanes_cap, long long* shor
     return n;
 }
 
+// Two regimes.  When chunks of two source tiles keep the whole launch within
+// one wave (short_chunks), every chunk is two tiles, staged in shared memory
+// at once: the launch is as short as its slowest CTA.  Otherwise the launch
+// should hold several waves of CTAs (6 resident on each of GB300's 152 SMs);
+// tiles_all counts the sink tiles of every system in it.  si_sinks >= 0: only
+// so many sinks of the SI class.
+int plan_classes(const SysInfo& si, int mode, int chunk_override, int lanes_cap, int tiles_all, bool short_chunks,
+                 size_t& part, int& tiles, ClassPlan out[3], int si_sinks)
+{
+    const int kTargetCtas = 8 * 6 * 152;
+    GravClass cls[3];
+    gravity_classes(si, mode, cls);
+    if (si_sinks >= 0) cls[0].s1 = si_sinks;
+    int n = 0;
+    for (const GravClass& q : cls) {
+        if (q.s1 - q.s0 <= 0) continue;
+        ClassPlan c;
+        memset(&c, 0, sizeof(c));
+        c.cls = q.cls;
+        c.s0 = q.s0;
+        c.nsink = q.s1 - q.s0;
+        c.j0 = q.j0;
+        c.nsrc = std::max(0, q.j1 - q.j0);
+        const int nsrc = c.nsrc;
+        class_shape(mode, c.nsink, nsrc, lanes_cap, c.lanes, c.spt);
+        c.tile_sinks = kTile / c.lanes * c.spt;
+        c.ntile = (c.nsink + c.tile_sinks - 1) / c.tile_sinks;
+        c.part0 = (int)part;
+        c.tile0 = tiles;
+        for (int l = 0; l < 2; l++) {   // a full tile, the last one
+            const int nsink = l ? c.nsink - (c.ntile - 1) * c.tile_sinks : c.tile_sinks;
+            int chunk = std::max(nsrc, 1);
+            if (mode == MODE_FP64_EXACT) {
+                // A class of few tiles and a long source list (the large bodies): the pair
+                // terms are formed by several CTAs, chunks of at least 32 sources and at
+                // most kExactCtas of them, and added in order by one.  A class with more
+                // tiles fills the GPU without chunks, whose terms pass through memory (24
+                // bytes each, kExactTerms at most).  chunk_override (an allocation-free
+                // caller) takes none.
+                if (chunk_override == 0 && nsrc > kTile && 2 * c.ntile <= kExactCtas &&
+                    part + (size_t)nsrc * c.nsink <= kExactTerms) {
+                    const long long w = ((long long)nsrc * c.ntile + kExactCtas - 1) / kExactCtas;
+                    chunk = (int)std::max(32ll, (w + 31) / 32 * 32);
+                }
+            } else {
+                if (chunk_override > 0) {
+                    chunk = chunk_override;
+                } else {
+                    // chunks of 2 to 4 source tiles, fewer when the launch already has enough
+                    // CTAs; no CTA's gravity then runs much longer than the others'
+                    const int want = std::max(1, kTargetCtas / std::max(1, tiles_all));
+                    const int w = (nsrc + want - 1) / want;
+                    chunk = short_chunks ? 2 * kTile
+                                         : std::min(std::max((w + kTile / 2) / kTile * kTile, 2 * kTile), 16 * kTile);
+                }
+                // the reducing CTA reads at most 2 batches of records per thread
+                const int max_chunks = 2 * kBatchRecords * std::max(1, kTile / (3 * nsink));
+                if ((nsrc + chunk - 1) / chunk > max_chunks)
+                    chunk = ((nsrc + max_chunks - 1) / max_chunks + kTile - 1) / kTile * kTile;
+                chunk = std::max(chunk, 1);
+            }
+            c.chunk[l] = chunk;
+            c.nchunk[l] = std::max(1, (nsrc + chunk - 1) / chunk);
+            c.recs[l] = c.nchunk[l] > 1 ? (mode == MODE_FP64_EXACT ? nsrc : c.nchunk[l]) * nsink : 0;
+        }
+        c.n_items = (c.ntile - 1) * c.nchunk[0] + c.nchunk[1];
+        part += (size_t)(c.ntile - 1) * c.recs[0] + c.recs[1];
+        tiles += (c.nchunk[0] > 1 ? c.ntile - 1 : 0) + (c.nchunk[1] > 1 ? 1 : 0);
+        out[n++] = c;
+    }
+    return n;
+}
+
 void plan_gravity_items(const SysInfo& si, int s, int mode, int chunk_override, int lanes_cap, int tiles_all,
                         bool short_chunks, const double* star_mass, std::vector<GravItem>& items, size_t& part,
                         int& tiles, const std::vector<int>* pair_slots)
 {
-    // Two regimes.  When chunks of two source tiles keep the whole launch within
-    // one wave (short_chunks), every chunk is two tiles, staged in shared memory
-    // at once: the launch is as short as its slowest CTA.  Otherwise the launch
-    // should hold several waves of CTAs (6 resident on each of GB300's 152 SMs);
-    // tiles_all counts the sink tiles of every system in it.
-    const int kTargetCtas = 8 * 6 * 152;
-    GravClass cls[3];
-    gravity_classes(si, mode, cls);
+    const size_t first = items.size();
     if (pair_slots) {   // the stars as sinks as usual; tiles of 32 records for the others
-        cls[0].s1 = si.n_star;
         for (int b = si.n_star; b < si.n_SI; b += 32) {
             GravItem g;
             memset(&g, 0, sizeof(g));
@@ -308,88 +373,21 @@ void plan_gravity_items(const SysInfo& si, int s, int mode, int chunk_override, 
             g.src0 = g.src1 = si.off;
             g.tile = -1;
             g.n_rec = (*pair_slots)[(b - si.n_star) / kPairBlock];
-            if (star_mass && si.n_star > 0) {
-                g.mstar_set = 1;
-                g.mstar_hi = (float)*star_mass;
-                g.mstar_lo = (float)(*star_mass - (double)g.mstar_hi);
-            }
             items.push_back(g);
         }
     }
-    for (const GravClass& q : cls) {
-        const int nsink_all = q.s1 - q.s0;
-        if (nsink_all <= 0) continue;
-        const int nsrc = std::max(0, q.j1 - q.j0);
-        int lanes, spt;
-        class_shape(mode, nsink_all, nsrc, lanes_cap, lanes, spt);
-        const int tile_sinks = kTile / lanes * spt;
-        const int ntile = (nsink_all + tile_sinks - 1) / tile_sinks;
-        for (int t = 0; t < ntile; t++) {
-            const int s0 = q.s0 + t * tile_sinks;
-            const int nsink = std::min(tile_sinks, q.s1 - s0);
-            int chunk = std::max(nsrc, 1);
-            if (mode == MODE_FP64_EXACT) {
-                // A class of few tiles and a long source list (the large bodies): the pair
-                // terms are formed by several CTAs, chunks of at least 32 sources and at
-                // most kExactCtas of them, and added in order by one.  A class with more
-                // tiles fills the GPU without chunks, whose terms pass through memory (24
-                // bytes each, kExactTerms at most).  chunk_override (an allocation-free
-                // caller) takes none.
-                if (chunk_override == 0 && nsrc > kTile && 2 * ntile <= kExactCtas &&
-                    part + (size_t)nsrc * nsink <= kExactTerms) {
-                    const long long c = ((long long)nsrc * ntile + kExactCtas - 1) / kExactCtas;
-                    chunk = (int)std::max(32ll, (c + 31) / 32 * 32);
-                }
-            } else {
-                if (chunk_override > 0) {
-                    chunk = chunk_override;
-                } else {
-                    // chunks of 2 to 4 source tiles, fewer when the launch already has enough
-                    // CTAs; no CTA's gravity then runs much longer than the others'
-                    const int want = std::max(1, kTargetCtas / std::max(1, tiles_all));
-                    const int c = (nsrc + want - 1) / want;
-                    chunk = short_chunks ? 2 * kTile
-                                         : std::min(std::max((c + kTile / 2) / kTile * kTile, 2 * kTile), 16 * kTile);
-                }
-                // the reducing CTA reads at most 2 batches of records per thread
-                const int nel = 3 * nsink;
-                const int max_chunks = 2 * kBatchRecords * std::max(1, kTile / nel);
-                if ((nsrc + chunk - 1) / chunk > max_chunks)
-                    chunk = ((nsrc + max_chunks - 1) / max_chunks + kTile - 1) / kTile * kTile;
-                chunk = std::max(chunk, 1);
-            }
-            const int nchunk = std::max(1, (nsrc + chunk - 1) / chunk);
-            GravItem g;
-            memset(&g, 0, sizeof(g));
-            g.sys = (int)s;
-            g.sink0 = si.off + s0;
-            g.nsink = nsink;
-            g.nchunk = nchunk;
-            g.lanes = lanes;
-            g.spt = spt;
-            g.cls = q.cls;
-            g.soff = si.off;
-            g.nstar = si.n_star;
-            g.nerr = si.n_err;
-            if (star_mass && si.n_star > 0) {
-                g.mstar_set = 1;
-                g.mstar_hi = (float)*star_mass;
-                g.mstar_lo = (float)(*star_mass - (double)g.mstar_hi);
-            }
-            g.tile = nchunk > 1 ? tiles++ : -1;
-            g.part_off = (int)part;
-            g.first_src = si.off + q.j0;
-            g.n_src = nsrc;
-            if (nchunk > 1) part += (size_t)(mode == MODE_FP64_EXACT ? nsrc : nchunk) * nsink;
-            for (int c = 0; c < nchunk; c++) {
-                g.chunk = c;
-                g.src0 = si.off + q.j0 + c * chunk;
-                g.src1 = si.off + std::min(q.j1, q.j0 + (c + 1) * chunk);
-                if (nsrc == 0) g.src0 = g.src1 = si.off;
-                items.push_back(g);
-            }
+    ClassPlan cls[3];
+    const int n = plan_classes(si, mode, chunk_override, lanes_cap, tiles_all, short_chunks, part, tiles, cls,
+                               pair_slots ? si.n_star : -1);
+    for (int k = 0; k < n; k++)
+        for (int q = 0; q < cls[k].n_items; q++) items.push_back(class_item(cls[k], si, s, q));
+    if (star_mass && si.n_star > 0)
+        for (size_t k = first; k < items.size(); k++) {
+            GravItem& g = items[k];
+            g.mstar_set = 1;
+            g.mstar_hi = (float)*star_mass;
+            g.mstar_lo = (float)(*star_mass - (double)g.mstar_hi);
         }
-    }
 }
 // Items of a cluster launch (FP32 modes): a tile whose source list is longer
 // than two tiles becomes kClusterChunks chunks, the CTAs of one cluster; the
@@ -418,9 +416,9 @@ static void plan_cluster_items(const SysInfo& si, int s, int mode, int lanes_cap
             g.sink0 = si.off + s0;
             g.nsink = std::min(tile_sinks, q.s1 - s0);
             g.nchunk = nchunk;
-            g.lanes = lanes;
-            g.spt = spt;
-            g.cls = q.cls;
+            g.lanes = (signed char)lanes;
+            g.spt = (signed char)spt;
+            g.cls = (signed char)q.cls;
             g.soff = si.off;
             g.nstar = si.n_star;
             g.nerr = si.n_err;
@@ -1286,8 +1284,8 @@ void red_sim::enqueue_try(std::vector<int>* kinds, std::vector<cudaEvent_t>* evs
                 n++;
                 P.items = d_pair_items;
                 n_launch = (int)pair_items.size();
-                P.cluster = P.packed = 0;
-                P.one_wave = pair_items.size() <= (size_t)6 * 152 ? 1 : 0;
+                P.cluster = P.one_wave = 0;
+                P.packed = 1;   // the instance that reads pair records
                 P.rec = d_rec;
                 P.rec_b0 = sinfo[0].off + sinfo[0].n_star;
                 P.rec_n = sinfo[0].n_SI - sinfo[0].n_star;

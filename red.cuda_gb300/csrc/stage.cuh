@@ -773,6 +773,8 @@ k_stage(const StageParams P, const int Vrt)
     __shared__ SmemStage sm;
     __shared__ double ops[kOpsMax][kMaxElem];
     __shared__ double terms[kRedSum ? 3 * kPairStride : 1];
+    constexpr bool kAlone = VT <= 0;   // instances that make standalone evaluations
+    if (kAlone && P.standalone) pdl_wait();   // the kernel before it may have written the items
     const GravItem it = P.items[blockIdx.x];
     const int s = P.stage;
     // Stage 0 follows the kernels that update the system records, y and the
@@ -781,7 +783,7 @@ k_stage(const StageParams P, const int Vrt)
     // after the last stage), y, ids, masses, K_q of stages <= s - 2 (the stage
     // velocity Kr[q] is written by stage q - 1, the acceleration Kv[q] by q).
     if (s == 0) {
-        pdl_wait();
+        if (!kAlone || !P.standalone) pdl_wait();
         if (P.head) {   // the collision check at the end of this try starts from an empty hash
             const long long nt = (long long)gridDim.x * blockDim.x;
             for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < P.head_n; k += nt) P.head[k] = -1;
@@ -939,7 +941,7 @@ k_stage(const StageParams P, const int Vrt)
     int mine_k = 0;
     bool mine_ok = false;
     if constexpr (kF32) {
-        if (it.n_rec > 0) {   // the pair records hold it (uniform)
+        if (PK && it.n_rec > 0) {   // the pair records hold it (uniform)
         } else if (PK && it.spt == 2) gravity_f32_pair<MODE>(sm, P, it, staged, th, tl, mine_ds, mine_k, mine_ok);
         else if (!PK && it.spt == 2) gravity_f32<MODE, 2>(sm, P, it, staged, th, tl, mine_ds, mine_k, mine_ok);
         else gravity_f32<MODE, 1>(sm, P, it, staged, th, tl, mine_ds, mine_k, mine_ok);
@@ -1080,7 +1082,7 @@ k_stage(const StageParams P, const int Vrt)
         }
     } else if constexpr (kRedSum) {
         if (elem) a = mine;
-    } else if (kF32 && it.n_rec > 0) {
+    } else if (PK && it.n_rec > 0) {
         if (elem)
             g_ds = sum_records_ds(P.rec + 3 * (long long)(it.sink0 - P.rec_b0) + t, 3LL * P.rec_n, 0, it.n_rec);
     } else {
