@@ -37,13 +37,13 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // 1, and with the programmatic-stream-serialization attribute while pdl_on()
 // holds on this thread.
 template <typename... KArgs, typename... Args>
-inline void launch_kx(void (*k)(KArgs...), unsigned grid, unsigned block, unsigned cluster, cudaStream_t s,
-                      Args&&... args)
+inline void launch_kx(void (*k)(KArgs...), unsigned grid, unsigned block, unsigned cluster, size_t smem,
+                      cudaStream_t s, Args&&... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute at[2];
     int na = 0;
@@ -66,7 +66,7 @@ inline void launch_kx(void (*k)(KArgs...), unsigned grid, unsigned block, unsign
 template <typename... KArgs, typename... Args>
 inline void launch_k(void (*k)(KArgs...), unsigned grid, unsigned block, cudaStream_t s, Args&&... args)
 {
-    launch_kx(k, grid, block, 1u, s, std::forward<Args>(args)...);
+    launch_kx(k, grid, block, 1u, (size_t)0, s, std::forward<Args>(args)...);
 }
 
 // ---------------------------------------------------------------------------

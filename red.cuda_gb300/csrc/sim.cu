@@ -577,8 +577,14 @@ struct red_sim {
     size_t try_cap = 0;
     unsigned* d_epoch = nullptr;
     NyTableau* d_ny = nullptr;
-    bool tries_whole() const { return use_try && !prop_on && !log_on; }   // the proposer reads Kv[0]
+    bool use_team = false;      // the same for an ensemble of sparse systems (k_team)
+    int team_cap = 0, n_team_ctas = 0;
+    TeamItem* d_teams = nullptr;
+    size_t teams_cap = 0;
+    bool tries_whole() const { return (use_try || use_team) && !prop_on && !log_on; }   // the proposer reads Kv[0]
     void plan_try();
+    void plan_team();
+    void launch_teams(bool hash);
     TryParams try_params();
     bool use_packed = false;    // the plan's stage launches take the packed-pair instance
     red_plan_info_t plan_info{};   // what the last red_autotune measured
@@ -655,7 +661,7 @@ red_sim::~red_sim()
     cudaFree(partial); cudaFree(tile_cnt); cudaFree(d_sys); cudaFree(d_sinfo); cudaFree(d_items); cudaFree(d_sparse_items);
     cudaFree(d_segs); cudaFree(d_pairs); cudaFree(d_events); cudaFree(d_nev); cudaFree(d_u);
     cudaFree(d_grid); cudaFree(d_head); cudaFree(d_next); cudaFree(d_cell); cudaFree(d_fsegs);
-    cudaFree(d_jobs); cudaFree(d_rec); cudaFree(d_pair_items); cudaFree(d_try); cudaFree(d_epoch); cudaFree(d_ny);
+    cudaFree(d_teams); cudaFree(d_jobs); cudaFree(d_rec); cudaFree(d_pair_items); cudaFree(d_try); cudaFree(d_epoch); cudaFree(d_ny);
     cudaFree(d_xfer);
     if (h_xfer) cudaFreeHost(h_xfer);
     if (h_sys) cudaFreeHost(h_sys);
@@ -932,6 +938,7 @@ void red_sim::build_plan()
         }
     }
     plan_try();
+    plan_team();
     // A plan of many waves whose tiles mostly hold 2 sinks per thread (FP32
     // modes) takes the packed-pair stage instance.
     // REDGB_PACKED=0 keeps the scalar instance.
@@ -1122,6 +1129,101 @@ void red_sim::plan_try()
     use_try = true;
 }
 
+// Whether an ensemble's tries run as one cluster launch each (k_team): every system
+// sparse, as for plan_try, with up to kTeamLarge large bodies and no gas drag.  A
+// team's size: the fewest CTAs of kTeamBodies small bodies, or of fewer bodies
+// (down to 128) as long as all teams are resident at once.  Teams are packed into
+// clusters largest first.  REDGB_TRY=0 keeps one launch per stage.
+void red_sim::plan_team()
+{
+    use_team = false;
+    const char* env = getenv("REDGB_TRY");
+    if (!allow_try || n_sys < 2 || (mode != MODE_MIXED && mode != MODE_FP32) || cfg.gas_disk ||
+        (env && env[0] == '0'))
+        return;
+    for (const SysInfo& si : sinfo) {
+        const int small = si.n - si.n_SI;
+        if (si.n_SI < 1 || si.n_SI > kTeamLarge || si.n_star > kTryMaxStars || small < 1 || si.n != si.n_massive ||
+            small > kTeamCtas * kTeamBodies)
+            return;
+    }
+    const int resident = kTeamCtas * team_clusters(mode, team_smem(kTeamBodies, n_stage));
+    if (resident < kTeamCtas) return;
+    auto size_of = [](const SysInfo& si, int nb) { return std::min(kTeamCtas, (si.n - si.n_SI + nb - 1) / nb); };
+    int nb = kTeamBodies;
+    for (int b : {128, 192, 256, 384}) {
+        long long ctas = 0;
+        for (const SysInfo& si : sinfo) ctas += size_of(si, b);
+        if (ctas <= resident) {
+            nb = b;
+            break;
+        }
+    }
+    std::vector<int> order(n_sys);
+    for (uint32_t s = 0; s < n_sys; s++) order[s] = (int)s;
+    auto size_at = [&](int s) { return std::max(size_of(sinfo[s], nb), size_of(sinfo[s], kTeamBodies)); };
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+        const int sa = size_at(a), sb = size_at(b);
+        if (sa != sb) return sa > sb;
+        return sinfo[a].n > sinfo[b].n;
+    });
+    std::vector<TeamItem> teams;
+    std::vector<int> used;           // CTAs taken per cluster
+    std::vector<size_t> open(kTeamCtas + 1, 0);   // first cluster that may have room for a team of this size
+    team_cap = 0;
+    for (int s : order) {
+        const int size = size_at(s);
+        size_t c = open[size];
+        while (c < used.size() && used[c] + size > kTeamCtas) c++;
+        open[size] = c;
+        if (c == used.size()) {
+            used.push_back(0);
+            teams.resize(teams.size() + kTeamCtas, TeamItem{-1, 0, 1, 0});
+        }
+        for (int r = 0; r < size; r++) teams[c * kTeamCtas + used[c] + r] = TeamItem{s, r, size, used[c]};
+        used[c] += size;
+        team_cap = std::max(team_cap, (sinfo[s].n - sinfo[s].n_SI + size - 1) / size);
+    }
+    if (teams.size() > teams_cap) {
+        cudaFree(d_teams);
+        d_teams = nullptr;
+        teams_cap = 0;
+        d_teams = dalloc<TeamItem>(teams.size());
+        teams_cap = teams.size();
+    }
+    CK(cudaMemcpy(d_teams, teams.data(), teams.size() * sizeof(TeamItem), cudaMemcpyHostToDevice));
+    n_team_ctas = (int)teams.size();
+    use_team = true;
+}
+
+void red_sim::launch_teams(bool hash)
+{
+    TeamParams T;
+    memset(&T, 0, sizeof(T));
+    T.scheme = scheme;
+    T.n_stage = n_stage;
+    T.adaptive = cfg.adaptive;
+    T.cap = team_cap;
+    T.items = d_teams;
+    T.sinfo = d_sinfo;
+    T.sys = d_sys;
+    T.y_r = y_r;
+    T.y_v = y_v;
+    T.mass = mass;
+    T.id = id;
+    T.pos_hi = pos_hi[0];
+    T.pos_lo = pos_lo[0];
+    T.tab = d_ny;
+    T.ctl = control_params();
+    if (hash) {
+        T.head = d_head;
+        T.next = d_next;
+        T.cell = d_cell;
+        T.grid = d_grid;
+    }
+    launch_team(T, n_team_ctas, mode, stream);
+}
+
 TryParams red_sim::try_params()
 {
     TryParams T;
@@ -1252,7 +1354,11 @@ void red_sim::enqueue_try(std::vector<int>* kinds, std::vector<cudaEvent_t>* evs
     mark(-1);
     const bool coll = cfg.threshold[RED_THRESHOLD_RADII_ENHANCE_FACTOR] > 0.0;
     const bool hash = coll && use_grid && !segs.empty();   // the small bodies' spatial hash
-    if (tries_whole()) {
+    if (tries_whole() && use_team) {
+        launch_teams(hash);
+        mark(0);
+        n++;
+    } else if (tries_whole()) {
         TryParams T = try_params();
         if (hash) {
             T.head = d_head;
@@ -1432,7 +1538,7 @@ void red_sim::launch_tries(uint32_t n)
 // are still pending.
 bool red_sim::launch_sparse_try(const std::vector<DevSys>& ds)
 {
-    if (item_begin.size() != n_sys + 1 || !graph || ds.size() != n_sys) return false;
+    if (item_begin.size() != n_sys + 1 || !graph || ds.size() != n_sys || tries_whole()) return false;
     sparse_items.clear();
     for (uint32_t s = 0; s < n_sys; s++) {
         const DevSys& d = ds[s];
@@ -2504,6 +2610,7 @@ int red_autotune(red_sim* sim)
     std::vector<Cand> cands;
     sim->allow_try = true;
     sim->plan_try();
+    sim->plan_team();
     if (sim->tries_whole()) cands.push_back({0, 32, true, false, true});   // a try as one launch
     sim->allow_pairs = true;
     sim->plan_pairs();

@@ -1250,7 +1250,8 @@ void launch_stage_variant(const StageParams& P, int n, int v, cudaStream_t s)
     if constexpr (MODE == MODE_MIXED || MODE == MODE_FP32) {
         if (P.cluster) {
             stage_attributes<MODE, EXACT>();
-            launch_kx(k_stage<MODE, EXACT, true, -1>, (unsigned)n, (unsigned)kTile, (unsigned)kClusterChunks, s, P,
+            launch_kx(k_stage<MODE, EXACT, true, -1>, (unsigned)n, (unsigned)kTile, (unsigned)kClusterChunks,
+                      (size_t)0, s, P,
                       v);
             return;
         }

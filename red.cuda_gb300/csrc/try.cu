@@ -1,4 +1,5 @@
-// try.cu -- k_try: a whole try of one sparse system (try.cuh).
+// try.cu -- k_try: a whole try of one sparse system; k_team: of an ensemble of them
+// (try.cuh).
 #include "try.cuh"
 
 namespace redgb {
@@ -201,10 +202,23 @@ __device__ __forceinline__ void solution(const NyTableau& T, double dt, float2 d
         v[c] = v[c] + dsn_to_double(dsn_mul(w[c], dt1));
     }
 }
+// FP32 mode takes a coordinate's high word alone, truncated as split_ds does: a
+// word rounded away from zero goes one ulp back, into the low word.
+template <int MODE>
+__device__ __forceinline__ float2 coordinate(float2 x)
+{
+    if (MODE == MODE_FP32 && x.x * x.y < 0.f) {
+        const float h = __uint_as_float(__float_as_uint(x.x) - 1u);
+        x.y += x.x - h;
+        x.x = h;
+    }
+    return x;
+}
 // The double-single position y + cdt v + inc.
+template <int MODE>
 __device__ __forceinline__ float2 position(double y, double cdt, double v, float2 inc)
 {
-    return dsn_add(to_ds(fma(cdt, v, y)), inc);
+    return coordinate<MODE>(dsn_add(to_ds(fma(cdt, v, y)), inc));
 }
 __device__ __forceinline__ void put_comp(float4* hi, float4* lo, int b, int c, float2 x)
 {
@@ -375,7 +389,7 @@ __device__ __forceinline__ void run_owner(const TryParams& P, OwnerSmem& sm, con
                 if (u1 > u0 && T.term[u1 - 1].q == s) coef = dsn_mul(T.term[--u1].a, dt2);
                 float2 r[1];
                 row_sum<1>(T, u0, u1, &sm.k[0][comp], 3, r);
-                base = position(y, T.c[s + 2] * dt, v, dsn_mul(r[0], dt2));
+                base = dsn_add(to_ds(fma(T.c[s + 2] * dt, v, y)), dsn_mul(r[0], dt2));
             }
             group_sync(2, W);
             const float2(*red)[3] = sm.red[s & 1];
@@ -386,7 +400,7 @@ __device__ __forceinline__ void run_owner(const TryParams& P, OwnerSmem& sm, con
             else if (GW > 3) g = dsn_add(g, red[3][comp]);
             if (!live) g = make_float2(0.f, 0.f);
             if (more) {
-                const float2 x = dsn_add(base, dsn_mul(coef, g));
+                const float2 x = coordinate<MODE>(dsn_add(base, dsn_mul(coef, g)));
                 const float h1 = __shfl_sync(0xffffffffu, x.x, 1), h2 = __shfl_sync(0xffffffffu, x.x, 2);
                 const float l0 = __shfl_sync(0xffffffffu, x.y, 0), l2 = __shfl_sync(0xffffffffu, x.y, 2);
                 const float h0 = __shfl_sync(0xffffffffu, x.x, 0), l1 = __shfl_sync(0xffffffffu, x.y, 1);
@@ -447,16 +461,15 @@ __device__ __forceinline__ void run_owner(const TryParams& P, OwnerSmem& sm, con
 
 }  // namespace
 
-// The pull of the small bodies bhi / blo [0, pad) on the large ones at stage s: a
-// record of this CTA's sums for each, 1 << P.lanes_log2 of the threads t per
-// large body.  The exchange waits for these records.
+// The pull of the small bodies bhi / blo [0, pad) on large body k: the sum over
+// the 1 << lg threads of a group.  pull_large: a record of this CTA's sums at
+// stage s for each large body, by the threads t.  The exchange waits for these
+// records.
 template <int MODE>
-__device__ __forceinline__ void pull_large(const TryParams& P, int s, int t, int pad, const float4* bhi,
-                                           const float4* blo, const float4* si_hi, const float4* si_lo, unsigned tag)
+__device__ __forceinline__ float2 large_sum(int lane, int lg, int k, int pad, const float4* bhi, const float4* blo,
+                                            const float4* si_hi, const float4* si_lo)
 {
-    const int nl = P.n_large, lg = P.lanes_log2, LS = 1 << lg;
-    if ((t & ~31) >> lg >= nl) return;   // uniform over the warp
-    const int lane = t & (LS - 1), g = t >> lg, k = min(g, nl - 1);
+    const int LS = 1 << lg;
     const float4 H = si_hi[k], L = si_lo[k];
     Ds3 a{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     for (int j0 = lane; j0 < pad; j0 += 16 << lg) {
@@ -466,7 +479,16 @@ __device__ __forceinline__ void pull_large(const TryParams& P, int s, int t, int
         for (int j = j0; j < j1; j += LS) pair_term<MODE>(bhi[j], blo[j], H, L, x, y, z);
         fold(a, x, y, z);
     }
-    const float2 part = reduce_scatter(a, lane, LS);   // x, y, z in lanes 0, 1, 2
+    return reduce_scatter(a, lane, LS);   // x, y, z in lanes 0, 1, 2
+}
+template <int MODE>
+__device__ __forceinline__ void pull_large(const TryParams& P, int s, int t, int pad, const float4* bhi,
+                                           const float4* blo, const float4* si_hi, const float4* si_lo, unsigned tag)
+{
+    const int nl = P.n_large, lg = P.lanes_log2;
+    if ((t & ~31) >> lg >= nl) return;   // uniform over the warp
+    const int lane = t & ((1 << lg) - 1), g = t >> lg, k = min(g, nl - 1);
+    const float2 part = large_sum<MODE>(lane, lg, k, pad, bhi, blo, si_hi, si_lo);
     const int l0 = (t & 31) - lane;
     const float yh = __shfl_sync(0xffffffffu, part.x, l0 + 1), yl = __shfl_sync(0xffffffffu, part.y, l0 + 1);
     const float zh = __shfl_sync(0xffffffffu, part.x, l0 + 2), zl = __shfl_sync(0xffffffffu, part.y, l0 + 2);
@@ -481,19 +503,18 @@ __device__ __forceinline__ void pull_large(const TryParams& P, int s, int t, int
 // part 0 the stars, the others (or part 0 too, if it is alone) a share of the
 // protoplanets each.
 template <int MODE>
-__device__ __forceinline__ void pull_small(const TryParams& P, int p, int b, int cnt, int pad, int np, const float4* bhi,
-                                           const float4* blo, const float4* si_hi, const float4* si_lo,
-                                           const float2* star_m, float2* parts)
+__device__ __forceinline__ void pull_small(int nl, int n_star, int step0, int p, int b, int cnt, int pad, int np,
+                                           const float4* bhi, const float4* blo, const float4* si_hi,
+                                           const float4* si_lo, const float2* star_m, float2* parts)
 {
-    const int nl = P.n_large;
     if (p >= np) return;
-    for (; b < cnt; b += np > 1 ? pad : P.pull) {
+    for (; b < cnt; b += np > 1 ? pad : step0) {
         const float4 H = bhi[b], L = blo[b];
         float2 ax = make_float2(0.f, 0.f), ay = ax, az = ax;
         if (p > 0 || np == 1) {
             const int step = np > 1 ? np - 1 : 1;
             Ds3 a{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            for (int k0 = P.n_star + (np > 1 ? p - 1 : 0); k0 < nl; k0 += 8 * step) {
+            for (int k0 = n_star + (np > 1 ? p - 1 : 0); k0 < nl; k0 += 8 * step) {
                 float x = 0.f, y = 0.f, z = 0.f;
                 const int k1 = min(nl, k0 + 8 * step);
 #pragma unroll 4
@@ -505,7 +526,7 @@ __device__ __forceinline__ void pull_small(const TryParams& P, int p, int b, int
             az = dsn_norm(a.zh, a.zl);
         }
         if (p == 0)
-            for (int k = 0; k < P.n_star; k++) star_term(si_hi[k], si_lo[k], star_m[k], H, L, ax, ay, az);
+            for (int k = 0; k < n_star; k++) star_term(si_hi[k], si_lo[k], star_m[k], H, L, ax, ay, az);
         float2* o = parts + 3 * (p * pad + b);
         o[0] = ax;
         o[1] = ay;
@@ -628,7 +649,7 @@ __global__ void __launch_bounds__(try_max_threads(DRAG)) k_try(const __grid_cons
         for (int s = 0; s < ns; s++) {
             const int q = s & 1;
             pull_large<MODE>(P, s, t, pad, bhi + q * pad, blo + q * pad, si_hi[q], si_lo[q], tag0 + 1 + s);
-            pull_small<MODE>(P, share, body, cnt, pad, np, bhi + q * pad, blo + q * pad, si_hi[q], si_lo[q], star_m,
+            pull_small<MODE>(nl, P.n_star, P.pull, share, body, cnt, pad, np, bhi + q * pad, blo + q * pad, si_hi[q], si_lo[q], star_m,
                              parts + (size_t)q * np * 3 * pad);
             if (s == 0 && P.head_n > 0) __threadfence();   // the cleared hash before the later records
             group_sync(1, main);
@@ -686,7 +707,7 @@ __global__ void __launch_bounds__(try_max_threads(DRAG)) k_try(const __grid_cons
 #pragma unroll
                 for (int c = 0; c < N; c++)
                     put_comp(bhi + q * pad, blo + q * pad, b, DRAG ? c : x % 3,
-                             position(yr[e + c], cdt, yv[e + c], dsn_mul(r[c], dt2)));
+                             position<MODE>(yr[e + c], cdt, yv[e + c], dsn_mul(r[c], dt2)));
             }
         }
         if (s == ns) break;
@@ -760,6 +781,300 @@ __global__ void __launch_bounds__(try_max_threads(DRAG)) k_try(const __grid_cons
     }
 }
 
+// ---------------------------------------------------------------------------
+// k_team
+// ---------------------------------------------------------------------------
+namespace {
+
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;\n" ::: "memory");
+}
+// Another CTA's copy of a shared-memory word.
+__device__ __forceinline__ unsigned peer(const void* local, int rank)
+{
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n"
+                 : "=r"(r)
+                 : "r"((unsigned)__cvta_generic_to_shared(local)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_peer(unsigned a, float2 v)
+{
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};\n" ::"r"(a), "f"(v.x), "f"(v.y) : "memory");
+}
+__device__ __forceinline__ void st_peer(unsigned a, float v)
+{
+    asm volatile("st.shared::cluster.f32 [%0], %1;\n" ::"r"(a), "f"(v) : "memory");
+}
+__device__ __forceinline__ void st_peer(unsigned a, unsigned long long v)
+{
+    asm volatile("st.shared::cluster.b64 [%0], %1;\n" ::"r"(a), "l"(v) : "memory");
+}
+
+struct TeamSmem {
+    float4 si_hi[3][kTeamLarge], si_lo[3][kTeamLarge];   // the large bodies, by stage mod 3
+    float2 star_m[kTryMaxStars];
+    float mass[kTeamLarge];
+    double ly[3 * kTeamLarge], lv[3 * kTeamLarge];
+    NyTableau T;
+    float2 part[2][kTeamLarge + kTeamCtas][3];   // partials of the bodies owned here, [stage parity][slot, team rank]
+    float2 k[kTeamLarge][kMaxStages][3];         // their accelerations
+    unsigned long long err, errs[kTeamCtas];     // this CTA's error; the team's, in its first CTA
+    DevSys sys;
+    int live[kTeamLarge];
+    double dt;
+    int runs;
+};
+
+}  // namespace
+
+template <int MODE>
+__global__ void __launch_bounds__(kTeamPull + kTeamBody + kTeamOwners, 1) k_team(const __grid_constant__ TeamParams P)
+{
+    __shared__ TeamSmem sm;
+    extern __shared__ __align__(16) unsigned char dyn[];
+    const int t = threadIdx.x;
+    const TeamItem it = P.items[blockIdx.x];
+    const int ns = P.n_stage;
+    pdl_wait();
+    pdl_trigger();
+    if (t == 0) {
+        int runs = 0;
+        double dt = 0.0;
+        if (it.sys >= 0) {
+            const volatile DevSys* V = P.sys + it.sys;
+            dt = V->dt_try;
+            runs = V->active && !V->halted && V->quota != 0;
+        }
+        sm.dt = dt;
+        sm.runs = runs;
+        sm.err = 0ull;
+    }
+    __syncthreads();
+    if (!sm.runs) {   // uniform over the team; the cluster's barriers still count this CTA
+        if (it.sys >= 0 && it.rank == 0 && t == 0) P.sys[it.sys].accepted = 0;
+        for (int k = 0; k < ns + 3; k++) cluster_sync();
+        return;
+    }
+    const double dt = sm.dt;
+    DevSys* S = P.sys + it.sys;
+    const SysInfo si = P.sinfo[it.sys];
+    const int nl = si.n_SI, n_star = si.n_star, small = si.n - nl;
+    const int nb = (small + it.size - 1) / it.size;
+    const int b0 = nl + it.rank * nb;
+    const int cnt = max(0, min(si.n - b0, nb));
+    const int first = si.off + b0;
+    const int pad = try_pad(nb), n3 = 3 * nb;
+    float4* bhi = reinterpret_cast<float4*>(dyn);               // [2][pad], by stage parity
+    float4* blo = bhi + 2 * pad;
+    float2* parts = reinterpret_cast<float2*>(blo + 2 * pad);   // [2][pad][3]
+    float2* ks = parts + (size_t)2 * 3 * pad;                   // [stage][nb][3]
+
+    // ---- load ----
+    for (int b = t; b < pad; b += blockDim.x) {
+        float4 H = make_float4(1.0e9f, 0.f, 0.f, 0.f), L = make_float4(0.f, 0.f, 0.f, 0.f);   // no body: no mass
+        if (b < cnt) {
+            const int i = first + b;
+            const int id = P.id[i];
+            const double m = P.mass[i];
+            split_ds(P.y_r[3 * i], H.x, L.x);
+            split_ds(P.y_r[3 * i + 1], H.y, L.y);
+            split_ds(P.y_r[3 * i + 2], H.z, L.z);
+            H.w = id >= 0 ? __double2float_rn(m) : 0.f;
+            L.w = id > 0 ? 1.f : 0.f;   // an inactive sink's gravity is zero
+        }
+        bhi[b] = H;
+        blo[b] = L;
+        bhi[pad + b] = H;
+        blo[pad + b] = L;
+    }
+    for (int k = t; k < (int)(sizeof(NyTableau) / 16); k += blockDim.x)
+        reinterpret_cast<uint4*>(&sm.T)[k] = reinterpret_cast<const uint4*>(P.tab)[k];
+    if (t < 3 * nl) {
+        sm.ly[t] = P.y_r[3 * si.off + t];
+        sm.lv[t] = P.y_v[3 * si.off + t];
+        put_comp(sm.si_hi[0], sm.si_lo[0], t / 3, t % 3, to_ds(sm.ly[t]));
+    }
+    if (t < nl) {
+        const int id = P.id[si.off + t];
+        const double m = id >= 0 ? P.mass[si.off + t] : 0.0;
+        const float mh = __double2float_rn(m);
+        sm.mass[t] = mh;
+        sm.live[t] = id > 0;
+        for (int q = 0; q < 3; q++) sm.si_hi[q][t].w = mh;
+        if (t < n_star) sm.star_m[t] = make_float2(mh, __double2float_rn(m - (double)mh));
+    }
+    if (it.rank == 0)
+        for (int k = t; k < (int)(sizeof(DevSys) / 4); k += blockDim.x)
+            reinterpret_cast<unsigned*>(&sm.sys)[k] = reinterpret_cast<const volatile unsigned*>(S)[k];
+    GridInfo grid{};
+    if (P.head) {
+        grid = P.grid[it.sys];
+        if (grid.enabled)   // this team's bodies alone go there; inserted after the barriers below
+            for (int k = it.rank * (int)blockDim.x + t; k <= grid.mask; k += it.size * (int)blockDim.x)
+                P.head[grid.toff + k] = -1;
+    }
+    const NyTableau& T = sm.T;
+    const float2 dt1 = to_ds(dt), dt2 = to_ds(dt * dt);
+    cluster_sync();
+
+    const bool puller = t < kTeamPull, owner = t >= kTeamPull + kTeamBody;
+    const int tb = t - kTeamPull;
+    const int lane = t & 31, ow = (t - kTeamPull - kTeamBody) >> 5;
+    const int comp = min(lane, 2);
+    int lg = 5;
+    while (lg > 2 && (nl << lg) > kTeamPull) lg--;
+
+    // phase s: pair terms of stage s, K of stage s - 1, positions of stage s + 1
+    for (int s = 0; s <= ns; s++) {
+        const int q = s & 1, c3 = s % 3;
+        if (puller) {
+            if (s < ns) {
+                if ((t & ~31) >> lg < nl) {   // uniform over the warp
+                    const int gl = t & ((1 << lg) - 1), g = t >> lg, k = min(g, nl - 1);
+                    const float2 v = large_sum<MODE>(gl, lg, k, pad, bhi + q * pad, blo + q * pad, sm.si_hi[c3],
+                                                     sm.si_lo[c3]);
+                    if (gl < 3 && g < nl)
+                        st_peer(peer(&sm.part[q][(k / it.size) * it.size + it.rank][gl], it.base + k % it.size), v);
+                }
+                pull_small<MODE>(nl, n_star, kTeamPull, 0, t, cnt, pad, 1, bhi + q * pad, blo + q * pad, sm.si_hi[c3],
+                                 sm.si_lo[c3], sm.star_m, parts + (size_t)q * 3 * pad);
+            }
+        } else if (!owner) {
+            for (int e = tb; e < 3 * cnt; e += kTeamBody) {
+                const int b = e / 3;
+                float2* k = ks + e;
+                if (s > 0) {
+                    float2 g = parts[(size_t)(q ^ 1) * 3 * pad + e];
+                    if (blo[b].w == 0.f) g = make_float2(0.f, 0.f);
+                    k[(size_t)(s - 1) * n3] = g;
+                }
+                if (s + 1 < ns) {
+                    float2 r[1];
+                    row_sum(T, s + 1, k, n3, r);
+                    put_comp(bhi + (q ^ 1) * pad, blo + (q ^ 1) * pad, b, e % 3,
+                             position<MODE>(P.y_r[3 * first + e], T.c[s + 1] * dt, P.y_v[3 * first + e],
+                                      dsn_mul(r[0], dt2)));
+                }
+            }
+            if (s == 0 && ns > 1 && tb < 3 * nl)
+                put_comp(sm.si_hi[1], sm.si_lo[1], tb / 3, tb % 3,
+                         to_ds(fma(T.c[1] * dt, sm.lv[tb], sm.ly[tb])));
+        } else if (s > 0) {
+            // a warp per large body owned here: slot u is body u size + rank
+            const int p3 = (s - 1) % 3;
+            for (int u = ow; u * it.size + it.rank < nl; u += kTeamOwners / 32) {
+                const int k = u * it.size + it.rank;
+                const float4 H = sm.si_hi[p3][k], L = sm.si_lo[p3][k];
+                Ds3 a{0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                if (lane >= n_star && lane < nl && lane != k) {
+                    float px = 0.f, py = 0.f, pz = 0.f;
+                    pair_term<MODE>(sm.si_hi[p3][lane], sm.si_lo[p3][lane], H, L, px, py, pz);
+                    fold(a, px, py, pz);
+                }
+                if (lane < n_star && lane != k) {
+                    float2 ax = make_float2(0.f, 0.f), ay = ax, az = ax;
+                    star_term(sm.si_hi[p3][lane], sm.si_lo[p3][lane], sm.star_m[lane], H, L, ax, ay, az);
+                    ds_merge(a.xh, a.xl, ax.x, ax.y);
+                    ds_merge(a.yh, a.yl, ay.x, ay.y);
+                    ds_merge(a.zh, a.zl, az.x, az.y);
+                }
+                if (lane < it.size) {
+                    const float2* pt = sm.part[q ^ 1][u * it.size + lane];
+                    ds_merge(a.xh, a.xl, pt[0].x, pt[0].y);
+                    ds_merge(a.yh, a.yl, pt[1].x, pt[1].y);
+                    ds_merge(a.zh, a.zl, pt[2].x, pt[2].y);
+                }
+                float2 g = reduce_scatter(a, lane, 32);
+                if (!sm.live[k]) g = make_float2(0.f, 0.f);
+                if (lane < 3) sm.k[u][s - 1][lane] = g;
+                __syncwarp();
+                if (s + 1 < ns) {
+                    float2 r[1];
+                    row_sum<1>(T, s + 1, &sm.k[u][0][comp], 3, r);
+                    const float2 x =
+                        position<MODE>(sm.ly[3 * k + comp], T.c[s + 1] * dt, sm.lv[3 * k + comp], dsn_mul(r[0], dt2));
+                    if (lane < 3) {
+                        const int n3s = (s + 1) % 3;
+                        float* h = reinterpret_cast<float*>(&sm.si_hi[n3s][k]) + lane;
+                        float* l = reinterpret_cast<float*>(&sm.si_lo[n3s][k]) + lane;
+                        for (int c = 0; c < it.size; c++) {
+                            st_peer(peer(h, it.base + c), x.x);
+                            st_peer(peer(l, it.base + c), x.y);
+                        }
+                    }
+                }
+            }
+        }
+        if (s < ns) cluster_sync();
+    }
+
+    // ---- the error of the team, in its first CTA ----
+    const int own_n = it.rank < nl ? (nl - it.rank + it.size - 1) / it.size : 0;
+    if (P.adaptive && !puller) {
+        unsigned long long eb = 0ull;
+        if (!owner) {
+            for (int e = tb; e < 3 * cnt; e += kTeamBody)
+                eb = max(eb, component_error<1>(T, P.scheme, dt1, ks + e, n3));
+        } else if (lane < 3) {
+            for (int u = ow; u < own_n; u += kTeamOwners / 32)
+                eb = max(eb, component_error<1>(T, P.scheme, dt1, &sm.k[u][0][lane], 3));
+        }
+        for (int m = 16; m > 0; m >>= 1) eb = max(eb, __shfl_xor_sync(0xffffffffu, eb, m));
+        if (lane == 0) atomicMax(&sm.err, eb);
+    }
+    __syncthreads();
+    if (t == 0) st_peer(peer(&sm.errs[it.rank], it.base), sm.err);
+    cluster_sync();
+    unsigned long long err = 0ull;
+    for (int c = 0; c < it.size; c++) {
+        unsigned long long e;
+        asm volatile("ld.shared::cluster.b64 %0, [%1];\n" : "=l"(e) : "r"(peer(&sm.errs[c], it.base)) : "memory");
+        err = max(err, e);
+    }
+    // control_system's test, the same in every CTA of the team
+    const double max_err = fabs(P.ctl.lambda * dt * __longlong_as_double((long long)err));
+    const bool accepted = !P.adaptive || max_err <= P.ctl.tolerance;
+    cluster_sync();   // the errors are read: CTAs may leave from here on
+    if (it.rank == 0 && t == kTeamPull - 1) {
+        control_of(P.ctl, sm.sys, P.adaptive ? err : 0ull);
+        store_control(S, sm.sys);
+    }
+    if (!accepted) return;
+    bool bad = false;
+    if (!puller && !owner) {
+        for (int e = tb; e < 3 * cnt; e += kTeamBody) {
+            double y[1] = {P.y_r[3 * first + e]}, v[1] = {P.y_v[3 * first + e]};
+            solution<1>(T, dt, dt1, dt2, ks + e, n3, y, v);
+            P.y_r[3 * first + e] = y[0];
+            P.y_v[3 * first + e] = v[0];
+            bad = bad || not_finite(y[0]) || not_finite(v[0]);
+            write_pos_c(P.pos_hi, P.pos_lo, first + e / 3, e % 3, y[0]);
+            if (grid.enabled) reinterpret_cast<int*>(bhi)[e] = cell_coord(y[0], grid.inv_h);
+        }
+    } else if (owner && lane < 3) {
+        for (int u = ow; u < own_n; u += kTeamOwners / 32) {
+            const int k = u * it.size + it.rank, x = 3 * (si.off + k) + lane;
+            double y[1] = {sm.ly[3 * k + lane]}, v[1] = {sm.lv[3 * k + lane]};
+            solution<1>(T, dt, dt1, dt2, &sm.k[u][0][lane], 3, y, v);
+            P.y_r[x] = y[0];
+            P.y_v[x] = v[0];
+            bad = bad || not_finite(y[0]) || not_finite(v[0]);
+            write_pos_c(P.pos_hi, P.pos_lo, si.off + k, lane, y[0]);
+        }
+    }
+    if (bad) S->status = 5;   // RED_ERR_NONFINITE
+    if (!grid.enabled) return;   // uniform
+    __syncthreads();
+    const int* cell = reinterpret_cast<const int*>(bhi);
+    for (int b = t; b < cnt; b += blockDim.x) {
+        const int4 cl = make_int4(cell[3 * b], cell[3 * b + 1], cell[3 * b + 2], 0);
+        P.cell[first + b] = cl;
+        P.next[first + b] = atomicExch(&P.head[grid.toff + bucket_of(cl.x, cl.y, cl.z, grid.mask)], first + b);
+    }
+}
+
 namespace {
 typedef void (*TryKernel)(const TryParams);
 TryKernel try_kernel(int mode, bool drag)
@@ -802,6 +1117,52 @@ void launch_try(const TryParams& P, int mode, cudaStream_t s)
     cfg.attrs = at;
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, try_kernel(mode, drag), P);
+}
+
+namespace {
+typedef void (*TeamKernel)(const TeamParams);
+TeamKernel team_kernel(int mode)
+{
+    return mode == MODE_MIXED ? k_team<MODE_MIXED> : mode == MODE_FP32 ? k_team<MODE_FP32> : nullptr;
+}
+}  // namespace
+
+int team_clusters(int mode, size_t smem)
+{
+    TeamKernel k = team_kernel(mode);
+    int dev = 0, most = 0, n = 0;
+    if (!k || cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+        return 0;
+    cudaFuncAttributes a;
+    if (cudaFuncGetAttributes(&a, k) != cudaSuccess || smem + a.sharedSizeBytes > (size_t)most ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes) !=
+            cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kTeamCtas);
+    cfg.blockDim = dim3(kTeamPull + kTeamBody + kTeamOwners);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kTeamCtas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+
+void launch_team(const TeamParams& P, int n_ctas, int mode, cudaStream_t s)
+{
+    launch_kx(team_kernel(mode), (unsigned)n_ctas, (unsigned)(kTeamPull + kTeamBody + kTeamOwners),
+              (unsigned)kTeamCtas, team_smem(P.cap, P.n_stage), s, P);
 }
 
 void set_tableau_try(const Tableau& tb, cudaStream_t s)

@@ -121,6 +121,54 @@ __host__ __device__ constexpr size_t try_smem(int nb, int n_stage, int pull)
 // Threads of a CTA at most.
 __host__ __device__ constexpr int try_max_threads(bool drag) { return drag ? 1024 : 928; }
 
+// ---------------------------------------------------------------------------
+// k_team: the same for an ensemble of sparse systems.  A system's small bodies
+// are shared by a team of up to kTeamCtas CTAs of one thread-block cluster, the
+// teams of a cluster side by side; the exchange goes through the CTAs' shared
+// memory, ordered by one cluster barrier per phase (the cluster's CTAs run the
+// same phases).  A large body's sum and its next position are formed by a warp
+// of the team in the phase after the partials, as long as that phase lasts.
+// ---------------------------------------------------------------------------
+constexpr int kTeamCtas = 8;
+constexpr int kTeamLarge = 16;         // large bodies of a system on this path
+constexpr int kTeamBodies = 512;       // small bodies of a CTA at most
+constexpr int kTeamPull = 512, kTeamBody = 256, kTeamOwners = 256;   // threads of the groups
+
+struct TeamItem {
+    int sys;                 // -1: an idle CTA
+    int rank, size;          // of the CTA in its team
+    int base;                // cluster rank of the team's first CTA
+};
+
+struct TeamParams {
+    int scheme, n_stage, adaptive;
+    int cap;                 // small bodies a CTA's shared memory is laid out for
+    const TeamItem* items;
+    const SysInfo* sinfo;
+    DevSys* sys;
+    double* y_r;
+    double* y_v;
+    const double* mass;
+    const int* id;
+    float4* pos_hi;
+    float4* pos_lo;
+    const NyTableau* tab;
+    ControlParams ctl;
+    int* head;               // the collision check's hash (null: none)
+    int* next;
+    int4* cell;
+    const GridInfo* grid;
+};
+
+__host__ __device__ constexpr size_t team_smem(int cap, int n_stage)
+{
+    return (size_t)try_pad(cap) * 2 * (2 * sizeof(float4) + 3 * sizeof(float2)) +
+           (size_t)cap * 3 * sizeof(float2) * n_stage;
+}
+// Clusters resident at once (0: none, or the query failed), and the launch.
+int team_clusters(int mode, size_t smem);
+void launch_team(const TeamParams& P, int n_ctas, int mode, cudaStream_t s);
+
 // CTAs of the cooperative launch that are resident at once per SM with this much
 // shared memory (0: none, or the query failed), and the launch.
 int try_ctas_per_sm(int mode, bool drag, int threads, size_t smem);
