@@ -1182,7 +1182,7 @@ void red_sim::plan_team()
         }
         for (int r = 0; r < size; r++) teams[c * kTeamCtas + used[c] + r] = TeamItem{s, r, size, used[c]};
         used[c] += size;
-        team_cap = std::max(team_cap, (sinfo[s].n - sinfo[s].n_SI + size - 1) / size);
+        team_cap = std::max(team_cap, team_bodies(sinfo[s].n - sinfo[s].n_SI, size));
     }
     if (teams.size() > teams_cap) {
         cudaFree(d_teams);

@@ -167,6 +167,60 @@ __device__ __forceinline__ float2 to_ds(double x)
     return a;
 }
 
+// Two double-single numbers side by side, in packed FP32 (one instruction for both).
+struct D2 {
+    float2 h, l;
+};
+__device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, dup2(-1.f), a); }   // a - b, rounded once
+__device__ __forceinline__ D2 fast2(float2 a, float2 b)   // |a| >= |b|
+{
+    const float2 s = __fadd2_rn(a, b);
+    return D2{s, sub2(b, sub2(s, a))};
+}
+__device__ __forceinline__ void two_sum2(float2 a, float2 b, float2& s, float2& e)
+{
+    s = __fadd2_rn(a, b);
+    const float2 bp = sub2(s, a);
+    e = __fadd2_rn(sub2(a, sub2(s, bp)), sub2(b, bp));
+}
+__device__ __forceinline__ D2 add2(D2 a, D2 b)
+{
+    float2 s, e;
+    two_sum2(a.h, b.h, s, e);
+    return fast2(s, __fadd2_rn(e, __fadd2_rn(a.l, b.l)));
+}
+__device__ __forceinline__ D2 sub2(D2 a, D2 b)
+{
+    return add2(a, D2{__fmul2_rn(b.h, dup2(-1.f)), __fmul2_rn(b.l, dup2(-1.f))});
+}
+__device__ __forceinline__ D2 mul2(D2 a, float2 b)   // both by the double-single number b
+{
+    const float2 p = __fmul2_rn(a.h, dup2(b.x));
+    const float2 r = __ffma2_rn(a.h, dup2(b.x), __fmul2_rn(p, dup2(-1.f)));
+    return fast2(p, __ffma2_rn(a.h, dup2(b.y), __ffma2_rn(a.l, dup2(b.x), r)));
+}
+// sum a_q K_q over a row of the tableau, K_q at k[q st] as (h0, h1, l0, l1)
+__device__ __forceinline__ D2 row_sum2(const NyTableau& T, int row, const float4* k, int st)
+{
+    float2 h = make_float2(0.f, 0.f), l = h;
+    const int u1 = T.beg[row + 1];
+#pragma unroll 2
+    for (int u = T.beg[row]; u < u1; u++) {
+        const float4 m = *reinterpret_cast<const float4*>(&T.term[u]);
+        const float4 x = k[__float_as_int(m.z) * st];
+        const float2 xh = make_float2(x.x, x.y), xl = make_float2(x.z, x.w);
+        const float2 p = __fmul2_rn(xh, dup2(m.x));
+        const float2 r = __ffma2_rn(xh, dup2(m.x), __fmul2_rn(p, dup2(-1.f)));
+        const float2 e = __ffma2_rn(xh, dup2(m.y), __ffma2_rn(xl, dup2(m.x), r));
+        float2 sum, t;
+        two_sum2(h, p, sum, t);
+        h = sum;
+        l = __fadd2_rn(l, __fadd2_rn(t, e));
+    }
+    return fast2(h, l);   // |l| is far below |h| unless both vanish
+}
+
 // The larger of a component's position and velocity errors, as bits (NaN above all).
 template <int N>
 __device__ __forceinline__ unsigned long long component_error(const NyTableau& T, int scheme, float2 dt,
@@ -181,6 +235,28 @@ __device__ __forceinline__ unsigned long long component_error(const NyTableau& T
                              ? dsn_sub(dsn_sub(dsn_add(k[c], k[10 * st + c]), k[11 * st + c]), k[12 * st + c])
                              : dsn_sub(k[3 * st + c], k[4 * st + c]);
         const double er = fabs(dsn_to_double(dsn_mul(r[c], dt))), ev = fabs(dsn_to_double(d));
+        double e = fmax(er, ev);
+        if (er != er || ev != ev) e = __longlong_as_double(0x7ff8000000000000ll);
+        m = max(m, (unsigned long long)__double_as_longlong(e));
+    }
+    return m;
+}
+__device__ __forceinline__ unsigned long long pair_error(const NyTableau& T, int scheme, float2 dt, const float4* k,
+                                                         int st, bool both)
+{
+    auto at = [&](int q) {
+        const float4 x = k[q * st];
+        return D2{make_float2(x.x, x.y), make_float2(x.z, x.w)};
+    };
+    const D2 r = mul2(row_sum2(T, kTryRowER, k, st), dt);
+    const D2 d = scheme == SCHEME_RKF78 ? sub2(sub2(add2(at(0), at(10)), at(11)), at(12)) : sub2(at(3), at(4));
+    const float2 rr[2] = {make_float2(r.h.x, r.l.x), make_float2(r.h.y, r.l.y)};
+    const float2 dd[2] = {make_float2(d.h.x, d.l.x), make_float2(d.h.y, d.l.y)};
+    unsigned long long m = 0ull;
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+        if (c == 1 && !both) break;
+        const double er = fabs(dsn_to_double(rr[c])), ev = fabs(dsn_to_double(dd[c]));
         double e = fmax(er, ev);
         if (er != er || ev != ev) e = __longlong_as_double(0x7ff8000000000000ll);
         m = max(m, (unsigned long long)__double_as_longlong(e));
@@ -818,7 +894,7 @@ struct TeamSmem {
     float mass[kTeamLarge];
     double ly[3 * kTeamLarge], lv[3 * kTeamLarge];
     NyTableau T;
-    float2 part[2][kTeamLarge + kTeamCtas][3];   // partials of the bodies owned here, [stage parity][slot, team rank]
+    float2 part[2][2 * (kTeamLarge + kTeamCtas)][3];   // partials of the bodies owned here: stage parity; slot, rank, half
     float2 k[kTeamLarge][kMaxStages][3];         // their accelerations
     unsigned long long err, errs[kTeamCtas];     // this CTA's error; the team's, in its first CTA
     DevSys sys;
@@ -861,15 +937,15 @@ __global__ void __launch_bounds__(kTeamPull + kTeamBody + kTeamOwners, 1) k_team
     DevSys* S = P.sys + it.sys;
     const SysInfo si = P.sinfo[it.sys];
     const int nl = si.n_SI, n_star = si.n_star, small = si.n - nl;
-    const int nb = (small + it.size - 1) / it.size;
+    const int nb = team_bodies(small, it.size);
     const int b0 = nl + it.rank * nb;
     const int cnt = max(0, min(si.n - b0, nb));
     const int first = si.off + b0;
-    const int pad = try_pad(nb), n3 = 3 * nb;
+    const int pad = try_pad(nb), np = 3 * nb / 2;   // components in pairs: nb is even
     float4* bhi = reinterpret_cast<float4*>(dyn);               // [2][pad], by stage parity
     float4* blo = bhi + 2 * pad;
     float2* parts = reinterpret_cast<float2*>(blo + 2 * pad);   // [2][pad][3]
-    float2* ks = parts + (size_t)2 * 3 * pad;                   // [stage][nb][3]
+    float4* ks = reinterpret_cast<float4*>(parts + (size_t)2 * 3 * pad);   // [stage][pair]: (h0, h1, l0, l1)
 
     // ---- load ----
     for (int b = t; b < pad; b += blockDim.x) {
@@ -923,42 +999,56 @@ __global__ void __launch_bounds__(kTeamPull + kTeamBody + kTeamOwners, 1) k_team
     const int tb = t - kTeamPull;
     const int lane = t & 31, ow = (t - kTeamPull - kTeamBody) >> 5;
     const int comp = min(lane, 2);
-    int lg = 5;
-    while (lg > 2 && (nl << lg) > kTeamPull) lg--;
+    const int mid = pad / 64 * 32;   // large_sum's halves
 
+    // pairs of components of the body group; the error and the solution follow the same split
+    const int pairs = (3 * cnt + 1) / 2;
+    const int share = min(pairs, kTeamRounds * kTeamBody);
+    const int x0 = puller ? share + t : tb, x1 = puller ? pairs : share, xs = puller ? kTeamPull : kTeamBody;
     // phase s: pair terms of stage s, K of stage s - 1, positions of stage s + 1
     for (int s = 0; s <= ns; s++) {
         const int q = s & 1, c3 = s % 3;
-        if (puller) {
-            if (s < ns) {
-                if ((t & ~31) >> lg < nl) {   // uniform over the warp
-                    const int gl = t & ((1 << lg) - 1), g = t >> lg, k = min(g, nl - 1);
-                    const float2 v = large_sum<MODE>(gl, lg, k, pad, bhi + q * pad, blo + q * pad, sm.si_hi[c3],
-                                                     sm.si_lo[c3]);
-                    if (gl < 3 && g < nl)
-                        st_peer(peer(&sm.part[q][(k / it.size) * it.size + it.rank][gl], it.base + k % it.size), v);
-                }
-                pull_small<MODE>(nl, n_star, kTeamPull, 0, t, cnt, pad, 1, bhi + q * pad, blo + q * pad, sm.si_hi[c3],
-                                 sm.si_lo[c3], sm.star_m, parts + (size_t)q * 3 * pad);
+        if (s < ns && !owner) {
+            // a warp per large body and half of the small ones
+            for (int g = t >> 5; g < 2 * nl; g += (kTeamPull + kTeamBody) / 32) {
+                const int k = g >> 1, half = g & 1, j0 = half ? mid : 0, j1 = half ? pad : mid;
+                const float2 v = large_sum<MODE>(lane, 5, k, j1 - j0, bhi + q * pad + j0, blo + q * pad + j0,
+                                                 sm.si_hi[c3], sm.si_lo[c3]);
+                if (lane < 3)
+                    st_peer(peer(&sm.part[q][((k / it.size) * it.size + it.rank) * 2 + half][lane],
+                                 it.base + k % it.size), v);
             }
-        } else if (!owner) {
-            for (int e = tb; e < 3 * cnt; e += kTeamBody) {
-                const int b = e / 3;
-                float2* k = ks + e;
+        }
+        if (s < ns && puller)
+            pull_small<MODE>(nl, n_star, kTeamPull, 0, t, cnt, pad, 1, bhi + q * pad, blo + q * pad, sm.si_hi[c3],
+                             sm.si_lo[c3], sm.star_m, parts + (size_t)q * 3 * pad);
+        if (!owner) {
+            // the body group's pairs first, the pull group takes the rest when it is done
+            for (int x = x0; x < x1; x += xs) {
+                const int e = 2 * x, b = e / 3, c = e - 3 * b;   // component c of body b, and the next one
+                const int b2 = c == 2 ? b + 1 : b, d = c == 2 ? 0 : c + 1;
+                const bool both = e + 1 < 3 * cnt;
+                float4* k = ks + x;
                 if (s > 0) {
-                    float2 g = parts[(size_t)(q ^ 1) * 3 * pad + e];
-                    if (blo[b].w == 0.f) g = make_float2(0.f, 0.f);
-                    k[(size_t)(s - 1) * n3] = g;
+                    const float4 g = *reinterpret_cast<const float4*>(parts + (size_t)(q ^ 1) * 3 * pad + e);
+                    const float m0 = blo[b].w, m1 = blo[b2].w;   // 1, or 0 for an inactive body
+                    k[(size_t)(s - 1) * np] = make_float4(m0 != 0.f ? g.x : 0.f, m1 != 0.f ? g.z : 0.f,
+                                                          m0 != 0.f ? g.y : 0.f, m1 != 0.f ? g.w : 0.f);
                 }
                 if (s + 1 < ns) {
-                    float2 r[1];
-                    row_sum(T, s + 1, k, n3, r);
-                    put_comp(bhi + (q ^ 1) * pad, blo + (q ^ 1) * pad, b, e % 3,
-                             position<MODE>(P.y_r[3 * first + e], T.c[s + 1] * dt, P.y_v[3 * first + e],
-                                      dsn_mul(r[0], dt2)));
+                    const double cdt = T.c[s + 1] * dt;
+                    const size_t i = 3 * (size_t)first + e, j = both ? i + 1 : i;
+                    const float2 u = to_ds(fma(cdt, P.y_v[i], P.y_r[i])), w = to_ds(fma(cdt, P.y_v[j], P.y_r[j]));
+                    const D2 r = add2(D2{make_float2(u.x, w.x), make_float2(u.y, w.y)},
+                                      mul2(row_sum2(T, s + 1, k, np), dt2));
+                    put_comp(bhi + (q ^ 1) * pad, blo + (q ^ 1) * pad, b, c,
+                             coordinate<MODE>(make_float2(r.h.x, r.l.x)));
+                    if (both)
+                        put_comp(bhi + (q ^ 1) * pad, blo + (q ^ 1) * pad, b2, d,
+                                 coordinate<MODE>(make_float2(r.h.y, r.l.y)));
                 }
             }
-            if (s == 0 && ns > 1 && tb < 3 * nl)
+            if (s == 0 && ns > 1 && tb >= 0 && tb < 3 * nl)
                 put_comp(sm.si_hi[1], sm.si_lo[1], tb / 3, tb % 3,
                          to_ds(fma(T.c[1] * dt, sm.lv[tb], sm.ly[tb])));
         } else if (s > 0) {
@@ -980,8 +1070,8 @@ __global__ void __launch_bounds__(kTeamPull + kTeamBody + kTeamOwners, 1) k_team
                     ds_merge(a.yh, a.yl, ay.x, ay.y);
                     ds_merge(a.zh, a.zl, az.x, az.y);
                 }
-                if (lane < it.size) {
-                    const float2* pt = sm.part[q ^ 1][u * it.size + lane];
+                if (lane < 2 * it.size) {
+                    const float2* pt = sm.part[q ^ 1][2 * u * it.size + lane];
                     ds_merge(a.xh, a.xl, pt[0].x, pt[0].y);
                     ds_merge(a.yh, a.yl, pt[1].x, pt[1].y);
                     ds_merge(a.zh, a.zl, pt[2].x, pt[2].y);
@@ -1012,11 +1102,11 @@ __global__ void __launch_bounds__(kTeamPull + kTeamBody + kTeamOwners, 1) k_team
 
     // ---- the error of the team, in its first CTA ----
     const int own_n = it.rank < nl ? (nl - it.rank + it.size - 1) / it.size : 0;
-    if (P.adaptive && !puller) {
+    if (P.adaptive) {
         unsigned long long eb = 0ull;
         if (!owner) {
-            for (int e = tb; e < 3 * cnt; e += kTeamBody)
-                eb = max(eb, component_error<1>(T, P.scheme, dt1, ks + e, n3));
+            for (int x = x0; x < x1; x += xs)
+                eb = max(eb, pair_error(T, P.scheme, dt1, ks + x, np, 2 * x + 1 < 3 * cnt));
         } else if (lane < 3) {
             for (int u = ow; u < own_n; u += kTeamOwners / 32)
                 eb = max(eb, component_error<1>(T, P.scheme, dt1, &sm.k[u][0][lane], 3));
@@ -1043,17 +1133,27 @@ __global__ void __launch_bounds__(kTeamPull + kTeamBody + kTeamOwners, 1) k_team
     }
     if (!accepted) return;
     bool bad = false;
-    if (!puller && !owner) {
-        for (int e = tb; e < 3 * cnt; e += kTeamBody) {
-            double y[1] = {P.y_r[3 * first + e]}, v[1] = {P.y_v[3 * first + e]};
-            solution<1>(T, dt, dt1, dt2, ks + e, n3, y, v);
-            P.y_r[3 * first + e] = y[0];
-            P.y_v[3 * first + e] = v[0];
-            bad = bad || not_finite(y[0]) || not_finite(v[0]);
-            write_pos_c(P.pos_hi, P.pos_lo, first + e / 3, e % 3, y[0]);
-            if (grid.enabled) reinterpret_cast<int*>(bhi)[e] = cell_coord(y[0], grid.inv_h);
+    if (!owner) {
+        const double cdt = T.cb * dt;
+        for (int x = x0; x < x1; x += xs) {
+            const D2 r = mul2(row_sum2(T, kTryRowRB, ks + x, np), dt2), w = mul2(row_sum2(T, kTryRowVB, ks + x, np), dt1);
+            const float2 rr[2] = {make_float2(r.h.x, r.l.x), make_float2(r.h.y, r.l.y)};
+            const float2 ww[2] = {make_float2(w.h.x, w.l.x), make_float2(w.h.y, w.l.y)};
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int e = 2 * x + h;
+                if (e >= 3 * cnt) break;
+                const double v0 = P.y_v[3 * first + e];
+                const double y = fma(cdt, v0, P.y_r[3 * first + e]) + dsn_to_double(rr[h]);
+                const double v = v0 + dsn_to_double(ww[h]);
+                P.y_r[3 * first + e] = y;
+                P.y_v[3 * first + e] = v;
+                bad = bad || not_finite(y) || not_finite(v);
+                write_pos_c(P.pos_hi, P.pos_lo, first + e / 3, e % 3, y);
+                if (grid.enabled) reinterpret_cast<int*>(bhi)[e] = cell_coord(y, grid.inv_h);
+            }
         }
-    } else if (owner && lane < 3) {
+    } else if (lane < 3) {
         for (int u = ow; u < own_n; u += kTeamOwners / 32) {
             const int k = u * it.size + it.rank, x = 3 * (si.off + k) + lane;
             double y[1] = {sm.ly[3 * k + lane]}, v[1] = {sm.lv[3 * k + lane]};

@@ -133,6 +133,8 @@ constexpr int kTeamCtas = 8;
 constexpr int kTeamLarge = 16;         // large bodies of a system on this path
 constexpr int kTeamBodies = 512;       // small bodies of a CTA at most
 constexpr int kTeamPull = 512, kTeamBody = 256, kTeamOwners = 256;   // threads of the groups
+constexpr int kTeamRounds = 2;         // pairs of components of a body-group thread before the pull group takes its share
+__host__ __device__ constexpr int team_bodies(int small, int size) { return ((small + size - 1) / size + 1) / 2 * 2; }   // per CTA: even
 
 struct TeamItem {
     int sys;                 // -1: an idle CTA
