@@ -578,7 +578,7 @@ struct red_sim {
     unsigned* d_epoch = nullptr;
     NyTableau* d_ny = nullptr;
     bool use_team = false;      // the same for an ensemble of sparse systems (k_team)
-    int team_cap = 0, n_team_ctas = 0;
+    int team_cluster = 0, team_cap = 0, n_team_ctas = 0;
     TeamItem* d_teams = nullptr;
     size_t teams_cap = 0;
     bool tries_whole() const { return (use_try || use_team) && !prop_on && !log_on; }   // the proposer reads Kv[0]
@@ -1141,49 +1141,62 @@ void red_sim::plan_team()
     if (!allow_try || n_sys < 2 || (mode != MODE_MIXED && mode != MODE_FP32) || cfg.gas_disk ||
         (env && env[0] == '0'))
         return;
+    int most = 1;   // CTAs of the largest team
     for (const SysInfo& si : sinfo) {
         const int small = si.n - si.n_SI;
         if (si.n_SI < 1 || si.n_SI > kTeamLarge || si.n_star > kTryMaxStars || small < 1 || si.n != si.n_massive ||
-            small > kTeamCtas * kTeamBodies)
+            small > kTeamSize * kTeamBodies)
             return;
+        most = std::max(most, (small + kTeamBodies - 1) / kTeamBodies);
     }
-    const int resident = kTeamCtas * team_clusters(mode, team_smem(kTeamBodies, n_stage));
-    if (resident < kTeamCtas) return;
-    auto size_of = [](const SysInfo& si, int nb) { return std::min(kTeamCtas, (si.n - si.n_SI + nb - 1) / nb); };
-    int nb = kTeamBodies;
-    for (int b : {128, 192, 256, 384}) {
-        long long ctas = 0;
-        for (const SysInfo& si : sinfo) ctas += size_of(si, b);
-        if (ctas <= resident) {
-            nb = b;
-            break;
-        }
+    int sms[kTeamCtas + 1] = {0}, best = 0;
+    for (int c = most; c <= kTeamCtas; c++) {
+        sms[c] = c * team_clusters(mode, c, team_smem(kTeamBodies, n_stage));
+        if (sms[c] > sms[best]) best = c;
     }
-    std::vector<int> order(n_sys);
-    for (uint32_t s = 0; s < n_sys; s++) order[s] = (int)s;
-    auto size_at = [&](int s) { return std::max(size_of(sinfo[s], nb), size_of(sinfo[s], kTeamBodies)); };
-    std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
-        const int sa = size_at(a), sb = size_at(b);
-        if (sa != sb) return sa > sb;
-        return sinfo[a].n > sinfo[b].n;
-    });
+    if (best == 0) return;
+    // all teams resident at once with 128 bodies or more per CTA, in the clusters that
+    // take the largest teams; else full CTAs, in the clusters that leave the fewest
+    // SMs idle (GB300: 1 and 2 none, 4 eight of 152, 8 32, 9 17, 10 22)
+    const int wide = sms[kTeamSize + 1] > sms[kTeamSize] ? kTeamSize + 1 : kTeamSize;
     std::vector<TeamItem> teams;
-    std::vector<int> used;           // CTAs taken per cluster
-    std::vector<size_t> open(kTeamCtas + 1, 0);   // first cluster that may have room for a team of this size
-    team_cap = 0;
-    for (int s : order) {
-        const int size = size_at(s);
-        size_t c = open[size];
-        while (c < used.size() && used[c] + size > kTeamCtas) c++;
-        open[size] = c;
-        if (c == used.size()) {
-            used.push_back(0);
-            teams.resize(teams.size() + kTeamCtas, TeamItem{-1, 0, 1, 0});
+    auto pack = [&](int nb, int cluster) {   // largest teams first; returns the clusters
+        auto size_of = [&](int s) {
+            const int small = sinfo[s].n - sinfo[s].n_SI;
+            return std::max(std::min(kTeamSize, (small + nb - 1) / nb), (small + kTeamBodies - 1) / kTeamBodies);
+        };
+        std::vector<int> order(n_sys);
+        for (uint32_t s = 0; s < n_sys; s++) order[s] = (int)s;
+        std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+            const int sa = size_of(a), sb = size_of(b);
+            return sa != sb ? sa > sb : sinfo[a].n > sinfo[b].n;
+        });
+        teams.clear();
+        std::vector<int> used;                               // CTAs taken per cluster
+        std::vector<size_t> open(std::max(cluster, kTeamSize) + 1, 0);   // first cluster with room for a size
+        team_cluster = cluster;
+        team_cap = 0;
+        for (int s : order) {
+            const int size = size_of(s);
+            size_t c = open[size];
+            while (c < used.size() && used[c] + size > cluster) c++;
+            open[size] = c;
+            if (c == used.size()) {
+                used.push_back(0);
+                teams.resize(teams.size() + cluster, TeamItem{-1, 0, 1, 0});
+            }
+            for (int r = 0; r < size; r++) teams[c * cluster + used[c] + r] = TeamItem{s, r, size, used[c]};
+            used[c] += size;
+            team_cap = std::max(team_cap, team_bodies(sinfo[s].n - sinfo[s].n_SI, size));
         }
-        for (int r = 0; r < size; r++) teams[c * kTeamCtas + used[c] + r] = TeamItem{s, r, size, used[c]};
-        used[c] += size;
-        team_cap = std::max(team_cap, team_bodies(sinfo[s].n - sinfo[s].n_SI, size));
+        return (int)used.size();
+    };
+    bool fits = false;
+    for (int b : {128, 192, 256, 384}) {
+        fits = sms[wide] > 0 && pack(b, wide) <= sms[wide] / wide;
+        if (fits) break;
     }
+    if (!fits) pack(kTeamBodies, best);
     if (teams.size() > teams_cap) {
         cudaFree(d_teams);
         d_teams = nullptr;
@@ -1203,6 +1216,7 @@ void red_sim::launch_teams(bool hash)
     T.scheme = scheme;
     T.n_stage = n_stage;
     T.adaptive = cfg.adaptive;
+    T.cluster = team_cluster;
     T.cap = team_cap;
     T.items = d_teams;
     T.sinfo = d_sinfo;

@@ -862,9 +862,12 @@ __global__ void __launch_bounds__(try_max_threads(DRAG)) k_try(const __grid_cons
 // ---------------------------------------------------------------------------
 namespace {
 
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;\n" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync()
 {
-    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;\n" ::: "memory");
+    cluster_arrive();
+    cluster_wait();
 }
 // Another CTA's copy of a shared-memory word.
 __device__ __forceinline__ unsigned peer(const void* local, int rank)
@@ -894,9 +897,9 @@ struct TeamSmem {
     float mass[kTeamLarge];
     double ly[3 * kTeamLarge], lv[3 * kTeamLarge];
     NyTableau T;
-    float2 part[2][2 * (kTeamLarge + kTeamCtas)][3];   // partials of the bodies owned here: stage parity; slot, rank, half
+    float2 part[2][2 * (kTeamLarge + kTeamSize)][3];   // partials of the bodies owned here: stage parity; slot, rank, half
     float2 k[kTeamLarge][kMaxStages][3];         // their accelerations
-    unsigned long long err, errs[kTeamCtas];     // this CTA's error; the team's, in its first CTA
+    unsigned long long err, all, errs[kTeamSize];     // this CTA's error; the team's; its CTAs', in the first of them
     DevSys sys;
     int live[kTeamLarge];
     double dt;
@@ -1116,17 +1119,35 @@ __global__ void __launch_bounds__(kTeamPull + kTeamBody + kTeamOwners, 1) k_team
     }
     __syncthreads();
     if (t == 0) st_peer(peer(&sm.errs[it.rank], it.base), sm.err);
-    cluster_sync();
-    unsigned long long err = 0ull;
-    for (int c = 0; c < it.size; c++) {
-        unsigned long long e;
-        asm volatile("ld.shared::cluster.b64 %0, [%1];\n" : "=l"(e) : "r"(peer(&sm.errs[c], it.base)) : "memory");
-        err = max(err, e);
+    cluster_arrive();
+    // the solution meanwhile, a pair's positions and velocities, where the stage positions were
+    double* sol = reinterpret_cast<double*>(dyn);   // [4][np]
+    if (!owner) {
+        const double cdt = T.cb * dt;
+        for (int x = x0; x < x1; x += xs) {
+            const D2 r = mul2(row_sum2(T, kTryRowRB, ks + x, np), dt2), w = mul2(row_sum2(T, kTryRowVB, ks + x, np), dt1);
+            const size_t i = 3 * (size_t)first + 2 * x, j = 2 * x + 1 < 3 * cnt ? i + 1 : i;
+            const double v0 = P.y_v[i], v1 = P.y_v[j];
+            double* o = sol + x;
+            o[0] = fma(cdt, v0, P.y_r[i]) + dsn_to_double(make_float2(r.h.x, r.l.x));
+            o[np] = fma(cdt, v1, P.y_r[j]) + dsn_to_double(make_float2(r.h.y, r.l.y));
+            o[2 * np] = v0 + dsn_to_double(make_float2(w.h.x, w.l.x));
+            o[3 * np] = v1 + dsn_to_double(make_float2(w.h.y, w.l.y));
+        }
     }
+    cluster_wait();
+    if (t < 32) {
+        unsigned long long e = 0ull;
+        if (t < it.size)
+            asm volatile("ld.shared::cluster.b64 %0, [%1];\n" : "=l"(e) : "r"(peer(&sm.errs[t], it.base)) : "memory");
+        for (int m = kTeamSize / 2; m > 0; m >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, m));
+        if (t == 0) sm.all = e;
+    }
+    cluster_sync();   // the errors are read: CTAs may leave from here on
     // control_system's test, the same in every CTA of the team
+    const unsigned long long err = sm.all;
     const double max_err = fabs(P.ctl.lambda * dt * __longlong_as_double((long long)err));
     const bool accepted = !P.adaptive || max_err <= P.ctl.tolerance;
-    cluster_sync();   // the errors are read: CTAs may leave from here on
     if (it.rank == 0 && t == kTeamPull - 1) {
         control_of(P.ctl, sm.sys, P.adaptive ? err : 0ull);
         store_control(S, sm.sys);
@@ -1134,23 +1155,17 @@ __global__ void __launch_bounds__(kTeamPull + kTeamBody + kTeamOwners, 1) k_team
     if (!accepted) return;
     bool bad = false;
     if (!owner) {
-        const double cdt = T.cb * dt;
         for (int x = x0; x < x1; x += xs) {
-            const D2 r = mul2(row_sum2(T, kTryRowRB, ks + x, np), dt2), w = mul2(row_sum2(T, kTryRowVB, ks + x, np), dt1);
-            const float2 rr[2] = {make_float2(r.h.x, r.l.x), make_float2(r.h.y, r.l.y)};
-            const float2 ww[2] = {make_float2(w.h.x, w.l.x), make_float2(w.h.y, w.l.y)};
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 const int e = 2 * x + h;
                 if (e >= 3 * cnt) break;
-                const double v0 = P.y_v[3 * first + e];
-                const double y = fma(cdt, v0, P.y_r[3 * first + e]) + dsn_to_double(rr[h]);
-                const double v = v0 + dsn_to_double(ww[h]);
+                const double y = sol[h * np + x], v = sol[(2 + h) * np + x];
                 P.y_r[3 * first + e] = y;
                 P.y_v[3 * first + e] = v;
                 bad = bad || not_finite(y) || not_finite(v);
                 write_pos_c(P.pos_hi, P.pos_lo, first + e / 3, e % 3, y);
-                if (grid.enabled) reinterpret_cast<int*>(bhi)[e] = cell_coord(y, grid.inv_h);
+                if (grid.enabled) reinterpret_cast<int*>(parts)[e] = cell_coord(y, grid.inv_h);
             }
         }
     } else if (lane < 3) {
@@ -1167,7 +1182,7 @@ __global__ void __launch_bounds__(kTeamPull + kTeamBody + kTeamOwners, 1) k_team
     if (bad) S->status = 5;   // RED_ERR_NONFINITE
     if (!grid.enabled) return;   // uniform
     __syncthreads();
-    const int* cell = reinterpret_cast<const int*>(bhi);
+    const int* cell = reinterpret_cast<const int*>(parts);
     for (int b = t; b < cnt; b += blockDim.x) {
         const int4 cl = make_int4(cell[3 * b], cell[3 * b + 1], cell[3 * b + 2], 0);
         P.cell[first + b] = cl;
@@ -1227,7 +1242,7 @@ TeamKernel team_kernel(int mode)
 }
 }  // namespace
 
-int team_clusters(int mode, size_t smem)
+int team_clusters(int mode, int cluster, size_t smem)
 {
     TeamKernel k = team_kernel(mode);
     int dev = 0, most = 0, n = 0;
@@ -1237,17 +1252,18 @@ int team_clusters(int mode, size_t smem)
     cudaFuncAttributes a;
     if (cudaFuncGetAttributes(&a, k) != cudaSuccess || smem + a.sharedSizeBytes > (size_t)most ||
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes) !=
-            cudaSuccess) {
+            cudaSuccess ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(kTeamCtas);
+    cfg.gridDim = dim3((unsigned)cluster);
     cfg.blockDim = dim3(kTeamPull + kTeamBody + kTeamOwners);
     cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = kTeamCtas;
+    at[0].val.clusterDim.x = (unsigned)cluster;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
@@ -1262,7 +1278,7 @@ int team_clusters(int mode, size_t smem)
 void launch_team(const TeamParams& P, int n_ctas, int mode, cudaStream_t s)
 {
     launch_kx(team_kernel(mode), (unsigned)n_ctas, (unsigned)(kTeamPull + kTeamBody + kTeamOwners),
-              (unsigned)kTeamCtas, team_smem(P.cap, P.n_stage), s, P);
+              (unsigned)P.cluster, team_smem(P.cap, P.n_stage), s, P);
 }
 
 void set_tableau_try(const Tableau& tb, cudaStream_t s)
