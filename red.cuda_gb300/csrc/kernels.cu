@@ -380,22 +380,6 @@ __global__ void __launch_bounds__(kSegment) k_ejhc(const EjhcParams P)
     }
 }
 
-// 1 / sqrt(x) in FP64 with few FP64 instructions (GB300 issues one warp of them
-// in 16 cycles): the FP32 hardware estimate y of the truncated x, then one
-// Householder step of third order, y + y e (1/2 + 3/8 e) with e = 1 - x y^2;
-// y^2 is exact (48 bits) and e^3 ~ 2^-63, so the result is within an ulp or
-// so.  x outside FP32's normal range takes the library's function.
-__device__ __forceinline__ double rsqrt_f64(double x)
-{
-    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-    const int e = (int)(b >> 52);   // negative x and NaN are above the range
-    if (!(e > 1023 - 126 && e < 1023 + 127)) return rsqrt(x);
-    const float xf = __uint_as_float(((unsigned)(e - 1023 + 127) << 23) | (unsigned)((b >> 29) & 0x7FFFFFu));
-    const double y = f2d_bits(rsqrtf(xf));
-    const double r = fma(-x, y * y, 1.0);
-    return fma(y * r, fma(r, 0.375, 0.5), y);
-}
-
 // Potential sums in FP64, each pair once: a CTA holds kTile bodies j (one per
 // thread) against a range of bodies i, and writes sum m_i m_j / r_ij over its
 // pairs with i < j, i < ni, j < nj (indices relative to the system; ids < 0 are

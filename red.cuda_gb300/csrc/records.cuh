@@ -1,4 +1,4 @@
-// records.cuh -- what the whole-try kernels share: the tagged
+// records.cuh -- what the whole-try kernels (try.cu, try64.cu) share: the tagged
 // exchange records, the barriers of a group of warps, the step control at the end.
 #pragma once
 #include "common.cuh"

@@ -114,7 +114,7 @@ Tableau make_tableau()
 }
 
 // A scheme's Nystroem form (try.cuh) from its tableau a (rows of n_stage), b.
-void ny_row(NyTableau& n, int row, const std::vector<double>& a)
+void ny_row(NyTableau& n, int row, const std::vector<double>& a, std::vector<double>& d)
 {
     int u = n.beg[row];
     for (size_t q = 0; q < a.size(); q++)
@@ -123,6 +123,7 @@ void ny_row(NyTableau& n, int row, const std::vector<double>& a)
             t.a.x = (float)a[q];
             t.a.y = (float)(a[q] - (double)t.a.x);
             t.q = (int)q;
+            d.push_back(a[q]);
         }
     n.beg[row + 1] = u;
 }
@@ -139,7 +140,7 @@ std::vector<double> times_a(const std::vector<double>& x, const std::vector<std:
     return y;
 }
 
-NyTableau make_nystroem(const Tableau& t, int scheme)
+NyTableau make_nystroem(const Tableau& t, int scheme, std::vector<double>& d)   // d: the terms' coefficients in FP64
 {
     const int ns = scheme == SCHEME_RKF78 ? 13 : scheme == SCHEME_RK4 ? 5 : scheme == SCHEME_RK2 ? 2 : 1;
     std::vector<std::vector<double>> a(ns, std::vector<double>(ns, 0.0));
@@ -171,15 +172,16 @@ NyTableau make_nystroem(const Tableau& t, int scheme)
         if (s < ns)
             for (double x : a[s]) c += x;
         n.c[s] = (double)c;
-        ny_row(n, s, s < ns ? times_a(a[s], a) : none);
+        ny_row(n, s, s < ns ? times_a(a[s], a) : none, d);
     }
-    for (int s = 0; s < kMaxStages; s++) ny_row(n, kTryRowV + s, s < ns ? a[s] : none);
+    for (int s = 0; s < kMaxStages; s++) ny_row(n, kTryRowV + s, s < ns ? a[s] : none, d);
     long double cb = 0.0L;
     for (double x : b) cb += x;
     n.cb = (double)cb;
-    ny_row(n, kTryRowRB, times_a(b, a));
-    ny_row(n, kTryRowVB, b);
-    ny_row(n, kTryRowER, times_a(er, a));
+    ny_row(n, kTryRowRB, times_a(b, a), d);
+    ny_row(n, kTryRowVB, b, d);
+    ny_row(n, kTryRowER, times_a(er, a), d);
+    d.resize(sizeof(n.term) / sizeof(n.term[0]), 0.0);
     return n;
 }
 
@@ -577,6 +579,7 @@ struct red_sim {
     size_t try_cap = 0;
     unsigned* d_epoch = nullptr;
     NyTableau* d_ny = nullptr;
+    double* d_ny64 = nullptr;   // its terms' coefficients in FP64
     bool use_team = false;      // the same for an ensemble of sparse systems (k_team)
     int team_cluster = 0, team_cap = 0, n_team_ctas = 0;
     TeamItem* d_teams = nullptr;
@@ -661,7 +664,7 @@ red_sim::~red_sim()
     cudaFree(partial); cudaFree(tile_cnt); cudaFree(d_sys); cudaFree(d_sinfo); cudaFree(d_items); cudaFree(d_sparse_items);
     cudaFree(d_segs); cudaFree(d_pairs); cudaFree(d_events); cudaFree(d_nev); cudaFree(d_u);
     cudaFree(d_grid); cudaFree(d_head); cudaFree(d_next); cudaFree(d_cell); cudaFree(d_fsegs);
-    cudaFree(d_teams); cudaFree(d_jobs); cudaFree(d_rec); cudaFree(d_pair_items); cudaFree(d_try); cudaFree(d_epoch); cudaFree(d_ny);
+    cudaFree(d_teams); cudaFree(d_jobs); cudaFree(d_rec); cudaFree(d_pair_items); cudaFree(d_try); cudaFree(d_epoch); cudaFree(d_ny); cudaFree(d_ny64);
     cudaFree(d_xfer);
     if (h_xfer) cudaFreeHost(h_xfer);
     if (h_sys) cudaFreeHost(h_sys);
@@ -817,9 +820,12 @@ void red_sim::create(const red_config_t* c, uint32_t n_systems, const uint32_t* 
     d_nev = dalloc<unsigned int>(1);
     Tableau tb = make_tableau();
     set_tableau(tb, stream);
-    const NyTableau ny = make_nystroem(tb, scheme);
+    std::vector<double> ny64;
+    const NyTableau ny = make_nystroem(tb, scheme, ny64);
     d_ny = dalloc<NyTableau>(1);
     CK(cudaMemcpy(d_ny, &ny, sizeof(ny), cudaMemcpyHostToDevice));
+    d_ny64 = dalloc<double>(ny64.size());
+    CK(cudaMemcpy(d_ny64, ny64.data(), ny64.size() * sizeof(double), cudaMemcpyHostToDevice));
     build_plan();
     prep_positions();
     CK(cudaStreamSynchronize(stream));
@@ -1078,16 +1084,19 @@ void red_sim::launch_pair_records(int s)
 }
 
 // Whether the tries of this sim run as one cooperative launch each, and its
-// shape: one system, FP32 pair terms, up to kTryMaxLarge large bodies and small
-// ones that only these act on, whose accelerations of all stages fit in the
-// shared memory of the SMs.  At least 32 small bodies per CTA: with fewer, a
-// CTA's stage is no shorter and the exchange has more partials.  REDGB_TRY=0
-// keeps one launch per stage.
+// shape: one system, not in FP64_EXACT (whose sums have an order) and in FP64
+// without gas drag, up to kTryMaxLarge large bodies and small ones that only these
+// act on, whose accelerations of all stages fit in the shared memory of the SMs.
+// At least 32 small bodies per CTA, in FP64 16 (261 bodies, RKF7(8): 66 -> 56 us per
+// try): with fewer, a CTA's stage is no shorter and the exchange has more partials.
+// REDGB_TRY=0 keeps one launch per stage.
 void red_sim::plan_try()
 {
     use_try = false;
     const char* env = getenv("REDGB_TRY");
-    if (!allow_try || n_sys != 1 || (mode != MODE_MIXED && mode != MODE_FP32) || (env && env[0] == '0')) return;
+    if (!allow_try || n_sys != 1 || mode == MODE_FP64_EXACT || (env && env[0] == '0')) return;
+    const bool drag = cfg.gas_disk == 1, f64 = mode == MODE_FP64;
+    if (f64 && drag) return;
     const SysInfo& si = sinfo[0];
     const int nl = si.n_SI, small = si.n - nl;
     if (nl < 1 || nl > kTryMaxLarge || si.n_star > kTryMaxStars || small < 1 || si.n != si.n_massive) return;
@@ -1095,7 +1104,8 @@ void red_sim::plan_try()
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !coop)
         return;
-    int g = std::max(nl, std::min(sms, (small + 31) / 32));
+    const int least = f64 ? 16 : 32;
+    int g = std::max(nl, std::min(sms, (small + least - 1) / least));
     if (g > sms) return;
     const int nb = (small + g - 1) / g;
     g = std::max(nl, (small + nb - 1) / nb);
@@ -1103,15 +1113,18 @@ void red_sim::plan_try()
     // group has a thread per body, what is left of 1024.  Per large body,
     // as many threads as the groups that form its sum have, with four small bodies
     // or more each.
-    const bool drag = cfg.gas_disk == 1;
-    const int pull = drag ? 448 : (nb > 64 ? 384 : 256);
-    const int bodies = drag ? std::min(try_pad(nb), 448) : std::min((3 * nb + 31) / 32 * 32, 352);
-    const int owners = drag ? 128 : 32 + std::min(160, (g + 31) / 32 * 32);
+    const int pull = f64 ? kTry64Pull : drag ? 448 : (nb > 64 ? 384 : 256);
+    const int bodies = drag ? std::min(try_pad(nb), 448) : std::min((3 * nb + 31) / 32 * 32, f64 ? kTry64Bodies : 352);
+    const int owners = drag ? 128 : 32 + std::min(f64 ? kTry64Owners - 32 : 160, (g + 31) / 32 * 32);
     const int pullers = drag ? pull + bodies : pull;
     int lg = 2;
     while (lg < 5 && (2 << lg) * nl <= pullers && try_pad(nb) >= 4 * (2 << lg)) lg++;
-    if (try_ctas_per_sm(mode, drag, pull + bodies + owners, try_smem(nb, n_stage, pull)) < 1) return;
-    const size_t recs = (size_t)nl * g * 4 + (size_t)nl * 8 * kTryCopies + g + nl + 1;
+    const int threads = pull + bodies + owners;
+    if ((f64 ? try64_ctas_per_sm(threads, try64_smem(nb, n_stage, nl))
+             : try_ctas_per_sm(mode, drag, threads, try_smem(nb, n_stage, pull))) < 1)
+        return;
+    const size_t words = f64 ? 3 : 2;   // records per body
+    const size_t recs = (size_t)nl * g * 2 * words + (size_t)nl * 4 * words * kTryCopies + g + nl + 1;
     if (recs > try_cap) {
         cudaFree(d_try);
         d_try = nullptr;
@@ -1263,9 +1276,11 @@ TryParams red_sim::try_params()
     T.pos_hi = pos_hi[0];
     T.pos_lo = pos_lo[0];
     T.tab = d_ny;
+    T.tab64 = d_ny64;
+    const size_t words = mode == MODE_FP64 ? 3 : 2;   // records per body
     T.part = d_try;
-    T.pos = T.part + (size_t)si.n_SI * try_cta * 4;
-    T.err = T.pos + (size_t)si.n_SI * 8 * kTryCopies;
+    T.pos = T.part + (size_t)si.n_SI * try_cta * 2 * words;
+    T.err = T.pos + (size_t)si.n_SI * 4 * words * kTryCopies;
     T.decision = T.err + try_cta + si.n_SI;
     T.epoch = d_epoch;
     T.gas = stage_params(0, false).gas;
@@ -1384,7 +1399,8 @@ void red_sim::enqueue_try(std::vector<int>* kinds, std::vector<cudaEvent_t>* evs
             if (n_stage > 2) T.head_n = (long long)table_size;
             else CK(cudaMemsetAsync(d_head, 0xff, table_size * sizeof(int), stream));
         }
-        launch_try(T, mode, stream);
+        if (mode == MODE_FP64) launch_try64(T, stream);
+        else launch_try(T, mode, stream);
         mark(0);
         n++;
     } else {

@@ -92,8 +92,9 @@ struct TryParams {
     float4* pos_hi;          // stage-0 copies
     float4* pos_lo;
     const NyTableau* tab;
-    uint4* part;             // [2][n_large][n_cta][2]
-    uint4* pos;              // [4][kTryCopies][n_large][2]
+    const double* tab64;     // the coefficients of its terms in FP64 (try64.cu)
+    uint4* part;             // [2][n_large][n_cta][2], in FP64 [..][3]
+    uint4* pos;              // [4][kTryCopies][n_large][2], in FP64 [..][3]
     uint4* err;              // [n_cta + n_large]
     uint4* decision;         // [1]
     unsigned* epoch;         // tries made by this kernel
@@ -174,6 +175,37 @@ __host__ __device__ constexpr size_t team_smem(int cap, int n_stage)
 // Clusters resident at once (0: none, or the query failed), and the launch.
 int team_clusters(int mode, int cluster, size_t smem);
 void launch_team(const TeamParams& P, int n_ctas, int mode, cudaStream_t s);
+
+// ---------------------------------------------------------------------------
+// k_try64: k_try in FP64 (try64.cu), without gas drag.  A pair of a small and a
+// large body is formed once, for both.  A warp takes 16 small bodies and, a
+// half-warp each, two large ones at a time: a CTA's ~108 bodies of the 16384-body
+// disk fill 7 x 16 lanes, but only 3.4 x 32.  A lane adds the large bodies' pull on
+// its small body in registers; the pull on the large ones is summed over the
+// half-warp, four of them at a time.  Records hold one double each, three per body.
+//
+// Bound by the FP64 pipe: ~24 warp instructions per 32 pairs, one in ~19 cycles and
+// SM, are ~17 of the 18.7 us of a stage of the 16384-body disk with 17 large bodies.
+// The stage kernel forms a pair twice, with 16 instructions and the library's root
+// each.  That disk, adaptive RKF7(8): 535 us per try with one launch per stage, 243
+// here; RKF7(8) with fixed steps, collisions on: 261 bodies 301 -> 56 us, 65000 small
+// and 34 large ones 2190 -> 1143 us.
+// ---------------------------------------------------------------------------
+constexpr int kTry64Pull = 512, kTry64Bodies = 224, kTry64Owners = 160;   // threads of the groups (the latter two: at most)
+constexpr int kTry64Threads = kTry64Pull + kTry64Bodies + kTry64Owners;
+__host__ __device__ constexpr int try64_pad(int nb) { return (nb + 15) / 16 * 16; }
+// shares of the pairs of 16 small bodies, a warp each
+__host__ __device__ constexpr int try64_parts(int nb)
+{
+    return 256 / try64_pad(nb) < 1 ? 1 : (256 / try64_pad(nb) > 4 ? 4 : 256 / try64_pad(nb));
+}
+__host__ __device__ constexpr size_t try64_smem(int nb, int n_stage, int nl)
+{
+    return sizeof(double) * ((size_t)try64_pad(nb) * (2 * 3 + 1 + 2 * 3 * try64_parts(nb)) +
+                             (size_t)nb * 3 * (n_stage + 2) + (size_t)nl * 3 * (try64_pad(nb) / 16));
+}
+int try64_ctas_per_sm(int threads, size_t smem);
+void launch_try64(const TryParams& P, cudaStream_t s);
 
 // CTAs of the cooperative launch that are resident at once per SM with this much
 // shared memory (0: none, or the query failed), and the launch.
