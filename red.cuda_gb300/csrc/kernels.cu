@@ -200,38 +200,90 @@ __device__ __forceinline__ void collide_exact(const CollParams& P, DevSys* S, in
 }
 
 // Brute-force tile pairs: the large bodies (SI class) against every later body.
-// One thread per later body j; the i tile (the SI bodies) sits in shared
-// memory.  FP32 double-single prefilter with a safety margin, red's FP64
-// test decides.
+// A thread takes four later bodies, as two pairs of packed FP32; the i tile (the SI
+// bodies) sits in shared memory, every value twice.
+//
+// The filter sees the FP32 copies of the positions alone: two bodies closer than
+// factor (R_i + R_j) are there closer than A_i + A_j, A = factor R + 2^-23 max |x|,
+// since a copy is off by up to 2^-24 |x| in each coordinate; 1e-4 and 1e-15 cover the
+// rounding of the filter.  The few that pass, and whatever compares with NaN or
+// infinity, take red's FP64 test.
+//
+// Bound by instruction issue: ~6 a pair, where double-single differences of one pair
+// at a time took ~24.  16384 bodies, all pairs: 158 -> 57 us. The
+// rare pairs go through one copy of the FP64 test: eight inlined ones cost a
+// 261-body step 5 us of instruction fetches.
+__device__ __forceinline__ float2 coll_reach(const float4 (&H)[2], const float (&R)[2], float fac)
+{
+    float a[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+        a[q] = fmaf(fmaf(fac, fabsf(R[q]), 0x1p-23f * fmaxf(fmaxf(fabsf(H[q].x), fabsf(H[q].y)), fabsf(H[q].z))),
+                    1.0001f, 1.0e-15f);
+    return make_float2(a[0], a[1]);
+}
 __device__ __forceinline__ void coll_pairs(const CollParams& P, int item)
 {
-    __shared__ float4 shi[kTile], slo[kTile];
+    __shared__ float4 sxy[kTile], sza[kTile];   // x, x, y, y; z, z, reach, reach
     const PairItem it = P.items[item];
     DevSys* S = P.sys + it.sys;
     if (!coll_runs(P, *S)) return;
     const SysInfo si = P.sinfo[it.sys];
     const int end = si.off + si.n;
     const int ni = min(kTile, it.i1 - it.i0);
-    if (threadIdx.x < ni) {
-        shi[threadIdx.x] = P.pos_hi[it.i0 + threadIdx.x];
-        slo[threadIdx.x] = P.pos_lo[it.i0 + threadIdx.x];
+    const int t = threadIdx.x;
+    const float fac = fabsf((float)P.factor);
+    if (t < ni) {
+        const float4 H[2] = {P.pos_hi[it.i0 + t], make_float4(0.f, 0.f, 0.f, 0.f)};
+        const float R[2] = {P.pos_lo[it.i0 + t].w, 0.f};
+        const float2 A = coll_reach(H, R, fac);
+        sxy[t] = make_float4(H[0].x, H[0].x, H[0].y, H[0].y);
+        sza[t] = make_float4(H[0].z, H[0].z, A.x, A.x);
+    }
+    constexpr int N = kCollBodies / 2;
+    float2 nx[N], ny[N], nz[N], A[N];
+#pragma unroll
+    for (int p = 0; p < N; p++) {
+        float4 H[2];
+        float R[2];
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const int j = it.j0 + (2 * p + q) * kTile + t;
+            H[q] = j < end ? P.pos_hi[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+            R[q] = j < end ? P.pos_lo[j].w : 0.f;
+        }
+        nx[p] = make_float2(-H[0].x, -H[1].x);
+        ny[p] = make_float2(-H[0].y, -H[1].y);
+        nz[p] = make_float2(-H[0].z, -H[1].z);
+        A[p] = coll_reach(H, R, fac);
     }
     __syncthreads();
-    const int j = it.j0 + threadIdx.x;
-    if (j >= end) return;
-    const float4 H = P.pos_hi[j], Lo = P.pos_lo[j];
-    const float fac = (float)P.factor;
+    if (it.j0 + t >= end) return;
     const double f = P.factor * P.factor;
-    const int nii = min(ni, j - it.i0);   // i < j
-    for (int ii = 0; ii < nii; ii++) {
-        const float4 h = shi[ii], l = slo[ii];
-        const float dx = (H.x - h.x) + (Lo.x - l.x);
-        const float dy = (H.y - h.y) + (Lo.y - l.y);
-        const float dz = (H.z - h.z) + (Lo.z - l.z);
-        const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-        const float th = fac * (Lo.w + l.w);
-        if (!(d2 <= 1.0001f * th * th + 1.0e-30f)) continue;
-        collide_exact(P, S, it.sys, it.i0 + ii, j, f);
+#pragma unroll 2
+    for (int ii = 0; ii < ni; ii++) {
+        const float4 u = sxy[ii], v = sza[ii];
+        bool near[2 * N];
+        bool any = false;
+#pragma unroll
+        for (int p = 0; p < N; p++) {
+            const float2 dx = __fadd2_rn(make_float2(u.x, u.y), nx[p]), dy = __fadd2_rn(make_float2(u.z, u.w), ny[p]);
+            const float2 dz = __fadd2_rn(make_float2(v.x, v.y), nz[p]), a = __fadd2_rn(make_float2(v.z, v.w), A[p]);
+            const float2 d2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx))), a2 = __fmul2_rn(a, a);
+            near[2 * p] = !(d2.x > a2.x);
+            near[2 * p + 1] = !(d2.y > a2.y);
+            any = any || near[2 * p] || near[2 * p + 1];
+        }
+        if (!any) continue;
+        const int i = it.i0 + ii;
+        unsigned m = 0;
+#pragma unroll
+        for (int q = 0; q < 2 * N; q++) {
+            const int j = it.j0 + q * kTile + t;
+            m |= near[q] && i < j && j < end ? 1u << q : 0u;   // a body is near itself
+        }
+#pragma unroll 1
+        for (; m; m &= m - 1) collide_exact(P, S, it.sys, i, it.j0 + (__ffs((int)m) - 1) * kTile + t, f);
     }
 }
 

@@ -90,7 +90,8 @@ struct Segment {
 };
 
 // Tile pair of the brute-force collision check: i in [i0, min(i0 + kTile, i1)),
-// j in the tile starting at j0, j > i (bodies of one system).
+// j in the kCollBodies * kTile bodies from j0 on, j > i (bodies of one system).
+constexpr int kCollBodies = 4;
 struct PairItem {
     int sys, i0, j0, i1;
 };

@@ -880,11 +880,9 @@ void red_sim::build_plan()
             fsegs.push_back(Segment{(int)s, si.off + b, si.off + std::min(si.n, b + kFinishBodies), 0});
         // collision check: the SI bodies (large radii) by brute force against
         // every later body, the rest through the spatial hash grid
-        const int T = (si.n + kTile - 1) / kTile;
-        const int TI = (si.n_SI + kTile - 1) / kTile;
-        for (int I = 0; I < TI; I++)
-            for (int J = I; J < T; J++)
-                pairs.push_back(PairItem{(int)s, si.off + I * kTile, si.off + J * kTile, si.off + si.n_SI});
+        for (int i0 = 0; i0 < si.n_SI; i0 += kTile)
+            for (int j0 = i0 / (kCollBodies * kTile) * (kCollBodies * kTile); j0 < si.n; j0 += kCollBodies * kTile)
+                pairs.push_back(PairItem{(int)s, si.off + i0, si.off + j0, si.off + si.n_SI});
         GridInfo& g = grid[s];
         memset(&g, 0, sizeof(g));
         const int n_small = si.n - si.n_SI;
