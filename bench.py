@@ -251,13 +251,16 @@ def roofline_for(sim, systems, kw, peaks, traffic_per_launch, ms_per_try):
     ns = n_stage(kw)
     name = KIND_NAMES[dom]
     if name == "stage":
-        # RKF7(8): (nnz_r + 2) * 48 B per body for stage r, + 4 * 48 B error read, over the try's launches
-        if kw["integrator"] == "rkf78":
+        if launches_per_try == 1 and ns > 1:
+            # a whole try in one launch: the state in and out, the FP32 position copies, mass and id
+            per_try = 48 + 48 + 32 + 12
+        elif kw["integrator"] == "rkf78":
+            # (nnz_r + 2) * 48 B per body for stage r, + 4 * 48 B error read, over the try's launches
             nnz = [0, 1, 2, 2, 3, 3, 4, 4, 6, 7, 8, 6, 9]
             per_try = sum((nnz[r] + 2) * 48 for r in range(1, ns)) + (4 * 48 if kw.get("adaptive") else 0)
         else:
             per_try = 3 * 3 * 48 + (2 * 48 if kw.get("adaptive") else 0)
-        per_launch = per_try * n_body / ns
+        per_launch = per_try * n_body / launches_per_try
     elif name == "finish":
         per_launch = 9 * 48 * n_body
     elif name == "collision":
@@ -273,7 +276,7 @@ def roofline_for(sim, systems, kw, peaks, traffic_per_launch, ms_per_try):
            "share": share, "ms_per_try_by_kind": {KIND_NAMES[k]: ms_per_try * share[KIND_NAMES[k]] for k in tot}}
     if name == "stage":
         # the same launch against the FP32 pipe: 20 FLOP per directed interaction
-        ipe = sum(ipe_of(s.playing) for s in systems)
+        ipe = sum(ipe_of(s.playing) for s in systems) * ns / launches_per_try
         tflops = 20.0 * ipe / (in_graph_ms * 1e-3) / 1e12
         out["gravity_fp32"] = {"achieved": tflops, "peak": FP32_NOMINAL_TFLOPS, "unit": "TFLOP/s",
                                "frac": tflops / FP32_NOMINAL_TFLOPS,
