@@ -57,9 +57,10 @@ enum { RED_EVENT_NONE = 0, RED_EVENT_HIT_CENTRUM, RED_EVENT_EJECTION, RED_EVENT_
 enum { RED_THRESHOLD_HIT_CENTRUM_DISTANCE = 0, RED_THRESHOLD_EJECTION_DISTANCE,
        RED_THRESHOLD_RADII_ENHANCE_FACTOR, RED_THRESHOLD_N };
 
-/* Arithmetic of the pairwise gravity (the rest of the path is FP64 always). */
+/* Arithmetic of the pairwise gravity.  State, step control and merges are FP64 always; MIXED and FP32 may
+ * form the stage sums in double-single FP32. */
 enum {
-    RED_PREC_MIXED = 0,      /* central-star term FP64; body-body pairs in FP32 on double-single
+    RED_PREC_MIXED = 0,      /* central-star term double-single; body-body pairs in FP32 on double-single
                                 coordinates, tile sums folded into double-single accumulators */
     RED_PREC_FP64 = 1,       /* every pair FP64, tiled and split over sources */
     RED_PREC_FP64_EXACT = 2, /* red's FP64 kernel arithmetic in red's order, no FMA: bit-identical

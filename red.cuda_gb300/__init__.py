@@ -2,8 +2,10 @@
 integration hot path.
 
 The compute path is libredgb.so behind the C ABI of include/redgb.h: the
-fused stage kernel (csrc/stage.cuh, one translation unit per arithmetic mode:
-csrc/stage_{mixed,fp32,fp64,exact}.cu), the step controller, y_{n+1},
+whole-try kernels of sparse systems and ensembles (csrc/try.cu, csrc/try64.cu),
+the fused stage kernel (csrc/stage.cuh, one translation unit per arithmetic mode:
+csrc/stage_{mixed,fp32,fp64,exact}.cu), the all-pairs kernel (csrc/pairs.cu),
+the step controller (csrc/control.cuh), y_{n+1},
 collision, ejection and state-transfer kernels (csrc/kernels.cu), the C++ host
 layer (planner, graph capture, events, autotuner: csrc/sim.cu), the
 allocation-free gravity entry point (csrc/noalloc.cu), the GPU disk generator
