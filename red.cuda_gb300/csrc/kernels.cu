@@ -327,6 +327,22 @@ __device__ __forceinline__ void grid_query(const CollParams& P, int seg, int loc
     if (i >= sg.b1 || i < si.off + si.n_SI) return;
     const double f = P.factor * P.factor;
     const int4 c = P.cell[i];
+    // A neighbouring cell is looked up if the body is within a collision distance of
+    // it: with cells of four such distances 2.2 of the 14 lists on average (512 disks:
+    // the check 123 -> ~50 us).  The body's place in its cell comes from the FP32 copy,
+    // off by less than 2^-21 (|c| + 2) edges.
+    const float4 H = P.pos_hi[i];
+    const float inv_h = (float)g.inv_h;
+    bool lo[3], hi[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const int ck = k == 0 ? c.x : (k == 1 ? c.y : c.z);
+        const float u = fmaf(k == 0 ? H.x : (k == 1 ? H.y : H.z), inv_h, -(float)ck);
+        const float reach = g.reach + 0x1p-21f * (fabsf((float)ck) + 2.0f);
+        const bool any = abs(ck) >= 1 << 18;   // too far out for FP32
+        lo[k] = any || !(u > reach);
+        hi[k] = any || !(u < 1.0f - reach);
+    }
     constexpr int kNb = 14;
     int cur[kNb];
     int4 nb[kNb];
@@ -340,7 +356,9 @@ __device__ __forceinline__ void grid_query(const CollParams& P, int seg, int loc
                 const bool fwd = dz > 0 || (dz == 0 && (dy > 0 || (dy == 0 && dx >= 0)));
                 if (!fwd) continue;
                 nb[q] = make_int4(c.x + dx, c.y + dy, c.z + dz, 0);
-                cur[q] = __ldcg(P.head + g.toff + bucket_of(nb[q].x, nb[q].y, nb[q].z, g.mask));
+                const bool near = (dx == 0 || (dx < 0 ? lo[0] : hi[0])) && (dy == 0 || (dy < 0 ? lo[1] : hi[1])) &&
+                                  (dz == 0 || hi[2]);
+                cur[q] = near ? __ldcg(P.head + g.toff + bucket_of(nb[q].x, nb[q].y, nb[q].z, g.mask)) : -1;
                 q++;
             }
     // a list is at most as long as the system's small-body count: the bound ends every walk

@@ -103,7 +103,7 @@ struct GridInfo {
     double inv_h;
     int toff, mask;
     int enabled;
-    int pad;
+    float reach;          // the largest collision distance in edges (at most)
 };
 
 // Compact collision / ejection record written by the device.

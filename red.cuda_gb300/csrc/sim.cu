@@ -893,8 +893,14 @@ void red_sim::build_plan()
         if (n_small > 1 && rmax > 0.0 && factor > 0.0) {
             // cell edge >= the largest collision distance f (R_i + R_j) of two small
             // bodies, widened a little so that rounding in x / h cannot split a pair
-            // by more than one cell
-            const double h = 2.0 * factor * rmax * (1.0 + 1.0e-6) + 1.0e-300;
+            // by more than one cell.  Four times that, so that most bodies look into
+            // their own cell alone (try of 512 disks 1.83 -> 1.76 ms, of 2053 bodies 21.3
+            // -> 20.8 us), unless the radii are enlarged so much that such cells hold many
+            // bodies: 16384 bodies, check at factor 50 and 300 the same (83, 830 us), at
+            // 1000 860 against 896 us, at 3000 1348 against 1520.
+            const double edges = factor <= 300.0 ? 4.0 : 1.0;
+            const double h = edges * (2.0 * factor * rmax * (1.0 + 1.0e-6) + 1.0e-300);
+            g.reach = (float)(1.0 / edges);
             size_t m = 1024;
             while (m < 4 * (size_t)n_small) m <<= 1;
             g.inv_h = 1.0 / h;
