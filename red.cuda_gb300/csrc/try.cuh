@@ -130,7 +130,7 @@ __host__ __device__ constexpr int try_max_threads(bool drag) { return drag ? 102
 // same phases).  A large body's sum and its next position are formed by a warp
 // of the team in the phase after the partials, as long as that phase lasts.  A
 // phase of a full CTA (512 bodies) takes ~4 us.  512 disks (1.1 M bodies), adaptive
-// RKF7(8), against one launch per stage: 2.55 -> 1.53 ms per try, 0.12 of them the collision check.
+// RKF7(8), against one launch per stage: 2.55 -> 1.45 ms per try, 0.05 of them the collision check.
 // ---------------------------------------------------------------------------
 constexpr int kTeamCtas = 10;          // largest cluster; a team is at most 8 of its CTAs
 constexpr int kTeamSize = 8;
