@@ -260,40 +260,19 @@ __device__ __forceinline__ void put_comp(float4* hi, float4* lo, int b, int c, f
     reinterpret_cast<float*>(lo + b)[c] = x.y;
 }
 
-// Gas drag of a body at (H, L) with velocity v, added to its acceleration g
-// (drag_factor_fast, common.cuh, with its FP64 part in double-single: GB300's
-// FP64 rate held a stage of the 65536-body gas-drag disk for ~7 us).  The gas
-// velocity and its difference from v are good to ~1e-13 of the difference, the
-// factor f is FP32 as there.
-__device__ __forceinline__ void gas_drag(const GasDev& G, double decr, float2 mstar, float4 H, float4 L,
-                                         const float2 (&v)[3], double cd, double radius, double density, float2* g)
+// Gas drag of a body at (H, L) with velocity v, added to its acceleration g: the
+// stage kernel's, in FP64 but for the drag factor (drag_factor_fast).  With the gas
+// velocity in double-single a massless first body, whose gas is at rest, gave NaN, and
+// its rounding grows where v_gas - v cancels.
+__device__ __forceinline__ void gas_drag(const GasDev& G, double decr, double mstar, float4 H, float4 L,
+                                         const double (&v)[3], double cd, double radius, double density, float2* g)
 {
-    const float2 x = dsn(H.x, L.x), y = dsn(H.y, L.y);
-    const float2 r2 = dsn_add(dsn_sqr(x), dsn_sqr(y));   // 0 on the disk's axis: NaN drag, as red's pow(0, p < 0)
-    const float2 ir = dsn_rsqrt(r2);
-    const float r = r2.x * ir.x;
-    const float q = 2.0f * (float)G.eta[0] * powf(r, (float)G.eta[1]);
-    const float d = -q / (1.0f + sqrtf(1.0f - q));       // the gas speed is 1 + d of the circular one
-    const float2 mi = dsn_mul(mstar, ir);
-    float2 s = dsn_mul(dsn_mul(mi, dsn_rsqrt(mi)), ir);  // sqrt(m / r) / r
-    s = dsn_mul(s, dsn_norm(1.0f, d));
-    const float2 ux = dsn_sub(dsn_mul(dsn(-y.x, -y.y), s), v[0]), uy = dsn_sub(dsn_mul(x, s), v[1]);
-    const float h = (float)G.sch[0] * powf(r, (float)G.sch[1]);
-    const float zh = H.z / h;
-    const float arg = zh * zh;
-    float dens;
-    if (0.1f < r) {
-        dens = (float)G.rho[0] * powf(r, (float)G.rho[1]) * expf(-arg);
-    } else {
-        const float a = (float)G.rho[0] * powf(0.1f, (float)G.rho[1] - 4.0f);
-        dens = a * (r * r) * (r * r) * expf(-arg);
-    }
-    const float un = sqrtf(ux.x * ux.x + uy.x * uy.x + v[2].x * v[2].x);
-    const float f = (float)decr * ((3.0f * (float)cd * dens * un) / (8.0f * (float)radius * (float)density));
-    const float2 f2 = make_float2(f, 0.f);
-    g[0] = dsn_add(g[0], dsn_mul(f2, ux));
-    g[1] = dsn_add(g[1], dsn_mul(f2, uy));
-    g[2] = dsn_sub(g[2], dsn_mul(f2, v[2]));
+    double f, gx, gy;
+    drag_factor_fast(G, decr, mstar, dsn_to_double(dsn(H.x, L.x)), dsn_to_double(dsn(H.y, L.y)),
+                     dsn_to_double(dsn(H.z, L.z)), v[0], v[1], v[2], cd, radius, density, f, gx, gy);
+    g[0] = dsn_add(g[0], to_ds(f * (gx - v[0])));
+    g[1] = dsn_add(g[1], to_ds(f * (gy - v[1])));
+    g[2] = dsn_sub(g[2], to_ds(f * v[2]));
 }
 
 struct OwnerSmem {   // of the CTA that owns a large body
@@ -669,7 +648,7 @@ __global__ void __launch_bounds__(try_max_threads(DRAG)) k_try(const __grid_cons
     const float2 dt1 = to_ds(dt), dt2 = to_ds(dt * dt);
     GridInfo grid{};
     if (P.head) grid = *P.grid;
-    const float2 mstar = DRAG ? to_ds(P.mass[P.off]) : make_float2(0.f, 0.f);
+    const double mstar = DRAG ? P.mass[P.off] : 0.0;
     for (int s = 0; s <= ns; s++) {
         if (DRAG && s < ns)
             pull_large<MODE>(P, s, t, pad, bhi + (s & 1) * pad, blo + (s & 1) * pad, si_hi[s & 1], si_lo[s & 1],
@@ -695,9 +674,9 @@ __global__ void __launch_bounds__(try_max_threads(DRAG)) k_try(const __grid_cons
                         const float4 H = bhi[q * pad + b], L = blo[q * pad + b];
                         float2 dv[N];
                         row_sum(T, kTryRowV + s - 1, k, n3, dv);
-                        float2 v[3];
+                        double v[3];
 #pragma unroll
-                        for (int c = 0; c < 3; c++) v[c] = dsn_add(to_ds(yv[e + c]), dsn_mul(dv[c], dt1));
+                        for (int c = 0; c < 3; c++) v[c] = yv[e + c] + dsn_to_double(dsn_mul(dv[c], dt1));
                         const int i = first + b;
                         gas_drag(P.gas, decr, mstar, H, L, v, P.cd[i], P.radius[i], P.density[i], g);
                     }
