@@ -57,8 +57,8 @@ enum { RED_EVENT_NONE = 0, RED_EVENT_HIT_CENTRUM, RED_EVENT_EJECTION, RED_EVENT_
 enum { RED_THRESHOLD_HIT_CENTRUM_DISTANCE = 0, RED_THRESHOLD_EJECTION_DISTANCE,
        RED_THRESHOLD_RADII_ENHANCE_FACTOR, RED_THRESHOLD_N };
 
-/* Arithmetic of the pairwise gravity.  State, step control and merges are FP64 always; MIXED and FP32 may
- * form the stage sums in double-single FP32. */
+/* Arithmetic of the gravity.  The rest of the path is FP64 always: state, stage sums, error norm, step
+ * control, merges (the factor of the gas drag is FP32 in MIXED and FP32, the gas velocity FP64). */
 enum {
     RED_PREC_MIXED = 0,      /* central-star term double-single; body-body pairs in FP32 on double-single
                                 coordinates, tile sums folded into double-single accumulators */

@@ -61,6 +61,40 @@ __device__ __forceinline__ bool not_finite(double x)
     return ((__double_as_longlong(x) >> 52) & 0x7ff) == 0x7ff;
 }
 
+// sum a_q K_q over the terms [u0, u1) of the tableau, or over a row, K_q at k[q st].
+// In FP64, as every stage sum, error and solution of the whole-try kernels.
+__device__ __forceinline__ double row_sum(const NyTableau& T, int u0, int u1, const double* k, int st)
+{
+    double a = 0.0;
+#pragma unroll 4
+    for (int u = u0; u < u1; u++) a = fma(T.term[u].a, k[T.term[u].q * st], a);
+    return a;
+}
+__device__ __forceinline__ double row_sum(const NyTableau& T, int row, const double* k, int st)
+{
+    return row_sum(T, T.beg[row], T.beg[row + 1], k, st);
+}
+// The larger of a component's position error er and velocity error ev, as bits (NaN above all).
+__device__ __forceinline__ unsigned long long error_bits(double er, double ev)
+{
+    double e = fmax(fabs(er), fabs(ev));
+    if (er != er || ev != ev) e = __longlong_as_double(0x7ff8000000000000ll);
+    return (unsigned long long)__double_as_longlong(e);
+}
+__device__ __forceinline__ unsigned long long component_error(const NyTableau& T, int scheme, double dt,
+                                                              const double* k, int st)
+{
+    return error_bits(dt * row_sum(T, kTryRowER, k, st),
+                      scheme == SCHEME_RKF78 ? ((k[0] + k[10 * st]) - k[11 * st]) - k[12 * st]
+                                             : k[3 * st] - k[4 * st]);
+}
+// The solution of a component from (y, v): y + dt (cb v + dt sum), v + dt sum.
+__device__ __forceinline__ void solution(const NyTableau& T, double dt, const double* k, int st, double& y, double& v)
+{
+    y = fma(dt, fma(dt, row_sum(T, kTryRowRB, k, st), T.cb * v), y);
+    v = fma(dt, row_sum(T, kTryRowVB, k, st), v);
+}
+
 // The step control on a copy of the system record; the fields it sets go back.
 __device__ __noinline__ void control_of(const ControlParams& P, DevSys& C, unsigned long long err)
 {

@@ -114,16 +114,14 @@ Tableau make_tableau()
 }
 
 // A scheme's Nystroem form (try.cuh) from its tableau a (rows of n_stage), b.
-void ny_row(NyTableau& n, int row, const std::vector<double>& a, std::vector<double>& d)
+void ny_row(NyTableau& n, int row, const std::vector<double>& a)
 {
     int u = n.beg[row];
     for (size_t q = 0; q < a.size(); q++)
         if (a[q] != 0.0) {
             NyTerm& t = n.term[u++];
-            t.a.x = (float)a[q];
-            t.a.y = (float)(a[q] - (double)t.a.x);
+            t.a = a[q];
             t.q = (int)q;
-            d.push_back(a[q]);
         }
     n.beg[row + 1] = u;
 }
@@ -140,7 +138,7 @@ std::vector<double> times_a(const std::vector<double>& x, const std::vector<std:
     return y;
 }
 
-NyTableau make_nystroem(const Tableau& t, int scheme, std::vector<double>& d)   // d: the terms' coefficients in FP64
+NyTableau make_nystroem(const Tableau& t, int scheme)
 {
     const int ns = scheme == SCHEME_RKF78 ? 13 : scheme == SCHEME_RK4 ? 5 : scheme == SCHEME_RK2 ? 2 : 1;
     std::vector<std::vector<double>> a(ns, std::vector<double>(ns, 0.0));
@@ -172,16 +170,15 @@ NyTableau make_nystroem(const Tableau& t, int scheme, std::vector<double>& d)   
         if (s < ns)
             for (double x : a[s]) c += x;
         n.c[s] = (double)c;
-        ny_row(n, s, s < ns ? times_a(a[s], a) : none, d);
+        ny_row(n, s, s < ns ? times_a(a[s], a) : none);
     }
-    for (int s = 0; s < kMaxStages; s++) ny_row(n, kTryRowV + s, s < ns ? a[s] : none, d);
+    for (int s = 0; s < kMaxStages; s++) ny_row(n, kTryRowV + s, s < ns ? a[s] : none);
     long double cb = 0.0L;
     for (double x : b) cb += x;
     n.cb = (double)cb;
-    ny_row(n, kTryRowRB, times_a(b, a), d);
-    ny_row(n, kTryRowVB, b, d);
-    ny_row(n, kTryRowER, times_a(er, a), d);
-    d.resize(sizeof(n.term) / sizeof(n.term[0]), 0.0);
+    ny_row(n, kTryRowRB, times_a(b, a));
+    ny_row(n, kTryRowVB, b);
+    ny_row(n, kTryRowER, times_a(er, a));
     return n;
 }
 
@@ -579,7 +576,6 @@ struct red_sim {
     size_t try_cap = 0;
     unsigned* d_epoch = nullptr;
     NyTableau* d_ny = nullptr;
-    double* d_ny64 = nullptr;   // its terms' coefficients in FP64
     bool use_team = false;      // the same for an ensemble of sparse systems (k_team)
     int team_cluster = 0, team_cap = 0, n_team_ctas = 0;
     TeamItem* d_teams = nullptr;
@@ -664,7 +660,7 @@ red_sim::~red_sim()
     cudaFree(partial); cudaFree(tile_cnt); cudaFree(d_sys); cudaFree(d_sinfo); cudaFree(d_items); cudaFree(d_sparse_items);
     cudaFree(d_segs); cudaFree(d_pairs); cudaFree(d_events); cudaFree(d_nev); cudaFree(d_u);
     cudaFree(d_grid); cudaFree(d_head); cudaFree(d_next); cudaFree(d_cell); cudaFree(d_fsegs);
-    cudaFree(d_teams); cudaFree(d_jobs); cudaFree(d_rec); cudaFree(d_pair_items); cudaFree(d_try); cudaFree(d_epoch); cudaFree(d_ny); cudaFree(d_ny64);
+    cudaFree(d_teams); cudaFree(d_jobs); cudaFree(d_rec); cudaFree(d_pair_items); cudaFree(d_try); cudaFree(d_epoch); cudaFree(d_ny);
     cudaFree(d_xfer);
     if (h_xfer) cudaFreeHost(h_xfer);
     if (h_sys) cudaFreeHost(h_sys);
@@ -820,12 +816,9 @@ void red_sim::create(const red_config_t* c, uint32_t n_systems, const uint32_t* 
     d_nev = dalloc<unsigned int>(1);
     Tableau tb = make_tableau();
     set_tableau(tb, stream);
-    std::vector<double> ny64;
-    const NyTableau ny = make_nystroem(tb, scheme, ny64);
+    const NyTableau ny = make_nystroem(tb, scheme);
     d_ny = dalloc<NyTableau>(1);
     CK(cudaMemcpy(d_ny, &ny, sizeof(ny), cudaMemcpyHostToDevice));
-    d_ny64 = dalloc<double>(ny64.size());
-    CK(cudaMemcpy(d_ny64, ny64.data(), ny64.size() * sizeof(double), cudaMemcpyHostToDevice));
     build_plan();
     prep_positions();
     CK(cudaStreamSynchronize(stream));
@@ -1280,7 +1273,6 @@ TryParams red_sim::try_params()
     T.pos_hi = pos_hi[0];
     T.pos_lo = pos_lo[0];
     T.tab = d_ny;
-    T.tab64 = d_ny64;
     const size_t words = mode == MODE_FP64 ? 3 : 2;   // records per body
     T.part = d_try;
     T.pos = T.part + (size_t)si.n_SI * try_cta * 2 * words;

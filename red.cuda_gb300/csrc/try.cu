@@ -85,200 +85,50 @@ __device__ __forceinline__ float2 reduce_scatter(const Ds3& a, int lane, int lan
     return dsn_norm(kh, kl);
 }
 
-// Adds a x to the double-single sum (h, l), rounding errors carried.
-__device__ __forceinline__ void ds_term(float& h, float& l, float2 a, float2 x)
+__device__ __forceinline__ void put_comp(float4* hi, float4* lo, int b, int c, double x)
 {
-    const float p = a.x * x.x;
-    const float e = fmaf(a.y, x.x, fmaf(a.x, x.y, fmaf(a.x, x.x, -p)));
-    float sum, t;
-    two_sum(h, p, sum, t);
-    h = sum;
-    l += t + e;
-}
-// sum a_q K_q over the terms [u0, u1) of the tableau for N components; K_q of
-// component c at k[q st + c].
-template <int N>
-__device__ __forceinline__ void row_sum(const NyTableau& T, int u0, int u1, const float2* k, int st, float2 (&out)[N])
-{
-    float h[N], l[N];
-#pragma unroll
-    for (int c = 0; c < N; c++) h[c] = l[c] = 0.f;
-#pragma unroll 2
-    for (int u = u0; u < u1; u++) {
-        const float4 m = *reinterpret_cast<const float4*>(&T.term[u]);
-        const float2* x = k + __float_as_int(m.z) * st;
-#pragma unroll
-        for (int c = 0; c < N; c++) ds_term(h[c], l[c], make_float2(m.x, m.y), x[c]);
-    }
-#pragma unroll
-    for (int c = 0; c < N; c++) out[c] = dsn_norm(h[c], l[c]);
-}
-template <int N>
-__device__ __forceinline__ void row_sum(const NyTableau& T, int row, const float2* k, int st, float2 (&out)[N])
-{
-    row_sum<N>(T, T.beg[row], T.beg[row + 1], k, st, out);
-}
-__device__ __forceinline__ float2 to_ds(double x)
-{
-    float2 a;
-    split_ds(x, a.x, a.y);
-    return a;
+    float h, l;
+    split_ds(x, h, l);
+    reinterpret_cast<float*>(hi + b)[c] = h;
+    reinterpret_cast<float*>(lo + b)[c] = l;
 }
 
-// Two double-single numbers side by side, in packed FP32 (one instruction for both).
-struct D2 {
-    float2 h, l;
-};
-__device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, dup2(-1.f), a); }   // a - b, rounded once
-__device__ __forceinline__ D2 fast2(float2 a, float2 b)   // |a| >= |b|
-{
-    const float2 s = __fadd2_rn(a, b);
-    return D2{s, sub2(b, sub2(s, a))};
-}
-__device__ __forceinline__ void two_sum2(float2 a, float2 b, float2& s, float2& e)
-{
-    s = __fadd2_rn(a, b);
-    const float2 bp = sub2(s, a);
-    e = __fadd2_rn(sub2(a, sub2(s, bp)), sub2(b, bp));
-}
-__device__ __forceinline__ D2 add2(D2 a, D2 b)
-{
-    float2 s, e;
-    two_sum2(a.h, b.h, s, e);
-    return fast2(s, __fadd2_rn(e, __fadd2_rn(a.l, b.l)));
-}
-__device__ __forceinline__ D2 sub2(D2 a, D2 b)
-{
-    return add2(a, D2{__fmul2_rn(b.h, dup2(-1.f)), __fmul2_rn(b.l, dup2(-1.f))});
-}
-__device__ __forceinline__ D2 mul2(D2 a, float2 b)   // both by the double-single number b
-{
-    const float2 p = __fmul2_rn(a.h, dup2(b.x));
-    const float2 r = __ffma2_rn(a.h, dup2(b.x), __fmul2_rn(p, dup2(-1.f)));
-    return fast2(p, __ffma2_rn(a.h, dup2(b.y), __ffma2_rn(a.l, dup2(b.x), r)));
-}
-// sum a_q K_q over a row of the tableau, K_q at k[q st] as (h0, h1, l0, l1)
-__device__ __forceinline__ D2 row_sum2(const NyTableau& T, int row, const float4* k, int st)
-{
-    float2 h = make_float2(0.f, 0.f), l = h;
-    const int u1 = T.beg[row + 1];
-#pragma unroll 2
-    for (int u = T.beg[row]; u < u1; u++) {
-        const float4 m = *reinterpret_cast<const float4*>(&T.term[u]);
-        const float4 x = k[__float_as_int(m.z) * st];
-        const float2 xh = make_float2(x.x, x.y), xl = make_float2(x.z, x.w);
-        const float2 p = __fmul2_rn(xh, dup2(m.x));
-        const float2 r = __ffma2_rn(xh, dup2(m.x), __fmul2_rn(p, dup2(-1.f)));
-        const float2 e = __ffma2_rn(xh, dup2(m.y), __ffma2_rn(xl, dup2(m.x), r));
-        float2 sum, t;
-        two_sum2(h, p, sum, t);
-        h = sum;
-        l = __fadd2_rn(l, __fadd2_rn(t, e));
-    }
-    return fast2(h, l);   // |l| is far below |h| unless both vanish
-}
-
-// The larger of a component's position and velocity errors, as bits (NaN above all).
-template <int N>
-__device__ __forceinline__ unsigned long long component_error(const NyTableau& T, int scheme, float2 dt,
-                                                              const float2* k, int st)
-{
-    float2 r[N];
-    row_sum(T, kTryRowER, k, st, r);
-    unsigned long long m = 0ull;
-#pragma unroll
-    for (int c = 0; c < N; c++) {
-        const float2 d = scheme == SCHEME_RKF78
-                             ? dsn_sub(dsn_sub(dsn_add(k[c], k[10 * st + c]), k[11 * st + c]), k[12 * st + c])
-                             : dsn_sub(k[3 * st + c], k[4 * st + c]);
-        const double er = fabs(dsn_to_double(dsn_mul(r[c], dt))), ev = fabs(dsn_to_double(d));
-        double e = fmax(er, ev);
-        if (er != er || ev != ev) e = __longlong_as_double(0x7ff8000000000000ll);
-        m = max(m, (unsigned long long)__double_as_longlong(e));
-    }
-    return m;
-}
-__device__ __forceinline__ unsigned long long pair_error(const NyTableau& T, int scheme, float2 dt, const float4* k,
-                                                         int st, bool both)
-{
-    auto at = [&](int q) {
-        const float4 x = k[q * st];
-        return D2{make_float2(x.x, x.y), make_float2(x.z, x.w)};
-    };
-    const D2 r = mul2(row_sum2(T, kTryRowER, k, st), dt);
-    const D2 d = scheme == SCHEME_RKF78 ? sub2(sub2(add2(at(0), at(10)), at(11)), at(12)) : sub2(at(3), at(4));
-    const float2 rr[2] = {make_float2(r.h.x, r.l.x), make_float2(r.h.y, r.l.y)};
-    const float2 dd[2] = {make_float2(d.h.x, d.l.x), make_float2(d.h.y, d.l.y)};
-    unsigned long long m = 0ull;
-#pragma unroll
-    for (int c = 0; c < 2; c++) {
-        if (c == 1 && !both) break;
-        const double er = fabs(dsn_to_double(rr[c])), ev = fabs(dsn_to_double(dd[c]));
-        double e = fmax(er, ev);
-        if (er != er || ev != ev) e = __longlong_as_double(0x7ff8000000000000ll);
-        m = max(m, (unsigned long long)__double_as_longlong(e));
-    }
-    return m;
-}
-// The solution of N components from (y, v): y + dt (cb v) + dt^2 sum, v + dt sum.
-template <int N>
-__device__ __forceinline__ void solution(const NyTableau& T, double dt, float2 dt1, float2 dt2, const float2* k, int st,
-                                         double (&y)[N], double (&v)[N])
-{
-    float2 r[N], w[N];
-    row_sum(T, kTryRowRB, k, st, r);
-    row_sum(T, kTryRowVB, k, st, w);
-    const double cdt = T.cb * dt;
-#pragma unroll
-    for (int c = 0; c < N; c++) {
-        y[c] = fma(cdt, v[c], y[c]) + dsn_to_double(dsn_mul(r[c], dt2));
-        v[c] = v[c] + dsn_to_double(dsn_mul(w[c], dt1));
-    }
-}
-// FP32 mode takes a coordinate's high word alone, truncated as split_ds does: a
-// word rounded away from zero goes one ulp back, into the low word.
-template <int MODE>
-__device__ __forceinline__ float2 coordinate(float2 x)
-{
-    if (MODE == MODE_FP32 && x.x * x.y < 0.f) {
-        const float h = __uint_as_float(__float_as_uint(x.x) - 1u);
-        x.y += x.x - h;
-        x.x = h;
-    }
-    return x;
-}
-// The double-single position y + cdt v + inc.
-template <int MODE>
-__device__ __forceinline__ float2 position(double y, double cdt, double v, float2 inc)
-{
-    return coordinate<MODE>(dsn_add(to_ds(fma(cdt, v, y)), inc));
-}
-__device__ __forceinline__ void put_comp(float4* hi, float4* lo, int b, int c, float2 x)
-{
-    reinterpret_cast<float*>(hi + b)[c] = x.x;
-    reinterpret_cast<float*>(lo + b)[c] = x.y;
-}
-
-// Gas drag of a body at (H, L) with velocity v, added to its acceleration g: the
-// stage kernel's, in FP64 but for the drag factor (drag_factor_fast).  With the gas
-// velocity in double-single a massless first body, whose gas is at rest, gave NaN, and
-// its rounding grows where v_gas - v cancels.
+// Gas drag of a body at (H, L) with velocity v, added to its acceleration a: the
+// stage kernel's, in FP64 but for the drag factor (drag_factor_fast).
+// With the gas velocity in double-single a massless first body, whose gas is at rest,
+// gave NaN, and its rounding grows where v_gas - v cancels.
 __device__ __forceinline__ void gas_drag(const GasDev& G, double decr, double mstar, float4 H, float4 L,
-                                         const double (&v)[3], double cd, double radius, double density, float2* g)
+                                         const double (&v)[3], double cd, double radius, double density,
+                                         double (&a)[3])
 {
     double f, gx, gy;
     drag_factor_fast(G, decr, mstar, dsn_to_double(dsn(H.x, L.x)), dsn_to_double(dsn(H.y, L.y)),
                      dsn_to_double(dsn(H.z, L.z)), v[0], v[1], v[2], cd, radius, density, f, gx, gy);
-    g[0] = dsn_add(g[0], to_ds(f * (gx - v[0])));
-    g[1] = dsn_add(g[1], to_ds(f * (gy - v[1])));
-    g[2] = dsn_sub(g[2], to_ds(f * v[2]));
+    a[0] = fma(f, gx - v[0], a[0]);
+    a[1] = fma(f, gy - v[1], a[1]);
+    a[2] = fma(f, -v[2], a[2]);
+}
+
+// row_sum of N components, each a chain of its own.
+template <int N>
+__device__ __forceinline__ void stage_sums(const NyTableau& T, int row, const double* k, int st, double (&out)[N])
+{
+#pragma unroll
+    for (int c = 0; c < N; c++) out[c] = 0.0;
+    const int u1 = T.beg[row + 1];
+#pragma unroll 2
+    for (int u = T.beg[row]; u < u1; u++) {
+        const double a = T.term[u].a;
+        const double* x = k + T.term[u].q * st;
+#pragma unroll
+        for (int c = 0; c < N; c++) out[c] = fma(a, x[c], out[c]);
+    }
 }
 
 struct OwnerSmem {   // of the CTA that owns a large body
     float4 hi[kTryMaxLarge], lo[kTryMaxLarge];
     float2 red[2][kTryMaxOwners / 32 - 1][3];
-    float2 k[kMaxStages][3];
+    double k[kMaxStages][3];
     unsigned long long err;
     DevSys sys;   // CTA 0's copy of the system record
 };
@@ -311,7 +161,6 @@ __device__ __forceinline__ void run_owner(const TryParams& P, OwnerSmem& sm, con
         }
     }
     const int body = P.off + k;
-    const float2 dt1 = to_ds(dt), dt2 = to_ds(dt * dt);
     const int comp = min(lane, 2);
     const double y = ly[3 * k + comp], v = lv[3 * k + comp];
     if (w == GW) {
@@ -332,7 +181,7 @@ __device__ __forceinline__ void run_owner(const TryParams& P, OwnerSmem& sm, con
         for (int s = 0; s < P.n_stage; s++) {
             if (s < 2) {
                 for (int e = lane; e < 3 * nl; e += 32)
-                    put_comp(sm.hi, sm.lo, e / 3, e % 3, to_ds(s == 0 ? ly[e] : fma(T.c[1] * dt, lv[e], ly[e])));
+                    put_comp(sm.hi, sm.lo, e / 3, e % 3, s == 0 ? ly[e] : fma(T.c[1] * dt, lv[e], ly[e]));
             } else {
                 for (int e = lane; e < 2 * nl; e += 32) {
                     const uint4 q = poll16(pos_records(P, s) + e, tag0 + 1 + s, S, dead);
@@ -367,14 +216,12 @@ __device__ __forceinline__ void run_owner(const TryParams& P, OwnerSmem& sm, con
             g0 = make_float2(__shfl_sync(0xffffffffu, g0.x, comp), __shfl_sync(0xffffffffu, g0.y, comp));
             // the position of stage s + 2 but for the term of K_s, its row's last one if present
             const bool more = s + 2 < P.n_stage;
-            float2 base = make_float2(0.f, 0.f), coef = base;
+            double base = 0.0, coef = 0.0;
             if (more) {
                 const int u0 = T.beg[s + 2];
                 int u1 = T.beg[s + 3];
-                if (u1 > u0 && T.term[u1 - 1].q == s) coef = dsn_mul(T.term[--u1].a, dt2);
-                float2 r[1];
-                row_sum<1>(T, u0, u1, &sm.k[0][comp], 3, r);
-                base = dsn_add(to_ds(fma(T.c[s + 2] * dt, v, y)), dsn_mul(r[0], dt2));
+                if (u1 > u0 && T.term[u1 - 1].q == s) coef = dt * dt * T.term[--u1].a;
+                base = fma(dt * dt, row_sum(T, u0, u1, &sm.k[0][comp], 3), fma(T.c[s + 2] * dt, v, y));
             }
             group_sync(2, W);
             const float2(*red)[3] = sm.red[s & 1];
@@ -383,9 +230,10 @@ __device__ __forceinline__ void run_owner(const TryParams& P, OwnerSmem& sm, con
             else if (GW > 1) g = dsn_add(g, red[1][comp]);
             if (GW > 4) g = dsn_add(g, dsn_add(red[3][comp], red[4][comp]));
             else if (GW > 3) g = dsn_add(g, red[3][comp]);
-            if (!live) g = make_float2(0.f, 0.f);
+            const double a_k = live ? dsn_to_double(g) : 0.0;
             if (more) {
-                const float2 x = coordinate<MODE>(dsn_add(base, dsn_mul(coef, g)));
+                float2 x;
+                split_ds(fma(coef, a_k, base), x.x, x.y);
                 const float h1 = __shfl_sync(0xffffffffu, x.x, 1), h2 = __shfl_sync(0xffffffffu, x.x, 2);
                 const float l0 = __shfl_sync(0xffffffffu, x.y, 0), l2 = __shfl_sync(0xffffffffu, x.y, 2);
                 const float h0 = __shfl_sync(0xffffffffu, x.x, 0), l1 = __shfl_sync(0xffffffffu, x.y, 1);
@@ -395,14 +243,13 @@ __device__ __forceinline__ void run_owner(const TryParams& P, OwnerSmem& sm, con
                              __float_as_uint(lane & 1 ? l2 : h2), tag0 + 3 + s);
                 }
             }
-            if (lane < 3) sm.k[s][lane] = g;
+            if (lane < 3) sm.k[s][lane] = a_k;
             __syncwarp();
         }
     }
     // the solution, the error, the decision: the last warp; CTA 0's others gather the errors
-    double rn[1] = {y}, vn[1] = {v};
     if (P.adaptive && w == GW) {
-        unsigned long long eb = component_error<1>(T, P.scheme, dt1, &sm.k[0][comp], 3);
+        unsigned long long eb = component_error(T, P.scheme, dt, &sm.k[0][comp], 3);
         const unsigned long long e1 = __shfl_sync(0xffffffffu, eb, 1), e2 = __shfl_sync(0xffffffffu, eb, 2);
         eb = max(eb, max(e1, e2));
         if (lane == 0) st_rec16(P.err + P.n_cta + k, (unsigned)eb, (unsigned)(eb >> 32), 0u, tag0 + 14);
@@ -429,7 +276,8 @@ __device__ __forceinline__ void run_owner(const TryParams& P, OwnerSmem& sm, con
         *P.epoch = tag0 / 16 + 1;
     }
     if (w != GW) return;
-    solution<1>(T, dt, dt1, dt2, &sm.k[0][comp], 3, rn, vn);
+    double rn = y, vn = v;
+    solution(T, dt, &sm.k[0][comp], 3, rn, vn);
     bool accepted = true;
     if (P.adaptive) {
         unsigned acc = 0u;
@@ -437,10 +285,10 @@ __device__ __forceinline__ void run_owner(const TryParams& P, OwnerSmem& sm, con
         accepted = __shfl_sync(0xffffffffu, acc, 0) == 1u;
     }
     if (lane < 3 && accepted) {
-        P.y_r[3 * body + lane] = rn[0];
-        P.y_v[3 * body + lane] = vn[0];
-        if (not_finite(rn[0]) || not_finite(vn[0])) S->status = 5;   // RED_ERR_NONFINITE
-        write_pos_c(P.pos_hi, P.pos_lo, body, lane, rn[0]);
+        P.y_r[3 * body + lane] = rn;
+        P.y_v[3 * body + lane] = vn;
+        if (not_finite(rn) || not_finite(vn)) S->status = 5;   // RED_ERR_NONFINITE
+        write_pos_c(P.pos_hi, P.pos_lo, body, lane, rn);
     }
 }
 
@@ -545,8 +393,8 @@ __global__ void __launch_bounds__(try_max_threads(DRAG)) k_try(const __grid_cons
     float4* blo = bhi + 2 * pad;
     float2* parts = reinterpret_cast<float2*>(blo + 2 * pad);   // [2][np][pad][3]
     const int n3 = 3 * nb;
-    float2* ks = parts + (size_t)2 * np * 3 * pad;              // accelerations, [stage][nb][3]
-    double* yr = reinterpret_cast<double*>(ks + (size_t)ns * n3);   // [nb][3]
+    double* ks = reinterpret_cast<double*>(parts + (size_t)2 * np * 3 * pad);   // accelerations, [stage][nb][3]
+    double* yr = ks + (size_t)ns * n3;                          // [nb][3]
     double* yv = yr + n3;
 
     // ---- everything the try starts from, read before this CTA's first record, so
@@ -645,7 +493,6 @@ __global__ void __launch_bounds__(try_max_threads(DRAG)) k_try(const __grid_cons
     // ---- the body group: K of the previous stage, positions of the next ----
     constexpr int N = DRAG ? 3 : 1;   // components of a thread; its item x: component x % 3 of body x / 3, or body x
     const int tb = t - P.pull, items = DRAG ? cnt : 3 * cnt;
-    const float2 dt1 = to_ds(dt), dt2 = to_ds(dt * dt);
     GridInfo grid{};
     if (P.head) grid = *P.grid;
     const double mstar = DRAG ? P.mass[P.off] : 0.0;
@@ -657,28 +504,27 @@ __global__ void __launch_bounds__(try_max_threads(DRAG)) k_try(const __grid_cons
         if (DRAG && s > 0) decr = gas_reduction_factor<false>(P.gas, tsys + stage_c(P.scheme, s - 1) * dt);
         for (int x = tb; x < items; x += P.bodies) {
             const int b = DRAG ? x : x / 3, e = N * x;
-            float2* k = ks + e;
+            double* k = ks + e;
             if (s > 0) {
                 const int q = (s - 1) & 1;
                 const float2* pt = parts + (size_t)q * np * 3 * pad + e;
                 const bool live = blo[b].w != 0.f;
-                float2 g[N];
+                double g[N];
 #pragma unroll
                 for (int c = 0; c < N; c++) {
-                    g[c] = pt[c];
-                    for (int u = 1; u < np; u++) g[c] = dsn_add(g[c], pt[3 * u * pad + c]);
-                    if (!live) g[c] = make_float2(0.f, 0.f);
+                    float2 a = pt[c];
+                    for (int u = 1; u < np; u++) a = dsn_add(a, pt[3 * u * pad + c]);
+                    g[c] = live ? dsn_to_double(a) : 0.0;
                 }
                 if constexpr (DRAG) {
                     if (!(1.0e-6 > decr)) {
-                        const float4 H = bhi[q * pad + b], L = blo[q * pad + b];
-                        float2 dv[N];
-                        row_sum(T, kTryRowV + s - 1, k, n3, dv);
                         double v[3];
+                        stage_sums(T, kTryRowV + s - 1, k, n3, v);
 #pragma unroll
-                        for (int c = 0; c < 3; c++) v[c] = yv[e + c] + dsn_to_double(dsn_mul(dv[c], dt1));
+                        for (int c = 0; c < 3; c++) v[c] = fma(dt, v[c], yv[e + c]);
                         const int i = first + b;
-                        gas_drag(P.gas, decr, mstar, H, L, v, P.cd[i], P.radius[i], P.density[i], g);
+                        gas_drag(P.gas, decr, mstar, bhi[q * pad + b], blo[q * pad + b], v, P.cd[i], P.radius[i],
+                                 P.density[i], g);
                     }
                 }
 #pragma unroll
@@ -686,20 +532,20 @@ __global__ void __launch_bounds__(try_max_threads(DRAG)) k_try(const __grid_cons
             }
             if (s + 1 < ns) {
                 const int q = (s + 1) & 1;
-                float2 r[N];
-                row_sum(T, s + 1, k, n3, r);
-                const double cdt = T.c[s + 1] * dt;
+                double r[N];
+                stage_sums(T, s + 1, k, n3, r);
+                const double cdt = T.c[s + 1] * dt, dt2 = dt * dt;
 #pragma unroll
                 for (int c = 0; c < N; c++)
                     put_comp(bhi + q * pad, blo + q * pad, b, DRAG ? c : x % 3,
-                             position<MODE>(yr[e + c], cdt, yv[e + c], dsn_mul(r[c], dt2)));
+                             fma(dt2, r[c], fma(cdt, yv[e + c], yr[e + c])));
             }
         }
         if (s == ns) break;
         if (s == 0) {   // the large bodies' positions of stage 1
             if (ns > 1)
                 for (int e = tb; e < 3 * nl; e += P.bodies)
-                    put_comp(si_hi[1], si_lo[1], e / 3, e % 3, to_ds(fma(T.c[1] * dt, lv[e], ly[e])));
+                    put_comp(si_hi[1], si_lo[1], e / 3, e % 3, fma(T.c[1] * dt, lv[e], ly[e]));
         } else if (s + 1 < ns) {
             const int q = (s + 1) & 1;
             for (int e = tb; e < 2 * nl; e += P.bodies) {
@@ -718,27 +564,17 @@ __global__ void __launch_bounds__(try_max_threads(DRAG)) k_try(const __grid_cons
     // ---- the error, the solution (formed while the decision is on its way) ----
     if (P.adaptive) {
         unsigned long long eb = 0ull;
-        for (int x = tb; x < items; x += P.bodies) eb = max(eb, component_error<N>(T, P.scheme, dt1, ks + N * x, n3));
+        for (int x = tb; x < items; x += P.bodies)   // the threads that formed the accelerations
+#pragma unroll
+            for (int c = 0; c < N; c++) eb = max(eb, component_error(T, P.scheme, dt, ks + N * x + c, n3));
         for (int m = 16; m > 0; m >>= 1) eb = max(eb, __shfl_xor_sync(0xffffffffu, eb, m));
         if ((tb & 31) == 0) atomicMax(&err_sm, eb);
         group_sync(3, P.bodies);
         if (tb == 0) st_rec16(P.err + blockIdx.x, (unsigned)err_sm, (unsigned)(err_sm >> 32), 0u, tag0 + 14);
     }
-    for (int x = tb; x < items; x += P.bodies) {
-        const int e = N * x;
-        double y[N], v[N];
+    for (int x = tb; x < items; x += P.bodies)
 #pragma unroll
-        for (int c = 0; c < N; c++) {
-            y[c] = yr[e + c];
-            v[c] = yv[e + c];
-        }
-        solution(T, dt, dt1, dt2, ks + e, n3, y, v);
-#pragma unroll
-        for (int c = 0; c < N; c++) {
-            yr[e + c] = y[c];
-            yv[e + c] = v[c];
-        }
-    }
+        for (int c = 0; c < N; c++) solution(T, dt, ks + N * x + c, n3, yr[N * x + c], yv[N * x + c]);
     if (P.adaptive) {
         if (tb == 0) take = poll16(P.decision, tag0 + 15, S, &dead).x == 1u;
         group_sync(3, P.bodies);
@@ -800,6 +636,36 @@ __device__ __forceinline__ void st_peer(unsigned a, unsigned long long v)
     asm volatile("st.shared::cluster.b64 [%0], %1;\n" ::"r"(a), "l"(v) : "memory");
 }
 
+// row_sum and component_error of a pair of components.
+__device__ __forceinline__ double2 pair_sums(const NyTableau& T, int row, const double2* k, int st)
+{
+    double2 r = make_double2(0.0, 0.0);
+    const int u1 = T.beg[row + 1];
+#pragma unroll 4
+    for (int u = T.beg[row]; u < u1; u++) {
+        const double a = T.term[u].a;
+        const double2 x = k[T.term[u].q * st];
+        r.x = fma(a, x.x, r.x);
+        r.y = fma(a, x.y, r.y);
+    }
+    return r;
+}
+__device__ __forceinline__ unsigned long long pair_error(const NyTableau& T, int scheme, double dt, const double2* k,
+                                                         int st, bool both)
+{
+    const double2 r = pair_sums(T, kTryRowER, k, st);
+    double2 d;
+    if (scheme == SCHEME_RKF78) {
+        const double2 a = k[0], b = k[10 * st], c = k[11 * st], e = k[12 * st];
+        d = make_double2(((a.x + b.x) - c.x) - e.x, ((a.y + b.y) - c.y) - e.y);
+    } else {
+        const double2 a = k[3 * st], b = k[4 * st];
+        d = make_double2(a.x - b.x, a.y - b.y);
+    }
+    const unsigned long long m = error_bits(dt * r.x, d.x);
+    return both ? max(m, error_bits(dt * r.y, d.y)) : m;
+}
+
 struct TeamSmem {
     float4 si_hi[3][kTeamLarge], si_lo[3][kTeamLarge];   // the large bodies, by stage mod 3
     float2 star_m[kTryMaxStars];
@@ -807,7 +673,7 @@ struct TeamSmem {
     double ly[3 * kTeamLarge], lv[3 * kTeamLarge];
     NyTableau T;
     float2 part[2][2 * (kTeamLarge + kTeamSize)][3];   // partials of the bodies owned here: stage parity; slot, rank, half
-    float2 k[kTeamLarge][kMaxStages][3];         // their accelerations
+    double k[kTeamLarge][kMaxStages][3];         // their accelerations
     unsigned long long err, all, errs[kTeamSize];     // this CTA's error; the team's; its CTAs', in the first of them
     DevSys sys;
     int live[kTeamLarge];
@@ -857,7 +723,7 @@ __global__ void __launch_bounds__(kTeamPull + kTeamBody + kTeamOwners, 1) k_team
     float4* bhi = reinterpret_cast<float4*>(dyn);               // [2][pad], by stage parity
     float4* blo = bhi + 2 * pad;
     float2* parts = reinterpret_cast<float2*>(blo + 2 * pad);   // [2][pad][3]
-    float4* ks = reinterpret_cast<float4*>(parts + (size_t)2 * 3 * pad);   // [stage][pair]: (h0, h1, l0, l1)
+    double2* ks = reinterpret_cast<double2*>(parts + (size_t)2 * 3 * pad);   // [stage][pair]
 
     // ---- load ----
     for (int b = t; b < pad; b += blockDim.x) {
@@ -882,7 +748,7 @@ __global__ void __launch_bounds__(kTeamPull + kTeamBody + kTeamOwners, 1) k_team
     if (t < 3 * nl) {
         sm.ly[t] = P.y_r[3 * si.off + t];
         sm.lv[t] = P.y_v[3 * si.off + t];
-        put_comp(sm.si_hi[0], sm.si_lo[0], t / 3, t % 3, to_ds(sm.ly[t]));
+        put_comp(sm.si_hi[0], sm.si_lo[0], t / 3, t % 3, sm.ly[t]);
     }
     if (t < nl) {
         const int id = P.id[si.off + t];
@@ -904,7 +770,7 @@ __global__ void __launch_bounds__(kTeamPull + kTeamBody + kTeamOwners, 1) k_team
                 P.head[grid.toff + k] = -1;
     }
     const NyTableau& T = sm.T;
-    const float2 dt1 = to_ds(dt), dt2 = to_ds(dt * dt);
+    const double dt2 = dt * dt;
     cluster_sync();
 
     const bool puller = t < kTeamPull, owner = t >= kTeamPull + kTeamBody;
@@ -940,29 +806,26 @@ __global__ void __launch_bounds__(kTeamPull + kTeamBody + kTeamOwners, 1) k_team
                 const int e = 2 * x, b = e / 3, c = e - 3 * b;   // component c of body b, and the next one
                 const int b2 = c == 2 ? b + 1 : b, d = c == 2 ? 0 : c + 1;
                 const bool both = e + 1 < 3 * cnt;
-                float4* k = ks + x;
+                double2* k = ks + x;
                 if (s > 0) {
                     const float4 g = *reinterpret_cast<const float4*>(parts + (size_t)(q ^ 1) * 3 * pad + e);
                     const float m0 = blo[b].w, m1 = blo[b2].w;   // 1, or 0 for an inactive body
-                    k[(size_t)(s - 1) * np] = make_float4(m0 != 0.f ? g.x : 0.f, m1 != 0.f ? g.z : 0.f,
-                                                          m0 != 0.f ? g.y : 0.f, m1 != 0.f ? g.w : 0.f);
+                    k[(size_t)(s - 1) * np] = make_double2(m0 != 0.f ? dsn_to_double(make_float2(g.x, g.y)) : 0.0,
+                                                           m1 != 0.f ? dsn_to_double(make_float2(g.z, g.w)) : 0.0);
                 }
                 if (s + 1 < ns) {
                     const double cdt = T.c[s + 1] * dt;
                     const size_t i = 3 * (size_t)first + e, j = both ? i + 1 : i;
-                    const float2 u = to_ds(fma(cdt, P.y_v[i], P.y_r[i])), w = to_ds(fma(cdt, P.y_v[j], P.y_r[j]));
-                    const D2 r = add2(D2{make_float2(u.x, w.x), make_float2(u.y, w.y)},
-                                      mul2(row_sum2(T, s + 1, k, np), dt2));
+                    const double2 r = pair_sums(T, s + 1, k, np);
                     put_comp(bhi + (q ^ 1) * pad, blo + (q ^ 1) * pad, b, c,
-                             coordinate<MODE>(make_float2(r.h.x, r.l.x)));
+                             fma(dt2, r.x, fma(cdt, P.y_v[i], P.y_r[i])));
                     if (both)
                         put_comp(bhi + (q ^ 1) * pad, blo + (q ^ 1) * pad, b2, d,
-                                 coordinate<MODE>(make_float2(r.h.y, r.l.y)));
+                                 fma(dt2, r.y, fma(cdt, P.y_v[j], P.y_r[j])));
                 }
             }
             if (s == 0 && ns > 1 && tb >= 0 && tb < 3 * nl)
-                put_comp(sm.si_hi[1], sm.si_lo[1], tb / 3, tb % 3,
-                         to_ds(fma(T.c[1] * dt, sm.lv[tb], sm.ly[tb])));
+                put_comp(sm.si_hi[1], sm.si_lo[1], tb / 3, tb % 3, fma(T.c[1] * dt, sm.lv[tb], sm.ly[tb]));
         } else if (s > 0) {
             // a warp per large body owned here: slot u is body u size + rank
             const int p3 = (s - 1) % 3;
@@ -988,15 +851,14 @@ __global__ void __launch_bounds__(kTeamPull + kTeamBody + kTeamOwners, 1) k_team
                     ds_merge(a.yh, a.yl, pt[1].x, pt[1].y);
                     ds_merge(a.zh, a.zl, pt[2].x, pt[2].y);
                 }
-                float2 g = reduce_scatter(a, lane, 32);
-                if (!sm.live[k]) g = make_float2(0.f, 0.f);
-                if (lane < 3) sm.k[u][s - 1][lane] = g;
+                const float2 g = reduce_scatter(a, lane, 32);
+                if (lane < 3) sm.k[u][s - 1][lane] = sm.live[k] ? dsn_to_double(g) : 0.0;
                 __syncwarp();
                 if (s + 1 < ns) {
-                    float2 r[1];
-                    row_sum<1>(T, s + 1, &sm.k[u][0][comp], 3, r);
-                    const float2 x =
-                        position<MODE>(sm.ly[3 * k + comp], T.c[s + 1] * dt, sm.lv[3 * k + comp], dsn_mul(r[0], dt2));
+                    float2 x;
+                    split_ds(fma(dt2, row_sum(T, s + 1, &sm.k[u][0][comp], 3),
+                                 fma(T.c[s + 1] * dt, sm.lv[3 * k + comp], sm.ly[3 * k + comp])),
+                             x.x, x.y);
                     if (lane < 3) {
                         const int n3s = (s + 1) % 3;
                         float* h = reinterpret_cast<float*>(&sm.si_hi[n3s][k]) + lane;
@@ -1018,10 +880,10 @@ __global__ void __launch_bounds__(kTeamPull + kTeamBody + kTeamOwners, 1) k_team
         unsigned long long eb = 0ull;
         if (!owner) {
             for (int x = x0; x < x1; x += xs)
-                eb = max(eb, pair_error(T, P.scheme, dt1, ks + x, np, 2 * x + 1 < 3 * cnt));
+                eb = max(eb, pair_error(T, P.scheme, dt, ks + x, np, 2 * x + 1 < 3 * cnt));
         } else if (lane < 3) {
             for (int u = ow; u < own_n; u += kTeamOwners / 32)
-                eb = max(eb, component_error<1>(T, P.scheme, dt1, &sm.k[u][0][lane], 3));
+                eb = max(eb, component_error(T, P.scheme, dt, &sm.k[u][0][lane], 3));
         }
         for (int m = 16; m > 0; m >>= 1) eb = max(eb, __shfl_xor_sync(0xffffffffu, eb, m));
         if (lane == 0) atomicMax(&sm.err, eb);
@@ -1034,14 +896,14 @@ __global__ void __launch_bounds__(kTeamPull + kTeamBody + kTeamOwners, 1) k_team
     if (!owner) {
         const double cdt = T.cb * dt;
         for (int x = x0; x < x1; x += xs) {
-            const D2 r = mul2(row_sum2(T, kTryRowRB, ks + x, np), dt2), w = mul2(row_sum2(T, kTryRowVB, ks + x, np), dt1);
+            const double2 r = pair_sums(T, kTryRowRB, ks + x, np), w = pair_sums(T, kTryRowVB, ks + x, np);
             const size_t i = 3 * (size_t)first + 2 * x, j = 2 * x + 1 < 3 * cnt ? i + 1 : i;
             const double v0 = P.y_v[i], v1 = P.y_v[j];
             double* o = sol + x;
-            o[0] = fma(cdt, v0, P.y_r[i]) + dsn_to_double(make_float2(r.h.x, r.l.x));
-            o[np] = fma(cdt, v1, P.y_r[j]) + dsn_to_double(make_float2(r.h.y, r.l.y));
-            o[2 * np] = v0 + dsn_to_double(make_float2(w.h.x, w.l.x));
-            o[3 * np] = v1 + dsn_to_double(make_float2(w.h.y, w.l.y));
+            o[0] = fma(dt2, r.x, fma(cdt, v0, P.y_r[i]));
+            o[np] = fma(dt2, r.y, fma(cdt, v1, P.y_r[j]));
+            o[2 * np] = fma(dt, w.x, v0);
+            o[3 * np] = fma(dt, w.y, v1);
         }
     }
     cluster_wait();
@@ -1080,12 +942,12 @@ __global__ void __launch_bounds__(kTeamPull + kTeamBody + kTeamOwners, 1) k_team
     } else if (lane < 3) {
         for (int u = ow; u < own_n; u += kTeamOwners / 32) {
             const int k = u * it.size + it.rank, x = 3 * (si.off + k) + lane;
-            double y[1] = {sm.ly[3 * k + lane]}, v[1] = {sm.lv[3 * k + lane]};
-            solution<1>(T, dt, dt1, dt2, &sm.k[u][0][lane], 3, y, v);
-            P.y_r[x] = y[0];
-            P.y_v[x] = v[0];
-            bad = bad || not_finite(y[0]) || not_finite(v[0]);
-            write_pos_c(P.pos_hi, P.pos_lo, si.off + k, lane, y[0]);
+            double y = sm.ly[3 * k + lane], v = sm.lv[3 * k + lane];
+            solution(T, dt, &sm.k[u][0][lane], 3, y, v);
+            P.y_r[x] = y;
+            P.y_v[x] = v;
+            bad = bad || not_finite(y) || not_finite(v);
+            write_pos_c(P.pos_hi, P.pos_lo, si.off + k, lane, y);
         }
     }
     if (bad) S->status = 5;   // RED_ERR_NONFINITE

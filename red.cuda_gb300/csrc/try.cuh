@@ -18,19 +18,21 @@
 // large body, its new position back to all) therefore has the time of a whole
 // stage to complete, and stage velocities are formed only for gas drag.
 //
-// The accelerations are double-single, as the pair and star sums leave them (the
-// star term is good to ~2e-14), and so are the sums over them, good to 2^-47: the
-// positions y_r + dt c v_y are formed in FP64, the increments are added as
-// double-single, and the solution adds its increments to the FP64 state.  GB300
-// issues an FP64 warp instruction every 19 cycles and SM and a dependent one
-// takes 64; the ~12 FP32 instructions of a double-single term take 3.
+// The pair and star sums leave the accelerations as double-single numbers (the star
+// term is good to ~2e-14); everything formed from them is FP64, as in the stage
+// kernel: the stage sums, positions and velocities, the drag, the error, the solution.
+// GB300 issues an FP64 warp instruction every 19 cycles and SM and a dependent one
+// takes 64, so a component's sum is one thread's chain, off the exchange's path but for
+// the last term.  (Double-single sums, ~12 FP32 instructions a term, took 56 instead of
+// 59 us per try of the 16384-body disk.  They round at 2^-47, and the modes promise
+// FP64.)
 //
 // Bound: latency -- of the exchange, two trips through L2 per two stages, and of
 // the instruction chains of a phase (~2.7 us per phase on the 16384-body disk, 1.3
 // of them the pull on the large bodies, whose records the exchange waits for).
 // Measured against one launch per stage, per try: 16384-body disk, adaptive
-// RKF7(8), 115 -> 57 us; 65536-body gas-drag disk 418 -> 175 us; 2053-body disk,
-// RK4, 33.2 -> 21.2 us.  What that took besides the layout: the system record is
+// RKF7(8), 115 -> 59 us; 65536-body gas-drag disk 418 -> 258 us (FP64 pipe: the rows of
+// velocities and the drag); 2053-body disk, RK4, 33.2 -> 20.6 us.  What that took besides the layout: the system record is
 // read by one thread of a CTA and the position records are written in kTryCopies
 // copies, because thousands of readers of one sector queue up for microseconds.
 //
@@ -63,7 +65,7 @@ constexpr int kTryPollLimit = 1 << 20;
 constexpr int kTryRowV = kMaxStages, kTryRowRB = 2 * kMaxStages, kTryRowVB = kTryRowRB + 1, kTryRowER = kTryRowVB + 1;
 constexpr int kTryRows = kTryRowER + 1;
 struct NyTerm {
-    float2 a;                // the coefficient, double-single
+    double a;                // the coefficient
     int q, pad;              // the stage
 };
 struct alignas(16) NyTableau {
@@ -92,7 +94,6 @@ struct TryParams {
     float4* pos_hi;          // stage-0 copies
     float4* pos_lo;
     const NyTableau* tab;
-    const double* tab64;     // the coefficients of its terms in FP64 (try64.cu)
     uint4* part;             // [2][n_large][n_cta][2], in FP64 [..][3]
     uint4* pos;              // [4][kTryCopies][n_large][2], in FP64 [..][3]
     uint4* err;              // [n_cta + n_large]
@@ -117,7 +118,7 @@ __host__ __device__ constexpr int try_parts(int nb, int pull)
 __host__ __device__ constexpr size_t try_smem(int nb, int n_stage, int pull)
 {
     return (size_t)try_pad(nb) * 2 * (2 * sizeof(float4) + (size_t)try_parts(nb, pull) * 3 * sizeof(float2)) +
-           (size_t)nb * 3 * (sizeof(float2) * n_stage + sizeof(double) * 2);
+           (size_t)nb * 3 * sizeof(double) * (n_stage + 2);
 }
 // Threads of a CTA at most.
 __host__ __device__ constexpr int try_max_threads(bool drag) { return drag ? 1024 : 928; }
@@ -128,9 +129,9 @@ __host__ __device__ constexpr int try_max_threads(bool drag) { return drag ? 102
 // teams of a cluster side by side; the exchange goes through the CTAs' shared
 // memory, ordered by one cluster barrier per phase (the cluster's CTAs run the
 // same phases).  A large body's sum and its next position are formed by a warp
-// of the team in the phase after the partials, as long as that phase lasts.  A
-// phase of a full CTA (512 bodies) takes ~4 us.  512 disks (1.1 M bodies), adaptive
-// RKF7(8), against one launch per stage: 2.55 -> 1.45 ms per try, 0.05 of them the collision check.
+// of the team in the phase after the partials, as long as that phase lasts.  512
+// disks (1.1 M bodies), adaptive RKF7(8), four tries with the states in and out, against
+// one launch per stage: 11.35 -> 8.29 ms (7.04 with double-single stage sums).
 // ---------------------------------------------------------------------------
 constexpr int kTeamCtas = 10;          // largest cluster; a team is at most 8 of its CTAs
 constexpr int kTeamSize = 8;
@@ -170,7 +171,7 @@ struct TeamParams {
 __host__ __device__ constexpr size_t team_smem(int cap, int n_stage)
 {
     return (size_t)try_pad(cap) * 2 * (2 * sizeof(float4) + 3 * sizeof(float2)) +
-           (size_t)cap * 3 * sizeof(float2) * n_stage;
+           (size_t)cap * 3 * sizeof(double) * n_stage;
 }
 // Clusters resident at once (0: none, or the query failed), and the launch.
 int team_clusters(int mode, int cluster, size_t smem);

@@ -86,31 +86,6 @@ __device__ __forceinline__ double warp_sum3(double x, double y, double z, int la
     return k;
 }
 
-struct Tab64 {   // the tableau in shared memory
-    NyTableau t;
-    double a[sizeof(NyTableau::term) / sizeof(NyTerm)];
-};
-__device__ __forceinline__ double row_sum64(const Tab64& T, int u0, int u1, const double* k, int st)
-{
-    double a = 0.0;
-#pragma unroll 4
-    for (int u = u0; u < u1; u++) a = fma(T.a[u], k[T.t.term[u].q * st], a);
-    return a;
-}
-__device__ __forceinline__ double row_sum64(const Tab64& T, int row, const double* k, int st)
-{
-    return row_sum64(T, T.t.beg[row], T.t.beg[row + 1], k, st);
-}
-__device__ __forceinline__ unsigned long long error64(const Tab64& T, int scheme, double dt, const double* k, int st)
-{
-    const double er = fabs(dt * row_sum64(T, kTryRowER, k, st));
-    const double ev = scheme == SCHEME_RKF78 ? fabs(((k[0] + k[10 * st]) - k[11 * st]) - k[12 * st])
-                                             : fabs(k[3 * st] - k[4 * st]);
-    double e = fmax(er, ev);
-    if (er != er || ev != ev) e = __longlong_as_double(0x7ff8000000000000ll);
-    return (unsigned long long)__double_as_longlong(e);
-}
-
 struct Owner64 {
     double pos[3 * kTryMaxLarge];
     double red[2][kTryMaxOwners / 32 - 1][3];
@@ -125,7 +100,7 @@ __device__ __forceinline__ const uint4* pos_records64(const TryParams& P, int s)
 }
 
 // run_owner (try.cu) in FP64.
-__device__ __forceinline__ void run_owner64(const TryParams& P, Owner64& sm, const Tab64& T, volatile int* dead,
+__device__ __forceinline__ void run_owner64(const TryParams& P, Owner64& sm, const NyTableau& T, volatile int* dead,
                                             unsigned tag0, double dt, const double* ly, const double* lv, int o)
 {
     const int k = blockIdx.x, nl = P.n_large;
@@ -160,7 +135,7 @@ __device__ __forceinline__ void run_owner64(const TryParams& P, Owner64& sm, con
         for (int s = 0; s < P.n_stage; s++) {
             for (int e = lane; e < 3 * nl; e += 32)
                 sm.pos[e] = s == 0 ? ly[e]
-                                   : (s == 1 ? fma(T.t.c[1] * dt, lv[e], ly[e])
+                                   : (s == 1 ? fma(T.c[1] * dt, lv[e], ly[e])
                                              : poll_rec(pos_records64(P, s) + e, tag0 + 1 + s, S, dead));
             __syncwarp();
             double ax = 0.0, ay = 0.0, az = 0.0;
@@ -181,11 +156,11 @@ __device__ __forceinline__ void run_owner64(const TryParams& P, Owner64& sm, con
             const bool more = s + 2 < P.n_stage;
             double base = 0.0, sum = 0.0, coef = 0.0;
             if (more) {
-                const int u0 = T.t.beg[s + 2];
-                int u1 = T.t.beg[s + 3];
-                if (u1 > u0 && T.t.term[u1 - 1].q == s) coef = T.a[--u1];
-                sum = row_sum64(T, u0, u1, &sm.k[0][comp], 3);
-                base = fma(T.t.c[s + 2] * dt, v, y);
+                const int u0 = T.beg[s + 2];
+                int u1 = T.beg[s + 3];
+                if (u1 > u0 && T.term[u1 - 1].q == s) coef = T.term[--u1].a;
+                sum = row_sum(T, u0, u1, &sm.k[0][comp], 3);
+                base = fma(T.c[s + 2] * dt, v, y);
             }
             __syncwarp();
             lanes_sync(2, W);
@@ -203,7 +178,7 @@ __device__ __forceinline__ void run_owner64(const TryParams& P, Owner64& sm, con
         }
     }
     if (P.adaptive && w == GW) {
-        unsigned long long eb = error64(T, P.scheme, dt, &sm.k[0][comp], 3);
+        unsigned long long eb = component_error(T, P.scheme, dt, &sm.k[0][comp], 3);
         const unsigned long long e1 = __shfl_sync(0xffffffffu, eb, 1), e2 = __shfl_sync(0xffffffffu, eb, 2);
         eb = max(eb, max(e1, e2));
         if (lane == 0) st_rec16(P.err + P.n_cta + k, (unsigned)eb, (unsigned)(eb >> 32), 0u, tag0 + 14);
@@ -229,8 +204,8 @@ __device__ __forceinline__ void run_owner64(const TryParams& P, Owner64& sm, con
         *P.epoch = tag0 / 16 + 1;
     }
     if (w != GW) return;
-    const double rn = fma(dt, fma(dt, row_sum64(T, kTryRowRB, &sm.k[0][comp], 3), T.t.cb * v), y);
-    const double vn = fma(dt, row_sum64(T, kTryRowVB, &sm.k[0][comp], 3), v);
+    double rn = y, vn = v;
+    solution(T, dt, &sm.k[0][comp], 3, rn, vn);
     bool accepted = true;
     if (P.adaptive) {
         unsigned acc = 0u;
@@ -251,7 +226,7 @@ __global__ void __launch_bounds__(kTry64Threads, 1) k_try64(const __grid_constan
 {
     __shared__ double si[2][3 * kTryMaxLarge], si_m[kTryMaxLarge];
     __shared__ double ly[3 * kTryMaxLarge], lv[3 * kTryMaxLarge];   // the large bodies' state at the start of the try
-    __shared__ Tab64 T;
+    __shared__ NyTableau T;
     __shared__ Owner64 own;
     __shared__ unsigned long long err_sm;
     __shared__ int dead, take;
@@ -299,8 +274,7 @@ __global__ void __launch_bounds__(kTry64Threads, 1) k_try64(const __grid_constan
     } else if (t >= main) {
         const int o = t - main;
         for (int k = o; k < (int)(sizeof(NyTableau) / 16); k += P.owners)
-            reinterpret_cast<uint4*>(&T.t)[k] = reinterpret_cast<const uint4*>(P.tab)[k];
-        for (int k = o; k < (int)(sizeof(T.a) / 8); k += P.owners) T.a[k] = P.tab64[k];
+            reinterpret_cast<uint4*>(&T)[k] = reinterpret_cast<const uint4*>(P.tab)[k];
         if (blockIdx.x == 0)
             for (int k = o; k < (int)(sizeof(DevSys) / 4); k += P.owners)
                 reinterpret_cast<unsigned*>(&own.sys)[k] = reinterpret_cast<const volatile unsigned*>(S)[k];
@@ -411,12 +385,12 @@ __global__ void __launch_bounds__(kTry64Threads, 1) k_try64(const __grid_constan
             }
             if (s + 1 < ns)
                 pos[((s + 1) & 1) * 3 * pad + e] =
-                    fma(dt * dt, row_sum64(T, s + 1, ks + e, n3), fma(T.t.c[s + 1] * dt, yv[e], yr[e]));
+                    fma(dt * dt, row_sum(T, s + 1, ks + e, n3), fma(T.c[s + 1] * dt, yv[e], yr[e]));
         }
         if (s == ns) break;
         if (s + 1 < ns)
             for (int e = tb; e < 3 * nl; e += P.bodies)
-                si[(s + 1) & 1][e] = s == 0 ? fma(T.t.c[1] * dt, lv[e], ly[e])
+                si[(s + 1) & 1][e] = s == 0 ? fma(T.c[1] * dt, lv[e], ly[e])
                                             : poll_rec(pos_records64(P, s + 1) + e, tag0 + 2 + s, S, &dead);
         // the last positions follow every CTA's clearing of the hash (n_stage > 3)
         if (s + 2 == ns && P.head) __threadfence();
@@ -424,17 +398,13 @@ __global__ void __launch_bounds__(kTry64Threads, 1) k_try64(const __grid_constan
     }
     if (P.adaptive) {
         unsigned long long eb = 0ull;
-        for (int e = tb; e < items; e += P.bodies) eb = max(eb, error64(T, P.scheme, dt, ks + e, n3));
+        for (int e = tb; e < items; e += P.bodies) eb = max(eb, component_error(T, P.scheme, dt, ks + e, n3));
         for (int m = 16; m > 0; m >>= 1) eb = max(eb, __shfl_xor_sync(0xffffffffu, eb, m));
         if ((tb & 31) == 0) atomicMax(&err_sm, eb);
         lanes_sync(3, P.bodies);
         if (tb == 0) st_rec16(P.err + blockIdx.x, (unsigned)err_sm, (unsigned)(err_sm >> 32), 0u, tag0 + 14);
     }
-    for (int e = tb; e < items; e += P.bodies) {
-        const double v = yv[e];
-        yr[e] = fma(dt, fma(dt, row_sum64(T, kTryRowRB, ks + e, n3), T.t.cb * v), yr[e]);
-        yv[e] = fma(dt, row_sum64(T, kTryRowVB, ks + e, n3), v);
-    }
+    for (int e = tb; e < items; e += P.bodies) solution(T, dt, ks + e, n3, yr[e], yv[e]);
     if (P.adaptive) {
         if (tb == 0) take = poll16(P.decision, tag0 + 15, S, &dead).x == 1u;
         lanes_sync(3, P.bodies);
