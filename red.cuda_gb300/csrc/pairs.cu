@@ -8,6 +8,17 @@ namespace {
 
 __device__ __forceinline__ float2 dup(float a) { return make_float2(a, a); }
 
+// x added to the double-single sums (h, l), two of them side by side in packed FP32:
+// Knuth's TwoSum as ds_add has it, differences as a - b = fma(b, -1, a).
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, dup(-1.f), a); }
+__device__ __forceinline__ void ds_add2(float2& h, float2& l, float2 x)
+{
+    const float2 s = __fadd2_rn(h, x);
+    const float2 t = sub2(s, h);
+    l = __fadd2_rn(l, __fadd2_rn(sub2(h, sub2(s, t)), sub2(x, t)));
+    h = s;
+}
+
 // One body j (h, l: its double-single position, h.w its mass) against the
 // thread's four sinks, held as two pairs: packed FP32, one instruction for two
 // pair terms.  With SYM the terms go both ways: (jx, jy, jz) += m_i d / |d|^3,
@@ -18,7 +29,10 @@ __device__ __forceinline__ void pair_step(float4 h, float4 l, const float2 (&nH)
                                           const float2 (&mi)[2], float2 (&a)[2][3], float& jx, float& jy, float& jz)
 {
     const float2 hx = dup(h.x), hy = dup(h.y), hz = dup(h.z), mj = dup(h.w);
-    float2 sx = make_float2(jx, 0.f), sy = make_float2(jy, 0.f), sz = make_float2(jz, 0.f);
+    // MIXED sums the four terms on the body before the running sum takes them
+    constexpr bool kApart = MODE == MODE_MIXED;
+    float2 sx = make_float2(kApart ? 0.f : jx, 0.f), sy = make_float2(kApart ? 0.f : jy, 0.f),
+           sz = make_float2(kApart ? 0.f : jz, 0.f);
 #pragma unroll
     for (int p = 0; p < 2; p++) {
         float2 dx = __fadd2_rn(hx, nH[p][0]), dy = __fadd2_rn(hy, nH[p][1]), dz = __fadd2_rn(hz, nH[p][2]);
@@ -44,9 +58,9 @@ __device__ __forceinline__ void pair_step(float4 h, float4 l, const float2 (&nH)
         }
     }
     if (SYM) {
-        jx = sx.x + sx.y;
-        jy = sy.x + sy.y;
-        jz = sz.x + sz.y;
+        jx = kApart ? jx + (sx.x + sx.y) : sx.x + sx.y;
+        jy = kApart ? jy + (sy.x + sy.y) : sy.x + sy.y;
+        jz = kApart ? jz + (sz.x + sz.y) : sz.x + sz.y;
     }
 }
 
@@ -59,19 +73,28 @@ struct PairSmem {
 
 // Lane l of a warp takes body (l + s) mod 32 of a group of 32 in step s, so the
 // 32 bodies are read without bank conflicts and each meets every sink of the warp
-// once; the running sum of a body moves one lane down per step.  FP32 sums of at
-// most 32 terms (two packed halves of 16) go into double-single ones: a body's
-// every 8 steps, a sink's every 32.
+// once; the running sum of a body moves one lane down per step.  Runs of FP32 sums go
+// into double-single ones: a body's every kRunJ steps (of four sinks), a sink's every kRun
+// (kRunOwn against its own block; with eight there the whole takes 1 % longer).
 //
-// Bound by the FP32 pipe (76 % busy): 22 operations a pair in MIXED and 16 in FP32
-// mode, where one-sided terms take 36 and 24; the other per-step work (two loads,
+// The runs of MIXED are as short as its accuracy needs: median relative error of the
+// accelerations of a field of protoplanets 1.3 % below the one-sided tiles' (16 terms to a
+// sum, in two halves), of a cube the same; with 32 terms to both sums, as FP32 mode
+// has them, 10 and 7 % above.  That costs 10 % (16384 bodies, four tries: 6.82 -> 7.49 ms).
+// In FP32 mode the rounding of the coordinates hides the sums': errors within 0.2 % of
+// the one-sided tiles' (rms) with the long runs, which are 10 % faster than runs of 16.
+//
+// Bound by the FP32 pipe (76 % busy with long runs): 22 operations a pair in MIXED and 16 in
+// FP32 mode, where one-sided terms take 36 and 24; the other per-step work (two loads,
 // three shuffles, three adds, the packed copies of the body) issues beside it.
-// 16384 bodies, adaptive RKF7(8) in MIXED: 2.74 -> 1.79 ms per try against the
-// one-sided tiles (1.70 with the packed collision filter); 65536 bodies, RK4 in FP32: 8.17 -> 5.58 ms.
+// 16384 bodies, adaptive RKF7(8) in MIXED: 2.74 -> 1.87 ms per try against the
+// one-sided tiles; 65536 bodies, RK4 in FP32: 8.17 -> 5.52 ms.
 template <int MODE>
 __global__ void __launch_bounds__(kTile, 4) k_pairs(const PairParams P)
 {
     __shared__ PairSmem sm;
+    constexpr int kRun = MODE == MODE_MIXED ? 8 : 32, kRunJ = 8;   // steps of a run: a sink's, a body's
+    constexpr int kRunOwn = MODE == MODE_MIXED ? 4 : 32;           // a sink's within its own block
     const PairJob job = P.jobs[blockIdx.x];
     pdl_wait();
     pdl_trigger();
@@ -115,16 +138,25 @@ __global__ void __launch_bounds__(kTile, 4) k_pairs(const PairParams P)
         if (sub + 1 < job.sub1) fetch(sub + 1);
         for (int g = 0; g < kTile; g += 32) {
             float2 a[2][3];
+            auto clear = [&]() {
 #pragma unroll
-            for (int p = 0; p < 2; p++)
+                for (int p = 0; p < 2; p++)
 #pragma unroll
-                for (int c = 0; c < 3; c++) a[p][c] = make_float2(0.f, 0.f);
+                    for (int c = 0; c < 3; c++) a[p][c] = make_float2(0.f, 0.f);
+            };
+            auto fold = [&]() {
+#pragma unroll
+                for (int p = 0; p < 2; p++)
+#pragma unroll
+                    for (int c = 0; c < 3; c++) ds_add2(acc_h[p][c], acc_l[p][c], a[p][c]);
+            };
             if (sym) {
 #pragma unroll 1
-                for (int s0 = 0; s0 < 32; s0 += 8) {
+                for (int s0 = 0; s0 < 32; s0 += kRunJ) {
                     float jx = 0.f, jy = 0.f, jz = 0.f;
+                    if (s0 % kRun == 0) clear();
 #pragma unroll
-                    for (int s = 0; s < 8; s++) {
+                    for (int s = 0; s < kRunJ; s++) {
                         if (s > 0) {
                             const int from = (lane + 1) & 31;
                             jx = __shfl_sync(0xffffffffu, jx, from);
@@ -134,7 +166,8 @@ __global__ void __launch_bounds__(kTile, 4) k_pairs(const PairParams P)
                         const int jj = g + ((lane + s0 + s) & 31);
                         pair_step<MODE, true>(sm.h[jj], MODE == MODE_MIXED ? sm.l[jj] : l, nH, nL, mi, a, jx, jy, jz);
                     }
-                    const int jj = g + ((lane + s0 + 7) & 31);
+                    if ((s0 + kRunJ) % kRun == 0) fold();
+                    const int jj = g + ((lane + s0 + kRunJ - 1) & 31);
                     const float v[3] = {jx, jy, jz};
 #pragma unroll
                     for (int c = 0; c < 3; c++) {
@@ -146,19 +179,17 @@ __global__ void __launch_bounds__(kTile, 4) k_pairs(const PairParams P)
                 }
             } else {
                 float jx = 0.f, jy = 0.f, jz = 0.f;
+#pragma unroll 1
+                for (int s0 = 0; s0 < 32; s0 += kRunOwn) {
+                    clear();
 #pragma unroll 4
-                for (int s = 0; s < 32; s++) {
-                    const int jj = g + ((lane + s) & 31);
-                    pair_step<MODE, false>(sm.h[jj], MODE == MODE_MIXED ? sm.l[jj] : l, nH, nL, mi, a, jx, jy, jz);
+                    for (int s = 0; s < kRunOwn; s++) {
+                        const int jj = g + ((lane + s0 + s) & 31);
+                        pair_step<MODE, false>(sm.h[jj], MODE == MODE_MIXED ? sm.l[jj] : l, nH, nL, mi, a, jx, jy, jz);
+                    }
+                    fold();
                 }
             }
-#pragma unroll
-            for (int p = 0; p < 2; p++)
-#pragma unroll
-                for (int c = 0; c < 3; c++) {
-                    ds_add(acc_h[p][c].x, acc_l[p][c].x, a[p][c].x);
-                    ds_add(acc_h[p][c].y, acc_l[p][c].y, a[p][c].y);
-                }
         }
         if (sym) {
             __syncthreads();
