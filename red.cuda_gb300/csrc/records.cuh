@@ -9,7 +9,11 @@ namespace redgb {
 
 namespace {
 
-// 16-byte records: three words and a tag, one 128-bit access each way.
+// 16-byte records: three words and a tag, one 128-bit access each way.  The compiler
+// keeps the load whole only if all four words are used: with x and the tag alone it made
+// two 32-bit loads of it, and a reader met the new tag beside the old x (one read in
+// 70 while the record changed).  So a record of three words is read for all three, and one of
+// two words or less goes through st_pair and poll_pair.
 __device__ __forceinline__ void st_rec16(uint4* p, unsigned x, unsigned y, unsigned z, unsigned tag)
 {
     asm volatile("{\n\t.reg .b128 q;\n\t.reg .b64 a, b;\n\tmov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\t"
@@ -45,6 +49,23 @@ __device__ __forceinline__ uint4 poll16(const uint4* p, unsigned tag, DevSys* S,
         if ((k & 63) == 63 && *dead) break;
     }
     return missing_record(S, dead);
+}
+
+// A record of two words.  The third one is their sum modulo 2 with the tag, so that all
+// four are needed and words of two records do not pass for one.
+__device__ __forceinline__ void st_pair(uint4* p, unsigned lo, unsigned hi, unsigned tag)
+{
+    st_rec16(p, lo, hi, lo ^ hi ^ tag, tag);
+}
+__device__ __forceinline__ uint2 poll_pair(const uint4* p, unsigned tag, DevSys* S, volatile int* dead)
+{
+    for (int k = 0; k < kTryPollLimit; k++) {
+        const uint4 v = ld_rec16(p);
+        if (v.w == tag && (v.x ^ v.y ^ v.z) == tag) return make_uint2(v.x, v.y);
+        if ((k & 63) == 63 && *dead) break;
+    }
+    const uint4 v = missing_record(S, dead);
+    return make_uint2(v.x, v.y);
 }
 
 // A barrier of some warps.  bar.sync is the aligned form: all lanes of a warp must

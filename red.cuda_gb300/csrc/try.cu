@@ -252,13 +252,13 @@ __device__ __forceinline__ void run_owner(const TryParams& P, OwnerSmem& sm, con
         unsigned long long eb = component_error(T, P.scheme, dt, &sm.k[0][comp], 3);
         const unsigned long long e1 = __shfl_sync(0xffffffffu, eb, 1), e2 = __shfl_sync(0xffffffffu, eb, 2);
         eb = max(eb, max(e1, e2));
-        if (lane == 0) st_rec16(P.err + P.n_cta + k, (unsigned)eb, (unsigned)(eb >> 32), 0u, tag0 + 14);
+        if (lane == 0) st_pair(P.err + P.n_cta + k, (unsigned)eb, (unsigned)(eb >> 32), tag0 + 14);
     }
     if (P.adaptive && k == 0) {
         if (w < GW) {
             unsigned long long m = 0ull;
             for (int j = o; j < P.n_cta + nl; j += 32 * GW) {
-                const uint4 q = poll16(P.err + j, tag0 + 14, S, dead);
+                const uint2 q = poll_pair(P.err + j, tag0 + 14, S, dead);
                 m = max(m, ((unsigned long long)q.y << 32) | q.x);
             }
             atomicMax(&sm.err, m);
@@ -267,7 +267,7 @@ __device__ __forceinline__ void run_owner(const TryParams& P, OwnerSmem& sm, con
         if (w == 0 && lane == 0) {
             // accepted or not: control_system's test, before the rest of the step control
             const double max_err = fabs(P.ctl.lambda * dt * __longlong_as_double((long long)sm.err));
-            st_rec16(P.decision, max_err <= P.ctl.tolerance ? 1u : 0u, 0u, 0u, tag0 + 15);
+            st_pair(P.decision, max_err <= P.ctl.tolerance ? 1u : 0u, 0u, tag0 + 15);
         }
     }
     if (k == 0 && o == 0) {
@@ -281,7 +281,7 @@ __device__ __forceinline__ void run_owner(const TryParams& P, OwnerSmem& sm, con
     bool accepted = true;
     if (P.adaptive) {
         unsigned acc = 0u;
-        if (lane == 0) acc = poll16(P.decision, tag0 + 15, S, dead).x;
+        if (lane == 0) acc = poll_pair(P.decision, tag0 + 15, S, dead).x;
         accepted = __shfl_sync(0xffffffffu, acc, 0) == 1u;
     }
     if (lane < 3 && accepted) {
@@ -574,13 +574,13 @@ __global__ void __launch_bounds__(try_max_threads(DRAG)) k_try(const __grid_cons
         for (int m = 16; m > 0; m >>= 1) eb = max(eb, __shfl_xor_sync(0xffffffffu, eb, m));
         if ((tb & 31) == 0) atomicMax(&err_sm, eb);
         group_sync(3, P.bodies);
-        if (tb == 0) st_rec16(P.err + blockIdx.x, (unsigned)err_sm, (unsigned)(err_sm >> 32), 0u, tag0 + 14);
+        if (tb == 0) st_pair(P.err + blockIdx.x, (unsigned)err_sm, (unsigned)(err_sm >> 32), tag0 + 14);
     }
     for (int x = tb; x < items; x += P.bodies)
 #pragma unroll
         for (int c = 0; c < N; c++) solution(T, dt, ks + N * x + c, n3, yr[N * x + c], yv[N * x + c]);
     if (P.adaptive) {
-        if (tb == 0) take = poll16(P.decision, tag0 + 15, S, &dead).x == 1u;
+        if (tb == 0) take = poll_pair(P.decision, tag0 + 15, S, &dead).x == 1u;
         group_sync(3, P.bodies);
         if (!take) return;
     } else {

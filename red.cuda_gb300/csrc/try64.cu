@@ -16,11 +16,11 @@ __device__ __forceinline__ void lanes_sync(int id, int threads)
 __device__ __forceinline__ void st_rec(uint4* p, double v, unsigned tag)
 {
     const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-    st_rec16(p, (unsigned)b, (unsigned)(b >> 32), 0u, tag);
+    st_pair(p, (unsigned)b, (unsigned)(b >> 32), tag);
 }
 __device__ __forceinline__ double poll_rec(const uint4* p, unsigned tag, DevSys* S, volatile int* dead)
 {
-    const uint4 v = poll16(p, tag, S, dead);
+    const uint2 v = poll_pair(p, tag, S, dead);
     return __longlong_as_double((long long)(((unsigned long long)v.y << 32) | v.x));
 }
 
@@ -181,13 +181,13 @@ __device__ __forceinline__ void run_owner64(const TryParams& P, Owner64& sm, con
         unsigned long long eb = component_error(T, P.scheme, dt, &sm.k[0][comp], 3);
         const unsigned long long e1 = __shfl_sync(0xffffffffu, eb, 1), e2 = __shfl_sync(0xffffffffu, eb, 2);
         eb = max(eb, max(e1, e2));
-        if (lane == 0) st_rec16(P.err + P.n_cta + k, (unsigned)eb, (unsigned)(eb >> 32), 0u, tag0 + 14);
+        if (lane == 0) st_pair(P.err + P.n_cta + k, (unsigned)eb, (unsigned)(eb >> 32), tag0 + 14);
     }
     if (P.adaptive && k == 0) {
         if (w < GW) {
             unsigned long long m = 0ull;
             for (int j = o; j < P.n_cta + nl; j += 32 * GW) {
-                const uint4 q = poll16(P.err + j, tag0 + 14, S, dead);
+                const uint2 q = poll_pair(P.err + j, tag0 + 14, S, dead);
                 m = max(m, ((unsigned long long)q.y << 32) | q.x);
             }
             atomicMax(&sm.err, m);
@@ -195,7 +195,7 @@ __device__ __forceinline__ void run_owner64(const TryParams& P, Owner64& sm, con
         lanes_sync(2, W);
         if (w == 0 && lane == 0) {
             const double max_err = fabs(P.ctl.lambda * dt * __longlong_as_double((long long)sm.err));
-            st_rec16(P.decision, max_err <= P.ctl.tolerance ? 1u : 0u, 0u, 0u, tag0 + 15);
+            st_pair(P.decision, max_err <= P.ctl.tolerance ? 1u : 0u, 0u, tag0 + 15);
         }
     }
     if (k == 0 && o == 0) {
@@ -209,7 +209,7 @@ __device__ __forceinline__ void run_owner64(const TryParams& P, Owner64& sm, con
     bool accepted = true;
     if (P.adaptive) {
         unsigned acc = 0u;
-        if (lane == 0) acc = poll16(P.decision, tag0 + 15, S, dead).x;
+        if (lane == 0) acc = poll_pair(P.decision, tag0 + 15, S, dead).x;
         accepted = __shfl_sync(0xffffffffu, acc, 0) == 1u;
     }
     if (lane < 3 && accepted) {
@@ -402,11 +402,11 @@ __global__ void __launch_bounds__(kTry64Threads, 1) k_try64(const __grid_constan
         for (int m = 16; m > 0; m >>= 1) eb = max(eb, __shfl_xor_sync(0xffffffffu, eb, m));
         if ((tb & 31) == 0) atomicMax(&err_sm, eb);
         lanes_sync(3, P.bodies);
-        if (tb == 0) st_rec16(P.err + blockIdx.x, (unsigned)err_sm, (unsigned)(err_sm >> 32), 0u, tag0 + 14);
+        if (tb == 0) st_pair(P.err + blockIdx.x, (unsigned)err_sm, (unsigned)(err_sm >> 32), tag0 + 14);
     }
     for (int e = tb; e < items; e += P.bodies) solution(T, dt, ks + e, n3, yr[e], yv[e]);
     if (P.adaptive) {
-        if (tb == 0) take = poll16(P.decision, tag0 + 15, S, &dead).x == 1u;
+        if (tb == 0) take = poll_pair(P.decision, tag0 + 15, S, &dead).x == 1u;
         lanes_sync(3, P.bodies);
         if (!take) return;
     } else {
