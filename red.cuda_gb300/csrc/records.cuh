@@ -32,20 +32,27 @@ __device__ __forceinline__ uint4 ld_rec16(const uint4* p)
     return v;
 }
 
-// Waits for the record with this tag.  A missing one stops the system; *dead
-// (shared memory) then ends the CTA's other waits.
+// A status that no earlier one is overwritten by.
+__device__ __forceinline__ void set_status(DevSys* S, int status) { atomicCAS(&S->status, 0, status); }
+
+// Waits for the record with this tag.  A missing one, or one whose writer has given
+// the try up, stops the system; *dead (shared memory) then ends the CTA's other waits
+// and marks its records (tag_of).
 __device__ __noinline__ uint4 missing_record(DevSys* S, volatile int* dead)
 {
     *dead = 1;
-    S->status = 4;   // RED_ERR_TIMEOUT
+    set_status(S, 4);   // RED_ERR_TIMEOUT
     S->halted = 1;
     return make_uint4(0x7fc00000u, 0x7fc00000u, 0x7fc00000u, 0u);
 }
+// A record of the try of this tag whose writer has given it up, at whatever stage.
+__device__ __forceinline__ bool given_up(unsigned got, unsigned tag) { return ((got ^ tag) & ~15u) == kTryAbort; }
 __device__ __forceinline__ uint4 poll16(const uint4* p, unsigned tag, DevSys* S, volatile int* dead)
 {
     for (int k = 0; k < kTryPollLimit; k++) {
         const uint4 v = ld_rec16(p);
         if (v.w == tag) return v;
+        if (given_up(v.w, tag)) break;
         if ((k & 63) == 63 && *dead) break;
     }
     return missing_record(S, dead);
@@ -62,10 +69,16 @@ __device__ __forceinline__ uint2 poll_pair(const uint4* p, unsigned tag, DevSys*
     for (int k = 0; k < kTryPollLimit; k++) {
         const uint4 v = ld_rec16(p);
         if (v.w == tag && (v.x ^ v.y ^ v.z) == tag) return make_uint2(v.x, v.y);
+        if (given_up(v.w, tag)) break;
         if ((k & 63) == 63 && *dead) break;
     }
     const uint4 v = missing_record(S, dead);
     return make_uint2(v.x, v.y);
+}
+
+__device__ __forceinline__ unsigned tag_of(unsigned tag, const volatile int* dead)
+{
+    return *dead ? tag ^ kTryAbort : tag;
 }
 
 // A barrier of some warps.  bar.sync is the aligned form: all lanes of a warp must
@@ -135,7 +148,7 @@ __device__ __forceinline__ void store_control(DevSys* S, const DevSys& C)
     S->active = C.active;
     S->quota = C.quota;
     S->err_last = C.err_last;
-    if (C.status) S->status = C.status;   // else as it is: other CTAs may set these
+    if (C.status) set_status(S, C.status);   // other CTAs may set these
     if (C.halted) S->halted = C.halted;
 }
 

@@ -240,7 +240,7 @@ __device__ __forceinline__ void run_owner(const TryParams& P, OwnerSmem& sm, con
                 if (lane < 2 * kTryCopies) {   // lanes 2 c, 2 c + 1: the two words of copy c
                     uint4* rec = P.pos + ((size_t)(((s + 2) & 3) * kTryCopies + (lane >> 1)) * nl + k) * 2 + (lane & 1);
                     st_rec16(rec, __float_as_uint(lane & 1 ? l0 : h0), __float_as_uint(lane & 1 ? l1 : h1),
-                             __float_as_uint(lane & 1 ? l2 : h2), tag0 + 3 + s);
+                             __float_as_uint(lane & 1 ? l2 : h2), tag_of(tag0 + 3 + s, dead));
                 }
             }
             if (lane < 3) sm.k[s][lane] = a_k;
@@ -248,16 +248,20 @@ __device__ __forceinline__ void run_owner(const TryParams& P, OwnerSmem& sm, con
         }
     }
     // the solution, the error, the decision: the last warp; CTA 0's others gather the errors
-    if (P.adaptive && w == GW) {
-        unsigned long long eb = component_error(T, P.scheme, dt, &sm.k[0][comp], 3);
-        const unsigned long long e1 = __shfl_sync(0xffffffffu, eb, 1), e2 = __shfl_sync(0xffffffffu, eb, 2);
-        eb = max(eb, max(e1, e2));
-        if (lane == 0) st_pair(P.err + P.n_cta + k, (unsigned)eb, (unsigned)(eb >> 32), tag0 + 14);
+    if (w == GW) {
+        unsigned long long eb = 0ull;
+        if (P.adaptive) {
+            eb = component_error(T, P.scheme, dt, &sm.k[0][comp], 3);
+            const unsigned long long e1 = __shfl_sync(0xffffffffu, eb, 1), e2 = __shfl_sync(0xffffffffu, eb, 2);
+            eb = max(eb, max(e1, e2));
+        }
+        if (lane == 0) st_pair(P.err + P.n_cta + k, (unsigned)eb, (unsigned)(eb >> 32), tag_of(tag0 + 14, dead));
     }
-    if (P.adaptive && k == 0) {
+    if (k == 0) {
         if (w < GW) {
+            // in fixed steps the owners' records alone: the last partial sums told of the CTAs
             unsigned long long m = 0ull;
-            for (int j = o; j < P.n_cta + nl; j += 32 * GW) {
+            for (int j = (P.adaptive ? 0 : P.n_cta) + o; j < P.n_cta + nl; j += 32 * GW) {
                 const uint2 q = poll_pair(P.err + j, tag0 + 14, S, dead);
                 m = max(m, ((unsigned long long)q.y << 32) | q.x);
             }
@@ -267,27 +271,28 @@ __device__ __forceinline__ void run_owner(const TryParams& P, OwnerSmem& sm, con
         if (w == 0 && lane == 0) {
             // accepted or not: control_system's test, before the rest of the step control
             const double max_err = fabs(P.ctl.lambda * dt * __longlong_as_double((long long)sm.err));
-            st_pair(P.decision, max_err <= P.ctl.tolerance ? 1u : 0u, 0u, tag0 + 15);
+            const bool heard = !*dead;
+            const bool take = heard && (!P.adaptive || max_err <= P.ctl.tolerance);
+            st_pair(P.decision, take ? 1u : 0u, 0u, tag_of(tag0 + 15, dead));
+            if (heard) {
+                control_of(P.ctl, sm.sys, P.adaptive ? sm.err : 0ull);
+                store_control(S, sm.sys);
+            } else {
+                S->accepted = 0;
+            }
+            *P.epoch = tag0 / 16 + 1;
         }
-    }
-    if (k == 0 && o == 0) {
-        control_of(P.ctl, sm.sys, P.adaptive ? sm.err : 0ull);
-        store_control(S, sm.sys);
-        *P.epoch = tag0 / 16 + 1;
     }
     if (w != GW) return;
     double rn = y, vn = v;
     solution(T, dt, &sm.k[0][comp], 3, rn, vn);
-    bool accepted = true;
-    if (P.adaptive) {
-        unsigned acc = 0u;
-        if (lane == 0) acc = poll_pair(P.decision, tag0 + 15, S, dead).x;
-        accepted = __shfl_sync(0xffffffffu, acc, 0) == 1u;
-    }
-    if (lane < 3 && accepted) {
+    unsigned take = 0u;
+    if (lane == 0) take = poll_pair(P.decision, tag0 + 15, S, dead).x;
+    take = __shfl_sync(0xffffffffu, take, 0);
+    if (lane < 3 && take == 1u) {
         P.y_r[3 * body + lane] = rn;
         P.y_v[3 * body + lane] = vn;
-        if (not_finite(rn) || not_finite(vn)) S->status = 5;   // RED_ERR_NONFINITE
+        if (not_finite(rn) || not_finite(vn)) set_status(S, 5);   // RED_ERR_NONFINITE
         write_pos_c(P.pos_hi, P.pos_lo, body, lane, rn);
     }
 }
@@ -462,7 +467,7 @@ __global__ void __launch_bounds__(try_max_threads(DRAG)) k_try(const __grid_cons
             start.runs = V->active && !V->halted && V->quota != 0;
             start.dt = dt;
             start.t = ts;
-            start.tag = ep * 16u;
+            start.tag = try_tag(ep);
             dead = 0;
             err_sm = 0ull;
         }
@@ -485,7 +490,8 @@ __global__ void __launch_bounds__(try_max_threads(DRAG)) k_try(const __grid_cons
         const int share = np > 1 ? t / pad : 0, body = np > 1 ? t % pad : t;
         for (int s = 0; s < ns; s++) {
             const int q = s & 1;
-            pull_large<MODE>(P, s, t, pad, bhi + q * pad, blo + q * pad, si_hi[q], si_lo[q], tag0 + 1 + s);
+            pull_large<MODE>(P, s, t, pad, bhi + q * pad, blo + q * pad, si_hi[q], si_lo[q],
+                             tag_of(tag0 + 1 + s, &dead));
             pull_small<MODE>(nl, P.n_star, P.pull, share, body, cnt, pad, np, bhi + q * pad, blo + q * pad, si_hi[q], si_lo[q], star_m,
                              parts + (size_t)q * np * 3 * pad);
             if (s == 0 && P.head_n > 0) __threadfence();   // the cleared hash before the later records
@@ -503,7 +509,7 @@ __global__ void __launch_bounds__(try_max_threads(DRAG)) k_try(const __grid_cons
     for (int s = 0; s <= ns; s++) {
         if (DRAG && s < ns)
             pull_large<MODE>(P, s, t, pad, bhi + (s & 1) * pad, blo + (s & 1) * pad, si_hi[s & 1], si_lo[s & 1],
-                             tag0 + 1 + s);
+                             tag_of(tag0 + 1 + s, &dead));
         double decr = 0.0;
         if (DRAG && s > 0) decr = gas_reduction_factor<false>(P.gas, tsys + stage_c(P.scheme, s - 1) * dt);
         for (int x = tb; x < items; x += P.bodies) {
@@ -574,18 +580,15 @@ __global__ void __launch_bounds__(try_max_threads(DRAG)) k_try(const __grid_cons
         for (int m = 16; m > 0; m >>= 1) eb = max(eb, __shfl_xor_sync(0xffffffffu, eb, m));
         if ((tb & 31) == 0) atomicMax(&err_sm, eb);
         group_sync(3, P.bodies);
-        if (tb == 0) st_pair(P.err + blockIdx.x, (unsigned)err_sm, (unsigned)(err_sm >> 32), tag0 + 14);
+        if (tb == 0)
+            st_pair(P.err + blockIdx.x, (unsigned)err_sm, (unsigned)(err_sm >> 32), tag_of(tag0 + 14, &dead));
     }
     for (int x = tb; x < items; x += P.bodies)
 #pragma unroll
         for (int c = 0; c < N; c++) solution(T, dt, ks + N * x + c, n3, yr[N * x + c], yv[N * x + c]);
-    if (P.adaptive) {
-        if (tb == 0) take = poll_pair(P.decision, tag0 + 15, S, &dead).x == 1u;
-        group_sync(3, P.bodies);
-        if (!take) return;
-    } else {
-        group_sync(3, P.bodies);
-    }
+    if (tb == 0) take = poll_pair(P.decision, tag0 + 15, S, &dead).x == 1u;
+    group_sync(3, P.bodies);
+    if (!take) return;
     int* cell = reinterpret_cast<int*>(parts);   // the pull group has left it
     bool bad = false;
     for (int e = tb; e < 3 * cnt; e += P.bodies) {
@@ -596,7 +599,7 @@ __global__ void __launch_bounds__(try_max_threads(DRAG)) k_try(const __grid_cons
         write_pos_c(P.pos_hi, P.pos_lo, first + e / 3, e % 3, r);
         if (grid.enabled) cell[e] = cell_coord(r, grid.inv_h);
     }
-    if (bad) S->status = 5;   // RED_ERR_NONFINITE
+    if (bad) set_status(S, 5);   // RED_ERR_NONFINITE
     if (!grid.enabled) return;   // uniform
     group_sync(3, P.bodies);
     for (int b = tb; b < cnt; b += P.bodies) {
@@ -954,7 +957,7 @@ __global__ void __launch_bounds__(kTeamPull + kTeamBody + kTeamOwners, 1) k_team
             write_pos_c(P.pos_hi, P.pos_lo, si.off + k, lane, y);
         }
     }
-    if (bad) S->status = 5;   // RED_ERR_NONFINITE
+    if (bad) set_status(S, 5);   // RED_ERR_NONFINITE
     if (!grid.enabled) return;   // uniform
     __syncthreads();
     const int* cell = reinterpret_cast<const int*>(parts);

@@ -42,10 +42,15 @@
 // again two stages later, when it has positions that the slot's reader formed
 // from it.  The positions take four sets: the group that sums body j's partials
 // can be three stages ahead of the group of body k, but not four, since the
-// partials of a stage wait for k's positions.  Every wait is bounded: after kTryPollLimit reads a
-// record counts as missing, the system's status becomes RED_ERR_TIMEOUT, the
-// system halts and no further wait is entered.  The launch is cooperative: all
-// its CTAs are resident together.
+// partials of a stage wait for k's positions.
+//
+// Every wait is bounded.  After kTryPollLimit reads a record counts as missing: the
+// system's status becomes RED_ERR_TIMEOUT and it halts, the CTA's other waits end at
+// once, and its own records carry kTryAbort, which ends the waits for them too.  No CTA
+// writes its solution before the first one, which hears of every CTA's and every owner's
+// try, has decided (in fixed steps too), and it takes no step then: state, time and
+// counters stay as they were.  (In fixed steps the decision costs 1.6 us of a try, 2053 bodies.)  The launch is
+// cooperative: all its CTAs are resident together.
 #pragma once
 #include "common.cuh"
 #include "control.cuh"
@@ -56,7 +61,13 @@ constexpr int kTryMaxOwners = 192;     // threads of the owner group, at most
 constexpr int kTryMaxLarge = 64;       // large bodies of a system on this path
 constexpr int kTryMaxStars = 4;
 constexpr int kTryCopies = 8;          // of the position records: 1/8 of the CTAs wait on each
-constexpr int kTryPollLimit = 1 << 20;
+#ifndef REDGB_TRY_POLL_LIMIT
+#define REDGB_TRY_POLL_LIMIT (1 << 20)     // about a second
+#endif
+constexpr int kTryPollLimit = REDGB_TRY_POLL_LIMIT;
+constexpr unsigned kTryAbort = 0x80000000u;   // in a record's tag: its writer has given the try up
+// The tags of a try follow this one; below kTryAbort.
+__host__ __device__ constexpr unsigned try_tag(unsigned epoch) { return (epoch & 0x07ffffffu) * 16u; }
 
 // Nystroem form of a scheme: its rows over the accelerations, nonzero terms only,
 // ascending stages.  Row s: the positions of stage s (dt^2 sum a K); kTryRowV + s:

@@ -171,22 +171,26 @@ __device__ __forceinline__ void run_owner64(const TryParams& P, Owner64& sm, con
                 const double px = __shfl_sync(0xffffffffu, x, lane % 3);
                 if (lane < 3 * kTryCopies)   // lanes 3 c .. 3 c + 2: copy c
                     st_rec(P.pos + ((size_t)(((s + 2) & 3) * kTryCopies + lane / 3) * nl + k) * 3 + lane % 3, px,
-                           tag0 + 3 + s);
+                           tag_of(tag0 + 3 + s, dead));
             }
             if (lane < 3) sm.k[s][lane] = g;
             __syncwarp();
         }
     }
-    if (P.adaptive && w == GW) {
-        unsigned long long eb = component_error(T, P.scheme, dt, &sm.k[0][comp], 3);
-        const unsigned long long e1 = __shfl_sync(0xffffffffu, eb, 1), e2 = __shfl_sync(0xffffffffu, eb, 2);
-        eb = max(eb, max(e1, e2));
-        if (lane == 0) st_pair(P.err + P.n_cta + k, (unsigned)eb, (unsigned)(eb >> 32), tag0 + 14);
+    if (w == GW) {
+        unsigned long long eb = 0ull;
+        if (P.adaptive) {
+            eb = component_error(T, P.scheme, dt, &sm.k[0][comp], 3);
+            const unsigned long long e1 = __shfl_sync(0xffffffffu, eb, 1), e2 = __shfl_sync(0xffffffffu, eb, 2);
+            eb = max(eb, max(e1, e2));
+        }
+        if (lane == 0) st_pair(P.err + P.n_cta + k, (unsigned)eb, (unsigned)(eb >> 32), tag_of(tag0 + 14, dead));
     }
-    if (P.adaptive && k == 0) {
+    if (k == 0) {
         if (w < GW) {
+            // in fixed steps the owners' records alone: the last partial sums told of the CTAs
             unsigned long long m = 0ull;
-            for (int j = o; j < P.n_cta + nl; j += 32 * GW) {
+            for (int j = (P.adaptive ? 0 : P.n_cta) + o; j < P.n_cta + nl; j += 32 * GW) {
                 const uint2 q = poll_pair(P.err + j, tag0 + 14, S, dead);
                 m = max(m, ((unsigned long long)q.y << 32) | q.x);
             }
@@ -194,28 +198,30 @@ __device__ __forceinline__ void run_owner64(const TryParams& P, Owner64& sm, con
         }
         lanes_sync(2, W);
         if (w == 0 && lane == 0) {
+            // accepted or not: control_system's test, before the rest of the step control
             const double max_err = fabs(P.ctl.lambda * dt * __longlong_as_double((long long)sm.err));
-            st_pair(P.decision, max_err <= P.ctl.tolerance ? 1u : 0u, 0u, tag0 + 15);
+            const bool heard = !*dead;
+            const bool take = heard && (!P.adaptive || max_err <= P.ctl.tolerance);
+            st_pair(P.decision, take ? 1u : 0u, 0u, tag_of(tag0 + 15, dead));
+            if (heard) {
+                control_of(P.ctl, sm.sys, P.adaptive ? sm.err : 0ull);
+                store_control(S, sm.sys);
+            } else {
+                S->accepted = 0;
+            }
+            *P.epoch = tag0 / 16 + 1;
         }
-    }
-    if (k == 0 && o == 0) {
-        control_of(P.ctl, sm.sys, P.adaptive ? sm.err : 0ull);
-        store_control(S, sm.sys);
-        *P.epoch = tag0 / 16 + 1;
     }
     if (w != GW) return;
     double rn = y, vn = v;
     solution(T, dt, &sm.k[0][comp], 3, rn, vn);
-    bool accepted = true;
-    if (P.adaptive) {
-        unsigned acc = 0u;
-        if (lane == 0) acc = poll_pair(P.decision, tag0 + 15, S, dead).x;
-        accepted = __shfl_sync(0xffffffffu, acc, 0) == 1u;
-    }
-    if (lane < 3 && accepted) {
+    unsigned take = 0u;
+    if (lane == 0) take = poll_pair(P.decision, tag0 + 15, S, dead).x;
+    take = __shfl_sync(0xffffffffu, take, 0);
+    if (lane < 3 && take == 1u) {
         P.y_r[3 * body + lane] = rn;
         P.y_v[3 * body + lane] = vn;
-        if (not_finite(rn) || not_finite(vn)) S->status = 5;   // RED_ERR_NONFINITE
+        if (not_finite(rn) || not_finite(vn)) set_status(S, 5);   // RED_ERR_NONFINITE
         write_pos_c(P.pos_hi, P.pos_lo, body, lane, rn);
     }
 }
@@ -284,7 +290,7 @@ __global__ void __launch_bounds__(kTry64Threads, 1) k_try64(const __grid_constan
             const unsigned ep = *(volatile unsigned*)P.epoch;
             start.runs = V->active && !V->halted && V->quota != 0;
             start.dt = dt;
-            start.tag = ep * 16u;
+            start.tag = try_tag(ep);
             dead = 0;
             err_sm = 0ull;
         }
@@ -356,6 +362,7 @@ __global__ void __launch_bounds__(kTry64Threads, 1) k_try64(const __grid_constan
                 }
             }
             lanes_sync(4, P.pull);
+            const unsigned tag = tag_of(tag0 + 1 + s, &dead);
             for (int e = t; e < 3 * nl; e += P.pull) {
                 const double* o = wp + e / 3 * bw * 3 + e % 3;
                 double a0 = 0.0, a1 = 0.0;
@@ -363,7 +370,7 @@ __global__ void __launch_bounds__(kTry64Threads, 1) k_try64(const __grid_constan
                     a0 += o[3 * u];
                     if (u + 1 < bw) a1 += o[3 * u + 3];
                 }
-                st_rec(P.part + ((size_t)(q * nl + e / 3) * P.n_cta + blockIdx.x) * 3 + e % 3, a0 + a1, tag0 + 1 + s);
+                st_rec(P.part + ((size_t)(q * nl + e / 3) * P.n_cta + blockIdx.x) * 3 + e % 3, a0 + a1, tag);
             }
             if (s == 0 && P.head_n > 0) __threadfence();   // the cleared hash before the later records
             lanes_sync(1, main);   // also before wp is written again
@@ -402,16 +409,13 @@ __global__ void __launch_bounds__(kTry64Threads, 1) k_try64(const __grid_constan
         for (int m = 16; m > 0; m >>= 1) eb = max(eb, __shfl_xor_sync(0xffffffffu, eb, m));
         if ((tb & 31) == 0) atomicMax(&err_sm, eb);
         lanes_sync(3, P.bodies);
-        if (tb == 0) st_pair(P.err + blockIdx.x, (unsigned)err_sm, (unsigned)(err_sm >> 32), tag0 + 14);
+        if (tb == 0)
+            st_pair(P.err + blockIdx.x, (unsigned)err_sm, (unsigned)(err_sm >> 32), tag_of(tag0 + 14, &dead));
     }
     for (int e = tb; e < items; e += P.bodies) solution(T, dt, ks + e, n3, yr[e], yv[e]);
-    if (P.adaptive) {
-        if (tb == 0) take = poll_pair(P.decision, tag0 + 15, S, &dead).x == 1u;
-        lanes_sync(3, P.bodies);
-        if (!take) return;
-    } else {
-        lanes_sync(3, P.bodies);
-    }
+    if (tb == 0) take = poll_pair(P.decision, tag0 + 15, S, &dead).x == 1u;
+    lanes_sync(3, P.bodies);
+    if (!take) return;
     int* cell = reinterpret_cast<int*>(parts);   // the pull group has left it
     bool bad = false;
     for (int e = tb; e < items; e += P.bodies) {
@@ -422,7 +426,7 @@ __global__ void __launch_bounds__(kTry64Threads, 1) k_try64(const __grid_constan
         write_pos_c(P.pos_hi, P.pos_lo, first + e / 3, e % 3, r);
         if (grid.enabled) cell[e] = cell_coord(r, grid.inv_h);
     }
-    if (bad) S->status = 5;   // RED_ERR_NONFINITE
+    if (bad) set_status(S, 5);   // RED_ERR_NONFINITE
     if (!grid.enabled) return;   // uniform
     lanes_sync(3, P.bodies);
     for (int b = tb; b < cnt; b += P.bodies) {
