@@ -157,6 +157,7 @@ __device__ __forceinline__ void run_owner(const TryParams& P, OwnerSmem& sm, con
             }
             const float2 part = reduce_scatter(a, lane, 32);
             if (lane < 3) sm.red[s & 1][w][lane] = part;
+            if (k == 0 && (s == 2 || s == 3) && P.head_n > 0) __threadfence();
             group_sync(2, W);   // two sets of `red`: the last warp reads one while the next is formed
         }
     }
@@ -494,7 +495,7 @@ __global__ void __launch_bounds__(try_max_threads(DRAG)) k_try(const __grid_cons
                              tag_of(tag0 + 1 + s, &dead));
             pull_small<MODE>(nl, P.n_star, P.pull, share, body, cnt, pad, np, bhi + q * pad, blo + q * pad, si_hi[q], si_lo[q], star_m,
                              parts + (size_t)q * np * 3 * pad);
-            if (s == 0 && P.head_n > 0) __threadfence();   // the cleared hash before the later records
+            if (s == 1 && P.head_n > 0) __threadfence();   // the cleared hash before the later records
             group_sync(1, main);
         }
         return;
@@ -565,9 +566,8 @@ __global__ void __launch_bounds__(try_max_threads(DRAG)) k_try(const __grid_cons
                 f[1] = __uint_as_float(v.y);
                 f[2] = __uint_as_float(v.z);
             }
-            // the last positions follow every CTA's clearing of the hash (n_stage > 3)
-            if (s + 2 == ns && P.head) __threadfence();
         }
+        if (DRAG && s == 1 && P.head_n > 0) __threadfence();   // these threads write partial sums too
         group_sync(1, main);
     }
 
@@ -586,7 +586,10 @@ __global__ void __launch_bounds__(try_max_threads(DRAG)) k_try(const __grid_cons
     for (int x = tb; x < items; x += P.bodies)
 #pragma unroll
         for (int c = 0; c < N; c++) solution(T, dt, ks + N * x + c, n3, yr[N * x + c], yv[N * x + c]);
-    if (tb == 0) take = poll_pair(P.decision, tag0 + 15, S, &dead).x == 1u;
+    if (tb == 0) {
+        take = poll_pair(P.decision, tag0 + 15, S, &dead).x == 1u;
+        if (P.head_n > 0) __threadfence();
+    }
     group_sync(3, P.bodies);
     if (!take) return;
     int* cell = reinterpret_cast<int*>(parts);   // the pull group has left it

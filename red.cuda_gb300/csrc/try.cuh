@@ -44,6 +44,12 @@
 // can be three stages ahead of the group of body k, but not four, since the
 // partials of a stage wait for k's positions.
 //
+// The cleared hash of the collision check precedes every insertion by a chain of fences
+// and records: a CTA's clearing, its barrier, a fence in each thread that writes its partial
+// sums (stage 1), the sums of stage 2; in the first CTA a fence after reading them, its
+// barrier, a fence in the thread that decides (stage 3), the decision; a fence after reading
+// that, a barrier, the insertions.  Schemes of one or two stages have the hash cleared before.
+//
 // Every wait is bounded.  After kTryPollLimit reads a record counts as missing: the
 // system's status becomes RED_ERR_TIMEOUT and it halts, the CTA's other waits end at
 // once, and its own records carry kTryAbort, which ends the waits for them too.  No CTA

@@ -117,6 +117,7 @@ __device__ __forceinline__ void run_owner64(const TryParams& P, Owner64& sm, con
             }
             const double part = warp_sum3(x, y, z, lane);
             if (lane < 3) sm.red[s & 1][w][lane] = part;
+            if (k == 0 && (s == 2 || s == 3) && P.head_n > 0) __threadfence();
             lanes_sync(2, W);   // two sets of `red`: the last warp reads one while the next is formed
         }
     }
@@ -372,7 +373,7 @@ __global__ void __launch_bounds__(kTry64Threads, 1) k_try64(const __grid_constan
                 }
                 st_rec(P.part + ((size_t)(q * nl + e / 3) * P.n_cta + blockIdx.x) * 3 + e % 3, a0 + a1, tag);
             }
-            if (s == 0 && P.head_n > 0) __threadfence();   // the cleared hash before the later records
+            if (s == 1 && P.head_n > 0) __threadfence();   // the cleared hash before the later records
             lanes_sync(1, main);   // also before wp is written again
         }
         return;
@@ -399,8 +400,6 @@ __global__ void __launch_bounds__(kTry64Threads, 1) k_try64(const __grid_constan
             for (int e = tb; e < 3 * nl; e += P.bodies)
                 si[(s + 1) & 1][e] = s == 0 ? fma(T.c[1] * dt, lv[e], ly[e])
                                             : poll_rec(pos_records64(P, s + 1) + e, tag0 + 2 + s, S, &dead);
-        // the last positions follow every CTA's clearing of the hash (n_stage > 3)
-        if (s + 2 == ns && P.head) __threadfence();
         lanes_sync(1, main);
     }
     if (P.adaptive) {
@@ -413,7 +412,10 @@ __global__ void __launch_bounds__(kTry64Threads, 1) k_try64(const __grid_constan
             st_pair(P.err + blockIdx.x, (unsigned)err_sm, (unsigned)(err_sm >> 32), tag_of(tag0 + 14, &dead));
     }
     for (int e = tb; e < items; e += P.bodies) solution(T, dt, ks + e, n3, yr[e], yv[e]);
-    if (tb == 0) take = poll_pair(P.decision, tag0 + 15, S, &dead).x == 1u;
+    if (tb == 0) {
+        take = poll_pair(P.decision, tag0 + 15, S, &dead).x == 1u;
+        if (P.head_n > 0) __threadfence();
+    }
     lanes_sync(3, P.bodies);
     if (!take) return;
     int* cell = reinterpret_cast<int*>(parts);   // the pull group has left it
