@@ -323,7 +323,7 @@ int red_mlp_predict(const void* w_bf16, const red_mlp_norm_t* norm, const float*
                     void* stream);
 /* Gradient of sum_r (y_r - t_r)^2 / (2 n) over n rows of normalised features xn
  * (n x 12) and targets tn, into grad (param_count floats) and loss (1 float);
- * device buffers, deterministic (fixed-order reduction). */
+ * device buffers, deterministic (fixed-order reduction), on any streams and threads at once. */
 int red_mlp_grad(const void* w_bf16, const float* xn, const float* tn, uint32_t n, float* grad, float* loss,
                  void* stream);
 /* One Adam step on FP32 master weights (device); refreshes the BF16 copy. */

@@ -460,10 +460,39 @@ int redgb_set_error(int code, const char* msg);
 static_assert(sizeof(red_mlp_norm_t) == sizeof(MlpNorm), "red_mlp_norm_t mirrors MlpNorm");
 
 namespace {
-std::mutex g_work_mu;
-float* g_work = nullptr;   // per-CTA gradients of red_mlp_grad, grown as needed
-size_t g_work_cap = 0;
-int g_work_dev = -1;
+// The per-CTA gradients of red_mlp_grad: allocated and freed in the order of the
+// caller's stream, so calls on several streams and threads have memory of their own (and
+// a captured call has the graph's).  A pool per device keeps kWorkKept bytes for the
+// next calls and gives back the rest whenever a stream is waited for.
+constexpr int kMaxDevices = 64;
+constexpr unsigned long long kWorkKept = 32ull << 20;   // two calls' largest workspaces
+std::mutex g_pool_mu;
+cudaMemPool_t g_pool[kMaxDevices] = {nullptr};
+
+cudaError_t work_pool(cudaMemPool_t* pool)
+{
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= kMaxDevices) return cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    if (!g_pool[dev]) {
+        cudaMemPoolProps p = {};
+        p.allocType = cudaMemAllocationTypePinned;
+        p.location.type = cudaMemLocationTypeDevice;
+        p.location.id = dev;
+        unsigned long long keep = kWorkKept;
+        cudaMemPool_t q = nullptr;
+        if ((e = cudaMemPoolCreate(&q, &p)) != cudaSuccess) return e;
+        if ((e = cudaMemPoolSetAttribute(q, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
+            cudaMemPoolDestroy(q);
+            return e;
+        }
+        g_pool[dev] = q;
+    }
+    *pool = g_pool[dev];
+    return cudaSuccess;
+}
 
 // The training kernels follow each other by programmatic dependent launch:
 // each waits for its predecessor before it reads anything.
@@ -503,26 +532,18 @@ int red_mlp_grad(const void* w_bf16, const float* xn, const float* tn, uint32_t 
     if (!w_bf16 || !xn || !tn || !grad || !loss || n == 0)
         return redgb_set_error(RED_ERR_ARG, "red_mlp_grad: bad argument");
     const int nblk = (int)std::min<uint32_t>((n - 1) / kTrainRows + 1, kTrainCtas);
-    const size_t need = (size_t)nblk * (kNParam + 1);
-    int dev = 0;
-    cudaGetDevice(&dev);
-    std::lock_guard<std::mutex> lk(g_work_mu);
-    if (need > g_work_cap || dev != g_work_dev) {
-        cudaStreamSynchronize((cudaStream_t)stream);
-        if (g_work) cudaFree(g_work);
-        g_work = nullptr;
-        g_work_cap = 0;
-        const cudaError_t e = cudaMalloc(&g_work, need * sizeof(float));
-        if (e != cudaSuccess) return cuda_fail(e, "red_mlp_grad: workspace");
-        g_work_cap = need;
-        g_work_dev = dev;
-    }
     cudaStream_t s = (cudaStream_t)stream;
+    cudaMemPool_t pool = nullptr;
+    float* work = nullptr;
+    cudaError_t e = work_pool(&pool);
+    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&work, (size_t)nblk * (kNParam + 1) * sizeof(float), pool, s);
+    if (e != cudaSuccess) return cuda_fail(e, "red_mlp_grad: workspace");
     const PdlScope pdl;
-    launch_k(k_mlp_train, (unsigned)nblk, (unsigned)kTrainThreads, s, (const __nv_bfloat16*)w_bf16, xn, tn, (int)n,
-             g_work);
-    launch_k(k_mlp_sum, (unsigned)(kNParam / 32 + 1), 32u * kSumWarps, s, (const float*)g_work, nblk, grad, loss);
-    const cudaError_t e = cudaGetLastError();
+    launch_k(k_mlp_train, (unsigned)nblk, (unsigned)kTrainThreads, s, (const __nv_bfloat16*)w_bf16, xn, tn, (int)n, work);
+    launch_k(k_mlp_sum, (unsigned)(kNParam / 32 + 1), 32u * kSumWarps, s, (const float*)work, nblk, grad, loss);
+    e = cudaGetLastError();
+    const cudaError_t f = cudaFreeAsync(work, s);
+    if (e == cudaSuccess) e = f;
     return e == cudaSuccess ? RED_OK : cuda_fail(e, "red_mlp_grad");
 }
 
