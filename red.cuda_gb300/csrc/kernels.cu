@@ -329,8 +329,9 @@ __device__ __forceinline__ void grid_query(const CollParams& P, int seg, int loc
     const int4 c = P.cell[i];
     // A neighbouring cell is looked up if the body is within a collision distance of
     // it: with cells of four such distances 2.2 of the 14 lists on average (512 disks:
-    // the check 123 -> ~50 us).  The body's place in its cell comes from the FP32 copy,
-    // off by less than 2^-21 (|c| + 2) edges.
+    // the check 123 -> ~50 us).  The body's place u in its cell, 0 .. 1, comes from the
+    // FP32 copy, off by less than 2^-21 (|c| + 2) edges; a u far from there (edges or
+    // positions out of FP32's range) tells nothing, and all neighbours are looked up.
     const float4 H = P.pos_hi[i];
     const float inv_h = (float)g.inv_h;
     bool lo[3], hi[3];
@@ -339,7 +340,7 @@ __device__ __forceinline__ void grid_query(const CollParams& P, int seg, int loc
         const int ck = k == 0 ? c.x : (k == 1 ? c.y : c.z);
         const float u = fmaf(k == 0 ? H.x : (k == 1 ? H.y : H.z), inv_h, -(float)ck);
         const float reach = g.reach + 0x1p-21f * (fabsf((float)ck) + 2.0f);
-        const bool any = abs(ck) >= 1 << 18;   // too far out for FP32
+        const bool any = abs(ck) >= 1 << 18 || !(fabsf(u) < 2.0f);   // too far out for FP32
         lo[k] = any || !(u > reach);
         hi[k] = any || !(u < 1.0f - reach);
     }
