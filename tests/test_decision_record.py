@@ -2,7 +2,8 @@
 
 * The exchange's two-word records (records.cuh, st_pair and poll_pair) in a ping-pong of
   many CTAs, the first word alternating as a decision's does: a reader never meets a
-  new tag beside an old word, also where it needs the first word alone.
+  new tag beside an old word, also where it needs the first word alone.  The three-word
+  records (st_rec16 and poll16) beside them.
 * Adaptive runs in which every second try or so is rejected: each body ends where its
   Kepler orbit has it at the handle's time.  The protoplanets and planetesimals have a
   mass of 1e-25, so that the star alone acts; RKF7(8) at a tolerance of 1e-10 keeps the
@@ -25,7 +26,7 @@ SHIM = r'''
 using namespace redgb;
 
 // CTA 0 sends round n to everyone and waits for every answer; one cooperative launch
-__global__ void k_rounds(uint4* word, uint4* answer, int rounds, DevSys* S, unsigned* wrong)
+__global__ void k_rounds(uint4* word, uint4* three, uint4* answer, int rounds, DevSys* S, unsigned* wrong)
 {
     __shared__ int dead;
     if (threadIdx.x == 0) dead = 0;
@@ -34,8 +35,12 @@ __global__ void k_rounds(uint4* word, uint4* answer, int rounds, DevSys* S, unsi
     for (int n = 1; n <= rounds; n++) {
         if (blockIdx.x == 0) {
             if (threadIdx.x == 0) st_pair(word, n & 1, 0u, n);
+            if (threadIdx.x == 32) st_rec16(three, n, ~(unsigned)n, 5u * n, n);
             for (int j = threadIdx.x; j < n_cta; j += blockDim.x)
                 if (poll_pair(answer + j, n, S, &dead).x != (unsigned)n * 3u) atomicAdd(wrong + 1, 1u);
+        } else if (threadIdx.x == 32) {
+            const uint4 v = poll16(three, n, S, &dead);
+            if (v.x != (unsigned)n || v.y != ~(unsigned)n || v.z != 5u * n) atomicAdd(wrong + 2, 1u);
         } else if (threadIdx.x == 0) {
             if (poll_pair(word, n, S, &dead).x != (unsigned)(n & 1)) atomicAdd(wrong, 1u);
             st_pair(answer + blockIdx.x - 1, (unsigned)n * 3u, ~(unsigned)n, n);
@@ -50,17 +55,17 @@ extern "C" int run_rounds(int n_cta, int rounds, unsigned* wrong, int* status)
     uint4* rec = nullptr;
     DevSys *S = nullptr, h;
     unsigned* w = nullptr;
-    cudaMalloc(&rec, (n_cta + 1) * sizeof(uint4));
+    cudaMalloc(&rec, (n_cta + 2) * sizeof(uint4));
     cudaMalloc(&S, sizeof(DevSys));
-    cudaMalloc(&w, 2 * sizeof(unsigned));
-    cudaMemset(rec, 0, (n_cta + 1) * sizeof(uint4));
+    cudaMalloc(&w, 3 * sizeof(unsigned));
+    cudaMemset(rec, 0, (n_cta + 2) * sizeof(uint4));
     cudaMemset(S, 0, sizeof(DevSys));
-    cudaMemset(w, 0, 2 * sizeof(unsigned));
-    uint4* answer = rec + 1;
-    void* args[] = {&rec, &answer, &rounds, &S, &w};
+    cudaMemset(w, 0, 3 * sizeof(unsigned));
+    uint4 *three = rec + 1, *answer = rec + 2;
+    void* args[] = {&rec, &three, &answer, &rounds, &S, &w};
     cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_rounds, dim3(n_cta + 1), dim3(64), args, 0, 0);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    if (e == cudaSuccess) e = cudaMemcpy(wrong, w, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(wrong, w, 3 * sizeof(unsigned), cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = cudaMemcpy(&h, S, sizeof(DevSys), cudaMemcpyDeviceToHost);
     *status = h.status;
     cudaFree(rec);
@@ -78,9 +83,9 @@ def test_records_are_whole(tmp_path):
     subprocess.check_call([nvcc, "-shared", "-Xcompiler", "-fPIC", "-gencode", "arch=compute_103a,code=sm_103a",
                            "-O3", "-std=c++17", "--expt-relaxed-constexpr", "-ftz=true",
                            "-I" + os.path.join(ROOT, "include"), "-I" + CSRC, "-o", str(so), str(src)])
-    wrong, status = (C.c_uint * 2)(), C.c_int(-1)
+    wrong, status = (C.c_uint * 3)(), C.c_int(-1)
     assert C.CDLL(str(so)).run_rounds(140, 20000, wrong, C.byref(status)) == 0
-    assert status.value == 0 and list(wrong) == [0, 0]
+    assert status.value == 0 and list(wrong) == [0, 0, 0]
 
 
 def vec(a):
