@@ -4,7 +4,8 @@ Workload (default): one planetesimal disk of N = 16384 bodies -- 1 star, 16
 protoplanets of 0.05 M_earth spaced 10 mutual Hill radii from 0.5 AU, 16367
 planetesimals log-uniform in [0.5, 3] AU -- integrated with adaptive RKF7(8)
 at tolerance 1e-10, collision detection on, mixed precision (FP32 pairwise
-gravity on double-single coordinates, FP64 star term, state and step control).
+gravity on double-single coordinates, double-single star term, FP64 state and step
+control).
 
 A step is a run of `tries_per_step` consecutive tries of the integrator over
 the disk (each try: 13 force evaluations, the error norm, step control,

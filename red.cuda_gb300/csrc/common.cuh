@@ -184,7 +184,7 @@ __device__ __forceinline__ double f2d_bits(float f)
     return __longlong_as_double((long long)(sign | (ee << 52) | ((unsigned long long)(u & 0x7FFFFFu) << 29)));
 }
 // 1 / sqrt(x) in FP64 with few FP64 instructions (GB300 issues one warp of them
-// in 16 cycles): the FP32 hardware estimate y of the truncated x, then one
+// in 19 cycles): the FP32 hardware estimate y of the truncated x, then one
 // Householder step of third order, y + y e (1/2 + 3/8 e) with e = 1 - x y^2;
 // y^2 is exact (48 bits) and e^3 ~ 2^-63, so the result is within an ulp or
 // so.  x outside FP32's normal range takes the library's function.

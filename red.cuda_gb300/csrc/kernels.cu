@@ -154,8 +154,8 @@ __global__ void __launch_bounds__(3 * kFinishBodies) k_finish(const FinishParams
 
 // ---------------------------------------------------------------------------
 // collision detection: kernel_pp_disk::check_for_collision (pp_disk.cu:320-371)
-// over tile pairs; an FP32 double-single prefilter with a safety margin picks
-// the candidates, red's FP64 test (no FMA) decides.
+// over tile pairs; an FP32 filter with a safety margin picks the candidates, red's
+// FP64 test (no FMA) decides.
 // ---------------------------------------------------------------------------
 // After a try the check runs for the systems that just accepted one (a halted
 // system makes no tries, so it never has `accepted` set); the explicit check
@@ -204,10 +204,14 @@ __device__ __forceinline__ void collide_exact(const CollParams& P, DevSys* S, in
 // bodies) sits in shared memory, every value twice.
 //
 // The filter sees the FP32 copies of the positions alone: two bodies closer than
-// factor (R_i + R_j) are there closer than A_i + A_j, A = factor R + 2^-23 max |x|,
-// since a copy is off by up to 2^-24 |x| in each coordinate; 1e-4 and 1e-15 cover the
-// rounding of the filter.  The few that pass, and whatever compares with NaN or
-// infinity, take red's FP64 test.
+// T = factor (R_i + R_j) are there closer than A_i + A_j, A = factor R + 2^-23 M, M the
+// largest |coordinate|.  A copy is its coordinate truncated, off by up to 2^-23 |x| towards
+// zero.  Coordinates of one sign: the errors' difference is at most the larger one, over
+// three of them sqrt(3) 2^-23 max(M_i, M_j), which is below 2^-23 (M_i + M_j) where T <
+// 0.26 max(M_i, M_j), since the M differ by at most T, and below 8e-7 T elsewhere.
+// Coordinates of opposite signs: at most 2^-23 of their distance.  The factor 1.0001 covers
+// the shares of T and the filter's own rounding, 1e-15 what FP32 flushes.  The few that
+// pass, and whatever compares with NaN or infinity, take red's FP64 test.
 //
 // Bound by instruction issue: ~6 a pair, where double-single differences of one pair
 // at a time took ~24.  16384 bodies, all pairs: 158 -> 57 us. The

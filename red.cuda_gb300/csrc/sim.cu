@@ -224,7 +224,7 @@ namespace redgb {
 // The gravity classes of one system: sinks [s0, s1) against sources [j0, j1)
 // (body indices relative to the system), red's interaction bounds
 // (red_type.h:670-692); the FP32 modes take the stars out of the sources (their
-// term is added in FP64 by the epilogue).
+// term is added in double-single by the epilogue).
 struct GravClass { int cls, s0, s1, j0, j1; };
 static void gravity_classes(const SysInfo& si, int mode, GravClass out[3])
 {
@@ -1016,13 +1016,13 @@ void red_sim::build_plan()
 // more.  REDGB_PAIRS=0 keeps one-sided tiles.
 void red_sim::plan_pairs()
 {
-    // One RKF7(8) try, one-sided / each pair once: 346 / 366 us at 4096 bodies, 629 /
-    // 501 at 6144, 903 / 647 at 8192 (MIXED; FP32 mode alike).
+    // One RKF7(8) try, one-sided / each pair once: 305 / 393 us at 4096 bodies, 436 / 401 at
+    // 5120, 579 / 507 at 6144, 943 / 629 at 8192 (MIXED; FP32 mode 258 / 301, 369 / 311, ..).
     constexpr int kPairMin = 5120;
     // Sub-blocks per job: jobs of a few waves (4 CTAs on each of 152 SMs) balance the
     // SMs, longer ones leave fewer records.  16384 bodies: 1.84 ms per RKF7(8) try at
     // two (1056 jobs), 1.86 at one; 65536, RK4 in FP32: 5.71 ms per try at eight (4160
-    // jobs), 5.80 at sixteen, 6.11 at 32 (before the pair terms lost an operation).
+    // jobs), 5.80 at sixteen, 6.11 at 32 (with earlier forms of the pair terms and sums).
     constexpr long long kPairJobs = 4096, kPairWaves = 2048;
     use_pairs = false;
     pair_slots.clear();

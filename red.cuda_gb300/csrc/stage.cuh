@@ -612,7 +612,7 @@ __device__ __forceinline__ void gravity_f64(SmemStage& sm, const StageParams& P,
 // pp_disk.cu:389-413).  red adds the pair terms of a sink one after the other
 // in index order; the terms themselves do not depend on the order.  So the
 // CTA's threads form the terms side by side (a square root and a division each,
-// ~60 FP64 instructions of which the SM issues a full warp in 16 cycles), and
+// ~60 FP64 instructions of which the SM issues a full warp in 19 cycles), and
 // one thread per (sink, component) adds them in order.  A pair that red skips
 // (the sink itself, an inactive source) adds +0.0: the sum starts at +0.0 and
 // round-to-nearest never makes it -0.0, so that changes no bit.
@@ -620,7 +620,7 @@ __device__ __forceinline__ void gravity_f64(SmemStage& sm, const StageParams& P,
 // An unchunked tile keeps the terms in shared memory, kPairBatch at a time.  A
 // chunked tile (few sinks against many sources: the large-body class) writes
 // them to `partial`, 3 nsink doubles per source, and the CTA that counts last
-// adds all of them (sum_terms): its chain of dependent additions, ~110 cycles
+// adds all of them (sum_terms): its chain of dependent additions, ~80 cycles
 // each, is then all that is serial.  4100-body disk (9 large bodies), adaptive
 // RKF7(8): 57.6 ms per try when one lane formed and added the terms of its
 // sink in turn, 2.46 ms now.
@@ -698,7 +698,7 @@ __device__ __forceinline__ double gravity_exact(SmemStage& sm, double* terms, co
 // The sums over the n sources of a chunked tile's terms (nel doubles per source,
 // contiguous), element threadIdx.x < nel, added in order.  All threads bring the
 // terms to shared memory, a batch ahead of the additions, so that these follow
-// each other at the latency of an FP64 addition (64 cycles).  (With each
+// each other at ~80 cycles, near the latency of an FP64 addition (64).  (With each
 // element loading its own terms to registers, a batch ahead, an addition took
 // ~115 cycles: 2.95 ms per try of the 4100-body disk, 2.46 ms now.)
 __device__ __forceinline__ double sum_terms(const double* base, int nel, int n, double* buf)

@@ -1,4 +1,4 @@
-// stage_mixed.cu -- k_stage instantiated for mode MIXED: double-single FP32 body-body pairs, FP64 star term.
+// stage_mixed.cu -- k_stage instantiated for mode MIXED: double-single FP32 body-body pairs and star term.
 // One translation unit per mode keeps the parallel build short; each unit
 // holds its own copy of the Butcher tableau in constant memory.
 #include "stage.cuh"

@@ -19,7 +19,7 @@
 // stage to complete, and stage velocities are formed only for gas drag.
 //
 // The pair and star sums leave the accelerations as double-single numbers (the star
-// term is good to ~2e-14); everything formed from them is FP64, as in the stage
+// term is good to ~7e-14); everything formed from them is FP64, as in the stage
 // kernel: the stage sums, positions and velocities, the drag, the error, the solution.
 // GB300 issues an FP64 warp instruction every 19 cycles and SM and a dependent one
 // takes 64, so a component's sum is one thread's chain, off the exchange's path but for
@@ -31,8 +31,8 @@
 // the instruction chains of a phase (~2.7 us per phase on the 16384-body disk, 1.3
 // of them the pull on the large bodies, whose records the exchange waits for).
 // Measured against one launch per stage, per try: 16384-body disk, adaptive
-// RKF7(8), 115 -> 59 us; 65536-body gas-drag disk 418 -> 258 us (FP64 pipe: the rows of
-// velocities and the drag); 2053-body disk, RK4, 33.2 -> 20.6 us.  What that took besides the layout: the system record is
+// RKF7(8), 115 -> 58 us; 65536-body gas-drag disk 418 -> 259 us (FP64 pipe: the rows of
+// velocities and the drag); 2053-body disk, RK4, 33.2 -> 21.3 us.  What that took besides the layout: the system record is
 // read by one thread of a CTA and the position records are written in kTryCopies
 // copies, because thousands of readers of one sector queue up for microseconds.
 //
@@ -148,7 +148,8 @@ __host__ __device__ constexpr int try_max_threads(bool drag) { return drag ? 102
 // same phases).  A large body's sum and its next position are formed by a warp
 // of the team in the phase after the partials, as long as that phase lasts.  512
 // disks (1.1 M bodies), adaptive RKF7(8), four tries with the states in and out, against
-// one launch per stage: 11.35 -> 8.29 ms (7.04 with double-single stage sums).
+// one launch per stage: 11.35 -> 8.46 ms (7.04 with double-single stage sums and longer
+// FP32 runs).  FP64 pipe 46 % busy, 46 % of the stall at the barriers.
 // ---------------------------------------------------------------------------
 constexpr int kTeamCtas = 10;          // largest cluster; a team is at most 8 of its CTAs
 constexpr int kTeamSize = 8;
